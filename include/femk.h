@@ -123,7 +123,8 @@ typedef struct femk_plan_options {
                              operator; 0: with the canonical CSR itself (the plain method) */
   int32_t column_tables;  /* 1 (default): a slice whose 32 rows share one column-offset sequence stores it once */
   int32_t cols16;         /* 1 (default): int16 column offsets in the FP64 sliced-ELL stream when they fit */
-  int32_t graph_replay;   /* 1 (default): CG / mixed chunks replayed as CUDA graphs; 0: launched one by one */
+  int32_t graph_replay;   /* 1 (default): CG / mixed chunks replayed as CUDA graphs; 0: launched one by one
+                             (systems whose operator stays on the chip run femk_pcg as one launch either way) */
   int32_t l2_hints;       /* L2 eviction hints of the FP64 CG kernels: -1 (default) on for P1, off for P2;
                              0 off; 1 matrix evict-first, gathers and vectors evict-last; 2 matrix evict-first,
                              vectors evict-last; 3 vectors evict-last only; 4 as 1 with streaming matrix loads */
@@ -233,9 +234,10 @@ int femk_spmv(const femk_plan* plan, const double* vals_dev, const double* x_dev
 int femk_prepare_operator(const femk_plan* plan, const double* vals_dev, void* stream);
 int femk_spmv_prepared(const femk_plan* plan, const double* x_dev, double* y_dev, void* stream);
 
-/* Opt-in CUDA-event timing of the FP64 CG loop's kernels (step SpMV, x/r/z update, p update),
- * accumulated over the iterations that ran since profiling was switched on. While it is on,
- * femk_pcg enqueues its chunks directly instead of replaying the chunk graph. */
+/* Opt-in timing of the FP64 CG loop's parts (step SpMV, x/r/z update, p update), accumulated over the
+ * iterations that ran since profiling was switched on. While it is on, femk_pcg enqueues its chunks
+ * directly instead of replaying the chunk graph, with CUDA events around each kernel; a solve that runs as
+ * a single launch times the same parts with the SM clock, each with the grid-wide wait that ends it. */
 int femk_set_profiling(femk_plan* plan, int on);
 int femk_get_profile(const femk_plan* plan, double* step_ms, double* update_ms, double* pupdate_ms,
                      int64_t* iterations);

@@ -28,7 +28,7 @@ namespace femk {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kChunk = 16;  // iterations enqueued between looks at the done flag
+constexpr int kChunk = kCgChunk;
 
 enum SpmvMode { kPlain = 0, kCgStep = 1, kInit = 2, kResid = 3 };
 
@@ -1044,14 +1044,6 @@ int launch_matfree(const femk_plan* p, const MatFree& m, const double* x, double
 }
 
 // One chunk of CG iterations on stream ws: the step SpMV and the two vector kernels per iteration.
-// Opt-in per-kernel timing of the CG loop (femk_set_profiling): events around the three kernels
-// of every iteration of a chunk; the chunked path runs without graph replay while it is on.
-struct ProfData {
-  cudaEvent_t ev[kChunk][4];
-  double ms[3] = {0.0, 0.0, 0.0};  // step SpMV, update, p update
-  int64_t iters = 0;
-};
-
 int enqueue_chunk(const femk_plan* p, const double* vals, double* x, const double* dinv, bool sell, int64_t iters,
                   cudaStream_t ws) {
   const int64_t vs = p->vstride;
@@ -1433,6 +1425,8 @@ extern "C" int femk_pcg(const femk_plan* p, const double* vals, const double* b,
   clear_error();
   FEMK_CHECK_ARG(p && vals && b && x, "femk_pcg: NULL argument");
   FEMK_CHECK_ARG(tol >= 0.0 && atol >= 0.0, "femk_pcg: negative tolerance");
+  if (pcg_persist_fits(p))
+    return pcg_persist(p, vals, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, (cudaStream_t)stream);
   return pcg_run(p, vals, nullptr, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, (cudaStream_t)stream);
 }
 

@@ -228,6 +228,12 @@ struct femk_plan {
   cudaStream_t batch_stream = nullptr;
   cudaEvent_t batch_ev = nullptr;
   int batch_graph_ok = 1;
+  // single-launch solvers of systems that stay on the chip (femk_persist.cu)
+  int persist_ok = 0;           // 1 unless the options pick the kernels of the chunked solvers
+  void* persist_ws = nullptr;   // f64[6 vstride] {z, p} pairs and vectors, then the GridWords
+  void* persist_words = nullptr;  // (in persist_ws) partial sums and arrival counters of the grid form
+  int persist_turn = 0;         // which arrival counter the next launch uses
+  void* persist_out = nullptr;  // pinned result
   void* prof = nullptr;         // per-kernel CG timing (femk_set_profiling)
   double* coef_tmp = nullptr;   // f64[ntet] element coefficients of a nodal parameter
   double* kcoef = nullptr;      // f64[ntet] exp(param) of the current assembly or matrix-free solve
@@ -281,6 +287,21 @@ int ensure_workspace(femk_plan* p);
 // graph capture); launch_sell_values enqueues the copies (FP64, and the unscaled FP32 values).
 int ensure_sell_values(femk_plan* p, bool fp32);
 int launch_sell_values(const femk_plan* p, const double* vals, bool fp32, cudaStream_t s);
+
+constexpr int kCgChunk = 16;  // CG iterations enqueued between looks at the done flag
+
+// Opt-in timing inside the FP64 CG loop (femk_set_profiling). The chunked solver records events around the three
+// kernels of every iteration of a chunk and runs without graph replay; the single launch reads its clock.
+struct ProfData {
+  cudaEvent_t ev[kCgChunk][4];
+  double ms[3] = {0.0, 0.0, 0.0};  // step SpMV, update, p update
+  int64_t iters = 0;
+};
+
+// Jacobi-PCG as one persistent launch (femk_persist.cu), for plans whose operator stays on the chip.
+bool pcg_persist_fits(const femk_plan* p);
+int pcg_persist(const femk_plan* p, const double* vals, const double* b, double* x, const double* dinv, double tol,
+                double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s);
 
 // Nodal P1 coefficient modes become a per-element coefficient (plan-owned f64[ntet], computed on
 // stream s) read as FEMK_COEF_LINEAR; other modes pass through unchanged.

@@ -1,0 +1,411 @@
+// Jacobi-PCG as one persistent launch, for systems whose operator stays on the chip (femk_persist.cuh).
+//
+// The chunked solver (femk_cg.cu) runs three kernels an iteration, each with its launch gap, its ramp and a
+// last-block reduction: at P1 32^3 (35,937 rows, 5.3 MB of operator) that takes 17.8 us an iteration, 13.3 us of it
+// in the kernels.
+// Here an iteration is two phases of one kernel, the same floating-point operations as k_update_r /
+// k_pupdate_x / the product, in the same order within a row:
+//   A  p_i = z_i + beta p_i;  q_i = sum_j a_ij (z_j + beta p_j);  <p, q>                     -> alpha
+//   B  x += alpha p;  r -= alpha q;  z = D^-1 r;  <r, z>, <r, r>                                  -> beta, stop test
+// The product forms the new direction at every gather from the pair {z_j, p_j} (one 16-byte load), so the
+// direction needs no phase, and no barrier, of its own. What is left is bound by the two barriers an iteration
+// (4.3 of the 7.1 us at 32^3) and, from 64^3 on, by the gathers and the operator's share that L2 holds. 512
+// threads: 768 and 1024 spill at 80 and 64 registers (64^3: 12.0 us an iteration, against 12.9 and 14.3).
+// The recurrence q = A z + beta q would gather z alone and gained 5-15 %, but its true residual at tolerances of
+// 1e-13 and below was up to 2.5 times larger, so the product keeps the textbook form.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <string>
+
+#include "femk_persist.cuh"
+
+namespace femk {
+namespace {
+
+constexpr int kPT = 512;                    // threads of a block, one block per SM
+constexpr int kPersistSmem = 220 * 1024;    // dynamic shared memory of a block (227 KB less the static part)
+// ... with int32 columns (no banded order): the gathers of the pairs then need L1, which is what shared memory
+// leaves (us an iteration with 220 / 100 KB: P2 26^3 29.2 / 18.5, shuffled P1 40^3 14.0 / 9.6; with int16 columns
+// P1 64^3 11.9 / 12.3, 80^3 20.6 / 30.8)
+constexpr int kPersistSmemWide = 100 * 1024;
+
+struct PersistOut {
+  double rr, gamma, atol2, ww, bb;
+  int32_t iter, status;
+  // a profiled solve, block 0: clock cycles of the products, the updates and the directions; of the whole loop,
+  // in cycles and in nanoseconds
+  long long cycles[3], loop_cycles, loop_ns;
+};
+
+struct PcgArgs {
+  const int64_t* sptr;
+  const void* cols;
+  const double* svals;
+  int64_t n, nslices;
+  const double* b;
+  double* x;
+  const double* dinv;
+  double2* zp;      // {z, p} of every row: what other blocks gather
+  double* work;     // r, p, q, D^-1 (vstride apart) of blocks whose rows do not fit in shared memory
+  int64_t vstride;
+  GridWords* words;
+  int32_t turn, skip;
+  long long limit;
+  int32_t smem;     // dynamic shared memory of a block
+  double tol2, atol2;
+  int32_t maxiter, relres, timed;
+  PersistOut* out;  // pinned host memory
+  int* err;
+};
+
+__device__ __forceinline__ long long global_ns() {
+  long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+template <int SET, typename IDX>
+__global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
+  extern __shared__ __align__(16) unsigned char ps_smem[];
+  __shared__ int32_t fit_s;
+  constexpr int W = kPT / 32;
+  constexpr bool ONE = SET == kOneBlock;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t nsl = (int32_t)a.nslices;
+  const int G = (int)gridDim.x, bid = (int)blockIdx.x;
+  BlockMatrix<IDX> m;
+  m.s0 = block_slice(a.sptr, nsl, bid, G);
+  m.ns = block_slice(a.sptr, nsl, bid + 1, G) - m.s0;
+  const int64_t e0 = __ldg(a.sptr + m.s0);
+  const int32_t r0 = m.s0 * 32, nr = m.ns * 32;
+  // shared memory: slice offsets, the block's x, r, p, q, D^-1 (and the pairs, when one block owns all), slices
+  int32_t* off = reinterpret_cast<int32_t*>(ps_smem);
+  const int32_t head = (4 * (m.ns + 1) + 15) & ~15;
+  const bool vin = ONE || head + 40 * nr <= a.smem;
+  double* vec = reinterpret_cast<double*>(ps_smem + head);
+  double* xs = vin ? vec : a.x + r0;
+  double* rs = vin ? vec + nr : a.work + r0;
+  double* ps = vin ? vec + 2 * nr : a.work + a.vstride + r0;
+  double* qs = vin ? vec + 3 * nr : a.work + 2 * a.vstride + r0;
+  double* ds = vin ? vec + 4 * nr : a.work + 3 * a.vstride + r0;
+  double2* zps = reinterpret_cast<double2*>(vec + 5 * nr);
+  unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
+  for (int32_t s = threadIdx.x; s <= m.ns; s += kPT) off[s] = (int32_t)(__ldg(a.sptr + m.s0 + s) - e0);
+  if (threadIdx.x == 0) fit_s = 0;
+  if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
+  __syncthreads();
+  const int32_t room = a.smem - (int32_t)(mat - ps_smem);
+  for (int32_t s = threadIdx.x; s < m.ns; s += kPT)
+    if ((int64_t)off[s + 1] * (8 + (int)sizeof(IDX)) <= room) atomicMax(&fit_s, s + 1);
+  __syncthreads();
+  m.fit = fit_s;
+  m.off = off;
+  m.gv = a.svals + e0;
+  m.gc = reinterpret_cast<const IDX*>(a.cols) + e0;
+  const int32_t held = off[m.fit];
+  double* sv = reinterpret_cast<double*>(mat);
+  IDX* sc = reinterpret_cast<IDX*>(sv + held);
+  for (int32_t k = threadIdx.x; k < held; k += kPT) {
+    sv[k] = __ldg(m.gv + k);
+    sc[k] = __ldg(m.gc + k);
+  }
+  m.sv = sv;
+  m.sc = sc;
+  __syncthreads();
+  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
+  // r = b - A x0, z = D^-1 r
+  // gathers of x and of the pairs, range-checked in the bounds-checked build
+  auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int32_t s = warp; s < m.ns; s += W) {
+    const int32_t i = s * 32 + lane, row = r0 + i;
+    if (row >= a.n) continue;
+    const double ax = block_row<16>(m, s, lane, row, xat);
+    const double bi = __ldg(a.b + row);
+    const double ri = bi - ax;
+    const double di = a.dinv ? __ldg(a.dinv + row) : 1.0;
+    const double zi = a.dinv ? di * ri : ri;
+    rs[i] = ri;
+    ds[i] = di;
+    ps[i] = 0.0;
+    if (ONE)
+      zps[i] = make_double2(zi, 0.0);
+    else
+      a.zp[row] = make_double2(zi, 0.0);
+    acc[0] += ri * zi;
+    acc[1] += ri * ri;
+    acc[2] += bi * bi;
+  }
+  if (vin)
+    for (int32_t i = threadIdx.x; i < nr; i += kPT)
+      if (r0 + i < a.n) xs[i] = a.x[r0 + i];
+  bool live = grid.template sum<3>(acc);
+  double gamma = acc[0], rr = acc[1], beta = 0.0;
+  const double bb = acc[2], atol2 = fmax(a.tol2 * bb, a.atol2);
+  int32_t status = isfinite(gamma) && isfinite(rr) ? FEMK_OK : FEMK_NONFINITE;
+  int32_t iter = 0;
+  bool done = !((a.dinv ? rr : gamma) > atol2) || a.maxiter <= 0 || status != FEMK_OK;
+  long long t0 = 0, ns0 = 0, spent[3] = {0, 0, 0}, first = 0;
+  if (a.timed) {
+    first = t0 = clock64();
+    ns0 = global_ns();
+  }
+  auto lap = [&](int k) {
+    const long long t = clock64();
+    spent[k] += t - t0;
+    t0 = t;
+  };
+  auto direction = [&](int32_t i) { return fma(beta, ps[i], a.dinv ? ds[i] * rs[i] : rs[i]); };
+  while (live && !done) {
+    double pq[1] = {0.0};
+    if (a.timed) {  // a profiled solve forms the directions in a pass of their own (the same bits)
+      for (int32_t i = warp * 32 + lane; i < nr; i += kPT)
+        if (r0 + i < a.n) ps[i] = direction(i);
+      lap(2);
+    }
+    for (int32_t s = warp; s < m.ns; s += W) {
+      const int32_t i = s * 32 + lane, row = r0 + i;
+      if (row >= a.n) continue;
+      const double qi = block_row<16>(m, s, lane, row, [&](int32_t j) {
+        if (!FEMK_IN_BOUNDS(j, a.n, a.err)) return 0.0;
+        const double2 v = ONE ? zps[j] : a.zp[j];
+        return fma(beta, v.y, v.x);
+      });
+      const double pi = a.timed ? ps[i] : direction(i);
+      ps[i] = pi;
+      qs[i] = qi;
+      pq[0] += pi * qi;
+    }
+    live = grid.template sum<1>(pq);
+    if (a.timed) lap(0);
+    if (!live) break;
+    if (!(pq[0] > 0.0) || !isfinite(pq[0])) {
+      status = isfinite(pq[0]) ? FEMK_BREAKDOWN : FEMK_NONFINITE;
+      break;
+    }
+    const double alpha = gamma / pq[0];
+    double rz[2] = {0.0, 0.0};
+    for (int32_t s = warp; s < m.ns; s += W) {
+      const int32_t i = s * 32 + lane, row = r0 + i;
+      if (row >= a.n) continue;
+      const double pi = ps[i];
+      xs[i] = fma(alpha, pi, xs[i]);
+      const double ri = fma(-alpha, qs[i], rs[i]);
+      const double zi = a.dinv ? ds[i] * ri : ri;
+      rs[i] = ri;
+      if (ONE)
+        zps[i] = make_double2(zi, pi);
+      else
+        a.zp[row] = make_double2(zi, pi);
+      rz[0] += ri * zi;
+      rz[1] += ri * ri;
+    }
+    live = grid.template sum<2>(rz);
+    if (a.timed) lap(1);
+    beta = rz[0] / gamma;
+    gamma = rz[0];
+    rr = rz[1];
+    ++iter;
+    if (!isfinite(gamma) || !isfinite(rr)) {
+      status = FEMK_NONFINITE;
+      done = true;
+    } else {
+      done = !((a.dinv ? rr : gamma) > atol2) || iter >= a.maxiter;
+    }
+  }
+  const long long last = t0, ns1 = a.timed ? global_ns() : 0;
+  if (vin) {
+    __syncthreads();
+    for (int32_t i = threadIdx.x; i < nr; i += kPT)
+      if (r0 + i < a.n) a.x[r0 + i] = xs[i];
+  }
+  double w2[1] = {0.0};
+  if (live && a.relres) {  // <b - A x, b - A x> of the returned x
+    double none[1] = {0.0};
+    live = grid.template sum<1>(none);
+    for (int32_t s = warp; s < m.ns; s += W) {
+      const int32_t row = r0 + s * 32 + lane;
+      if (row >= a.n) continue;
+      const double wi = __ldg(a.b + row) - block_row<16>(m, s, lane, row, xat);
+      w2[0] += wi * wi;
+    }
+    if (live) live = grid.template sum<1>(w2);
+  }
+  grid.leave();
+  if (bid == 0 && threadIdx.x == 0) {
+    a.out->rr = rr;
+    a.out->gamma = gamma;
+    a.out->atol2 = atol2;
+    a.out->ww = w2[0];
+    a.out->bb = bb;
+    a.out->iter = iter;
+    a.out->status = live ? status : FEMK_TIMEOUT;
+    for (int k = 0; k < 3; ++k) a.out->cycles[k] = spent[k];
+    a.out->loop_cycles = last - first;
+    a.out->loop_ns = ns1 - ns0;
+  }
+}
+
+// One launch of a persistent kernel: co-resident blocks (a cluster, or a cooperative grid).
+template <typename Args>
+int launch_set(const femk_plan* p, void (*kern)(Args), int set, int grid, const Args& a, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kPT);
+  cfg.dynamicSmemBytes = (size_t)a.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  cfg.attrs = at;
+  cfg.numAttrs = 0;
+  if (set == kOneCluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = grid;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  } else if (set == kGrid) {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.numAttrs = 1;
+  }
+  counted_launch();
+  FEMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
+  return FEMK_OK;
+}
+
+// shared-memory limit and cluster size of a kernel, set once per device
+template <typename Args>
+int prepare_kernel(void (*kern)(Args), int set, int device, std::atomic<uint64_t>& ready) {
+  const uint64_t bit = 1ull << (device & 63);
+  if (ready.load(std::memory_order_acquire) & bit) return FEMK_OK;
+  FEMK_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmem));
+  if (set == kOneCluster)
+    FEMK_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  ready.fetch_or(bit, std::memory_order_release);
+  return FEMK_OK;
+}
+
+template <int SET, typename IDX>
+int launch_pcg(const femk_plan* p, const PcgArgs& a, int grid, cudaStream_t s) {
+  static std::atomic<uint64_t> ready{0};
+  FEMK_TRY(prepare_kernel(k_pcg_persist<SET, IDX>, SET, p->device, ready));
+  return launch_set(p, k_pcg_persist<SET, IDX>, SET, grid, a, s);
+}
+
+// Bytes of the sliced-ELL operator: what every iteration reads.
+int64_t operator_bytes(const femk_plan* p) { return p->sell_nnz * (p->sell_c16 ? 10 : 12); }
+
+// One allocation for all of the solver's global memory: the pairs, the vectors of blocks whose rows do not fit
+// in shared memory, and the grid's words.
+int ensure_persist(femk_plan* p) {
+  if (!p->persist_ws) {
+    const size_t vec = sizeof(double) * 6 * (size_t)p->vstride;
+    char* ws = nullptr;
+    FEMK_CUDA_TRY(cudaMalloc(&ws, vec + sizeof(GridWords)));
+    p->persist_ws = ws;
+    p->persist_words = ws + vec;
+    FEMK_CUDA_TRY(cudaMemset(p->persist_words, 0, sizeof(GridWords)));
+  }
+  if (!p->persist_out) FEMK_CUDA_TRY(cudaMallocHost(&p->persist_out, sizeof(PersistOut)));
+  return FEMK_OK;
+}
+
+}  // namespace
+
+// Up to 80 MB of operator the single launch wins, above it the chunked solver does: past that the operator, the
+// vectors and the pairs no longer stay in L2 together. B200, FP64 PCG to 1e-8, us an iteration, chunked ->
+// single launch: P1 32^3 (5.3 MB) 17.8 -> 7.1, 64^3 (41 MB) 21.3 -> 12.0, 80^3 (79 MB) 28.3 -> 18.5, 84^3 (91 MB)
+// 31.6 -> 31.5, 88^3 (105 MB) 33.6 -> 47.6; P2 26^3 (57 MB) 27.0 -> 18.5, 32^3 (104 MB) 36.8 -> 40.1.
+bool pcg_persist_fits(const femk_plan* p) {
+  return p->persist_ok && p->coop && p->use_sell && p->sell_cols && operator_bytes(p) <= 80000000;
+}
+
+int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double* x, const double* dinv, double tol,
+                double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s) {
+  femk_plan* p = const_cast<femk_plan*>(pc);
+  FEMK_TRY(ensure_persist(p));
+  FEMK_TRY(ensure_sell_values(p, false));
+  FEMK_TRY(launch_sell_values(p, vals, false, s));
+  PersistOut* out = (PersistOut*)p->persist_out;
+  out->status = FEMK_TIMEOUT;
+  PcgArgs a{};
+  a.sptr = p->sell_ptr;
+  a.cols = p->sell_c16 ? (const void*)p->sell_c16 : (const void*)p->sell_cols;
+  a.svals = p->sell_vals;
+  a.n = p->n;
+  a.nslices = p->n_slices;
+  a.b = b;
+  a.x = x;
+  a.dinv = dinv;
+  a.zp = (double2*)p->persist_ws;
+  a.work = (double*)p->persist_ws + 2 * p->vstride;
+  a.vstride = p->vstride;
+  a.words = (GridWords*)p->persist_words;
+  a.turn = p->persist_turn;
+  a.skip = p->skip_arrival;
+  a.limit = p->barrier_spin;
+  a.smem = p->sell_c16 ? kPersistSmem : kPersistSmemWide;
+  a.tol2 = tol * tol;
+  a.atol2 = atol * atol;
+  a.maxiter = maxiter;
+  a.relres = relres_out != nullptr;
+  ProfData* pd = (ProfData*)p->prof;
+  a.timed = pd != nullptr;
+  a.out = out;
+  a.err = p->dev_err;
+  // One block, with no wait for others, when all of it fits one SM. Then one cluster of up to 16 blocks: its
+  // barrier is twice as fast as the grid's, until 16 SMs take longer over the rows than that gains (us an
+  // iteration, cluster against grid: 2-D P1 100^2, 319 slices, 4.1 / 5.7; P1 20x22x24, 378 slices, 5.8 / 7.0;
+  // 2-D P2 60^2, 458 slices, 6.3 / 6.9; 2-D P2 70^2, 622 slices, 7.0 / 6.7; P1 28^3, 763 slices, 8.4 / 7.2).
+  // 16 slices a block: a slice a warp (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148).
+  const int64_t one = 4 * (p->n_slices + 1) + 16 + p->n_slices * 32 * 56 + operator_bytes(p);
+  int set = kGrid, grid = (int)std::min<int64_t>(std::min(p->n_sm, kMaxBlocks), (p->n_slices + 15) / 16);
+  if (one <= a.smem) {
+    set = kOneBlock, grid = 1;
+  } else if (p->n_slices <= 32 * kMaxCluster) {
+    set = kOneCluster, grid = 2;
+    while (grid < kMaxCluster && grid * 16 < p->n_slices) grid *= 2;
+  }
+  const bool c16 = p->sell_c16 != nullptr;
+  switch (set) {
+    case kOneBlock:
+      FEMK_TRY((c16 ? launch_pcg<kOneBlock, int16_t>(p, a, grid, s) : launch_pcg<kOneBlock, int32_t>(p, a, grid, s)));
+      break;
+    case kOneCluster:
+      FEMK_TRY((c16 ? launch_pcg<kOneCluster, int16_t>(p, a, grid, s) : launch_pcg<kOneCluster, int32_t>(p, a, grid, s)));
+      break;
+    default:
+      FEMK_TRY((c16 ? launch_pcg<kGrid, int16_t>(p, a, grid, s) : launch_pcg<kGrid, int32_t>(p, a, grid, s)));
+      break;
+  }
+  if (set == kGrid) p->persist_turn ^= 1;
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  if (iters_out) *iters_out = out->iter;
+  if (relres_out) *relres_out = std::sqrt(out->ww) / (std::sqrt(out->bb) + 1e-30);
+  if (pd && out->loop_cycles > 0) {
+    const double ms = 1e-6 * (double)out->loop_ns / (double)out->loop_cycles;  // per cycle
+    for (int k = 0; k < 3; ++k) pd->ms[k] += ms * (double)out->cycles[k];
+    pd->iters += out->iter;
+  }
+  switch (out->status) {
+    case FEMK_BREAKDOWN:
+      set_error("femk_pcg: <p, A p> <= 0 (operator not symmetric positive definite)");
+      return FEMK_BREAKDOWN;
+    case FEMK_NONFINITE:
+      set_error("femk_pcg: non-finite value in a CG reduction");
+      return FEMK_NONFINITE;
+    case FEMK_TIMEOUT:
+      set_error("femk_pcg: a grid-wide wait of the persistent solver gave up");
+      return FEMK_TIMEOUT;
+    default:
+      break;
+  }
+  FEMK_TRY(check_bounds(p, s, "femk_pcg"));
+  if ((dinv ? out->rr : out->gamma) > out->atol2) {
+    set_error("femk_pcg: iteration cap reached above tolerance");
+    return FEMK_NOT_CONVERGED;
+  }
+  return FEMK_OK;
+}
+
+}  // namespace femk

@@ -1,0 +1,204 @@
+// Building blocks of the single-launch (persistent, cooperatively launched) Krylov solvers for systems
+// whose operator stays on the chip: shared memory first, L2 for the rest.
+//
+// Each block owns a run of consecutive 32-row slices of the sliced-ELL operator for the whole solve. As many
+// of its slices as fit are copied into shared memory once (values and columns), the others are read from L2 in
+// every product; the block's parts of the solver vectors live in shared memory too. Only what other blocks
+// gather goes through global memory.
+//
+// Reductions double as barriers over the blocks, and every block ends up with the same bits:
+//  * one block: __syncthreads;
+//  * one cluster of up to 16 blocks: every block stores its partial sums into every other block's shared
+//    memory and crosses the hardware cluster barrier (0.7-1.0 us measured with 2-16 blocks of 512 threads);
+//  * a cooperative grid, one block an SM: every block stores its partials in global memory and adds one to a
+//    counter (release), waits until the counter says that all have (acquire), and adds all partials itself in
+//    block order: 2.1 us, the same for 2 and for 148 blocks. Words that carry the partial and a phase number
+//    together, polled by all blocks, need no second read but took 1.0-5.4 us (the polls of 148 blocks contend),
+//    and 3.0-3.8 us in mailboxes of each reader's own.
+// Only the grid's wait is a spin, and it is bounded: a block that runs out of its clock64 budget gives up and
+// arrives no more, so the others run out too; the kernel returns and the host reports FEMK_TIMEOUT.
+#pragma once
+
+#include <stdint.h>
+
+#include "femk_internal.cuh"
+
+namespace femk {
+
+enum BlockSet { kOneBlock = 0, kOneCluster = 1, kGrid = 2 };
+
+constexpr int kSumValues = 3;    // values a phase can sum at once
+constexpr int kMaxBlocks = 256;  // blocks of a grid
+constexpr int kMaxCluster = 16;
+
+// Global scratch of the grid form: the partials of two alternating phases and two alternating counters. A
+// launch counts on counter[turn] and zeroes the other one, which the next launch uses.
+struct GridWords {
+  double part[2][kSumValues][kMaxBlocks];
+  unsigned int counter[2][32];  // a line apart
+};
+
+__device__ __forceinline__ unsigned int cluster_rank() {
+  unsigned int r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// stores a double at the address that `p` (own shared memory) has in block `rank` of the cluster
+__device__ __forceinline__ void st_cluster(const double* p, unsigned int rank, double v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Sums of NV values a thread over all blocks, the same bits in every thread of every block, and a barrier:
+// what any block wrote before the call is visible to all after it (plain loads included).
+template <int SET, int THREADS>
+struct BlockSum {
+  GridWords* words;
+  int turn;
+  long long limit;
+  int skip;            // testing: the block that never arrives (-1: none)
+  unsigned int phase;  // sums done
+
+  template <int NV>
+  __device__ __forceinline__ bool sum(double (&v)[NV]) {
+    constexpr int W = THREADS / 32;
+    constexpr int NB = SET == kGrid ? kMaxBlocks / 32 : kMaxCluster;
+    __shared__ double red[2][kSumValues][W];
+    __shared__ double tot[2][kSumValues][NB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int par = (int)(phase & 1);
+    const int G = (int)gridDim.x;
+    ++phase;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      v[j] = warp_sum(v[j]);
+      if (lane == 0) red[par][j][warp] = v[j];
+    }
+    __syncthreads();
+    if (SET == kOneBlock) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[j] = warp_sum(lane < W ? red[par][j][lane] : 0.0);
+      return true;
+    }
+    if (SET == kOneCluster) {
+      if (warp == 0) {
+        const unsigned int me = cluster_rank();
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          const double t = warp_sum(lane < W ? red[par][j][lane] : 0.0);
+          if (lane < G) st_cluster(&tot[par][j][me], lane, t);
+        }
+      }
+      cluster_sync();
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[j] = warp_sum(lane < G ? tot[par][j][lane] : 0.0);
+      return true;
+    }
+    int ok = 1;
+    if (warp == 0) {
+      double t[NV];
+#pragma unroll
+      for (int j = 0; j < NV; ++j) t[j] = warp_sum(lane < W ? red[par][j][lane] : 0.0);
+      if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) __stcg(&words->part[par][j][blockIdx.x], t[j]);
+        unsigned int* c = &words->counter[turn][0];
+        const unsigned int want = (unsigned int)G * phase;  // wraps with the counter
+        if (!((int)blockIdx.x == skip))
+          asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
+        const long long t0 = clock64();
+        unsigned int seen, polls = 0;
+        for (;;) {
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(c) : "memory");
+          if ((int)(seen - want) >= 0) break;
+          if ((++polls & 63u) == 0u && clock64() - t0 > limit) {
+            ok = 0;
+            break;
+          }
+        }
+      }
+    }
+    ok = __syncthreads_and(ok);
+    const int groups = (G + 31) >> 5;
+    if (warp < groups) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const double t = warp_sum((int)threadIdx.x < G ? __ldcg(&words->part[par][j][threadIdx.x]) : 0.0);
+        if (lane == 0) tot[par][j][warp] = t;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NV; ++j) v[j] = warp_sum(lane < groups ? tot[par][j][lane] : 0.0);
+    return ok != 0;
+  }
+
+  // before the kernel returns: no block of a cluster leaves while another may store into its shared memory
+  __device__ __forceinline__ void leave() {
+    if (SET == kOneCluster) cluster_sync();
+  }
+};
+
+// One block's share of the operator: slices [s0, s1), of which the first `fit` are in shared memory.
+template <typename IDX>
+struct BlockMatrix {
+  int32_t s0, ns, fit;   // first slice, slices, slices held in shared memory
+  const int32_t* off;    // shared: ns + 1 entry offsets from the block's first entry
+  const double* sv;      // shared values and columns of the first `fit` slices
+  const IDX* sc;
+  const double* gv;      // the block's entries in global memory
+  const IDX* gc;
+};
+
+// First slice of block b: the blocks get equal shares of the work, counted as the stored entries plus 8 a row
+// for the vector updates (rows may be of unequal length). Every thread gets the same answer.
+constexpr int kSliceWork = 8 * 32;
+__device__ __forceinline__ int32_t block_slice(const int64_t* __restrict__ sptr, int32_t nslices, int b, int blocks) {
+  const int64_t want = (__ldg(sptr + nslices) + (int64_t)kSliceWork * nslices) * b / blocks;
+  int32_t lo = 0, hi = nslices;
+  while (lo < hi) {
+    const int32_t mid = (lo + hi) >> 1;
+    if (__ldg(sptr + mid) + (int64_t)kSliceWork * mid < want)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// Row sum of one lane's row, entries 32 apart, up to B loads in flight; g(column) is the operand. The entries
+// add in k order, as everywhere else.
+template <int B, bool SHARED, typename IDX, typename G>
+__device__ __forceinline__ double lane_row(const double* vb, const IDX* cb, int32_t w, int32_t row, const G& g) {
+  double acc = 0.0;
+  for (int32_t k0 = 0; k0 < w; k0 += B) {
+    double v[B];
+    int32_t c[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int32_t j = (k0 + u) * 32;
+      const bool ok = k0 + u < w;
+      c[u] = ok ? (int32_t)(SHARED ? cb[j] : __ldg(cb + j)) : 0;
+      v[u] = ok ? (SHARED ? vb[j] : __ldg(vb + j)) : 0.0;
+      if (sizeof(IDX) == 2) c[u] += row;
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (k0 + u < w) acc += v[u] * g(c[u]);
+  }
+  return acc;
+}
+
+template <int B, typename IDX, typename G>
+__device__ __forceinline__ double block_row(const BlockMatrix<IDX>& m, int32_t s, int lane, int32_t row, const G& g) {
+  const int32_t o = m.off[s], w = (m.off[s + 1] - o) >> 5;
+  if (s < m.fit) return lane_row<B, true>(m.sv + o + lane, m.sc + o + lane, w, row, g);
+  return lane_row<B, false>(m.gv + o + lane, m.gc + o + lane, w, row, g);
+}
+
+}  // namespace femk

@@ -839,10 +839,11 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
                   p->sell_ptr, p->sell_cols, p->sell_c16,  p->sell_vals, p->sell_vals32,
                   p->bar,      p->batch_ws,  p->bicg_ws,   p->bicg_state, p->sell_cuptr, p->sell_cu,
                   p->coef_tmp, p->theta_ws, p->cmp_ws, p->gm_ws, p->dev_err, p->astr_ptr, p->astr_elem,
-                  p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn};
+                  p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn, p->persist_ws};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (p->state_host) cudaFreeHost(p->state_host);
+  if (p->persist_out) cudaFreeHost(p->persist_out);
   if (p->cg_exec) cudaGraphExecDestroy(p->cg_exec);
   for (cudaEvent_t e : p->cg_ev)
     if (e) cudaEventDestroy(e);
@@ -927,6 +928,9 @@ int apply_options(femk_plan* p, const femk_plan_options& o) {
   p->sell_batch = o.sell_batch;
   p->vec_blocks = o.vec_blocks;
   p->cg_split = o.split_updates;
+  // options that choose among the chunked solvers' kernels keep the plan on those
+  p->persist_ok = o.solver_layout == 1 && o.cols16 == 1 && o.l2_hints == -1 && o.ring64 == -1 &&
+                  o.sell_batch == 16 && o.vec_blocks == 0 && o.split_updates == 1;
   p->skip_arrival = o.test_skip_arrival;
   p->mixed_delta2 = o.mixed_delta2;
   int khz = 0;
