@@ -57,6 +57,8 @@ Vecs vecs_of(const femk_plan* p) {
   return {w, w + vs, w + 2 * vs, w + 3 * vs, w + 4 * vs, w + 5 * vs, w + 6 * vs, w + 7 * vs};
 }
 
+static_assert(sizeof(BicgResult) <= 2 * sizeof(BicgState), "the pinned mirrors hold either");
+
 enum Kind { kInitR = 0, kQ = 1, kT = 2, kResid = 3 };
 
 // Epilogue of each SpMV kind (row, (A v)[row]):
@@ -385,6 +387,19 @@ int solve_prepared(femk_plan* p, const double* b, double* x, const double* dinv,
   const Vecs v = vecs_of(p);
   BicgState* st = (BicgState*)p->bicg_state;
   BicgState* host = (BicgState*)p->bicg_host;
+  if (bicg_persist_fits(p)) {
+    BicgResult* r = (BicgResult*)p->bicg_host;
+    FEMK_TRY(bicg_persist(p, b, x, dinv, (double*)p->bicg_ws, tol, atol, maxiter, ws, r));
+    *out = BicgState{};
+    out->rr = r->rr;
+    out->ss = r->ss;
+    out->atol2 = r->atol2;
+    out->bb = r->bb;
+    out->k = r->k;
+    out->iters = r->iters;
+    out->status = r->status;
+    return FEMK_OK;
+  }
   k_bicg_setup<<<counted_launch() + 1, 1, 0, ws>>>(st, tol * tol, atol * atol, maxiter);
   FEMK_TRY(launch_spmv<kInitR>(p, x, b, v, st, ws));
   const bool graph = p->cg_graph != 0;

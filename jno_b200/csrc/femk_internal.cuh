@@ -303,6 +303,15 @@ bool pcg_persist_fits(const femk_plan* p);
 int pcg_persist(const femk_plan* p, const double* vals, const double* b, double* x, const double* dinv, double tol,
                 double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s);
 
+// BiCGStab as one persistent launch on the plan's prepared operator; ws: 8 vectors of vstride doubles; *out: pinned.
+struct BicgResult {
+  double rr, ss, atol2, bb;  // final <r, r>, <b - A x, b - A x>, stop bound, <b, b>
+  int32_t k, iters, status;
+};
+bool bicg_persist_fits(const femk_plan* p);
+int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, double* ws, double tol, double atol,
+                 int32_t maxiter, cudaStream_t s, BicgResult* out);
+
 // Nodal P1 coefficient modes become a per-element coefficient (plan-owned f64[ntet], computed on
 // stream s) read as FEMK_COEF_LINEAR; other modes pass through unchanged.
 int resolve_coef(const femk_plan* p, const double* param, int mode, cudaStream_t s, const double** param_out,

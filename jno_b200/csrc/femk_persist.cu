@@ -1,4 +1,5 @@
-// Jacobi-PCG as one persistent launch, for systems whose operator stays on the chip (femk_persist.cuh).
+// Jacobi-PCG and BiCGStab as one persistent launch, for systems whose operator stays on the chip
+// (femk_persist.cuh).
 //
 // The chunked solver (femk_cg.cu) runs three kernels an iteration, each with its launch gap, its ramp and a
 // last-block reduction: at P1 32^3 (35,937 rows, 5.3 MB of operator) that takes 17.8 us an iteration, 13.3 us of it
@@ -47,7 +48,7 @@ struct PcgArgs {
   double* x;
   const double* dinv;
   double2* zp;      // {z, p} of every row: what other blocks gather
-  double* work;     // r, p, q, D^-1 (vstride apart) of blocks whose rows do not fit in shared memory
+  double* work;     // r, p, q (vstride apart) of blocks whose rows do not fit in shared memory
   int64_t vstride;
   GridWords* words;
   int32_t turn, skip;
@@ -68,7 +69,6 @@ __device__ __forceinline__ long long global_ns() {
 template <int SET, typename IDX>
 __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   extern __shared__ __align__(16) unsigned char ps_smem[];
-  __shared__ int32_t fit_s;
   constexpr int W = kPT / 32;
   constexpr bool ONE = SET == kOneBlock;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -77,7 +77,6 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   BlockMatrix<IDX> m;
   m.s0 = block_slice(a.sptr, nsl, bid, G);
   m.ns = block_slice(a.sptr, nsl, bid + 1, G) - m.s0;
-  const int64_t e0 = __ldg(a.sptr + m.s0);
   const int32_t r0 = m.s0 * 32, nr = m.ns * 32;
   // shared memory: slice offsets, the block's x, r, p, q, D^-1 (and the pairs, when one block owns all), slices
   int32_t* off = reinterpret_cast<int32_t*>(ps_smem);
@@ -88,31 +87,11 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   double* rs = vin ? vec + nr : a.work + r0;
   double* ps = vin ? vec + 2 * nr : a.work + a.vstride + r0;
   double* qs = vin ? vec + 3 * nr : a.work + 2 * a.vstride + r0;
-  double* ds = vin ? vec + 4 * nr : a.work + 3 * a.vstride + r0;
+  const double* ds = vin ? vec + 4 * nr : a.dinv + r0;  // not read without a preconditioner
   double2* zps = reinterpret_cast<double2*>(vec + 5 * nr);
   unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
-  for (int32_t s = threadIdx.x; s <= m.ns; s += kPT) off[s] = (int32_t)(__ldg(a.sptr + m.s0 + s) - e0);
-  if (threadIdx.x == 0) fit_s = 0;
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
-  __syncthreads();
-  const int32_t room = a.smem - (int32_t)(mat - ps_smem);
-  for (int32_t s = threadIdx.x; s < m.ns; s += kPT)
-    if ((int64_t)off[s + 1] * (8 + (int)sizeof(IDX)) <= room) atomicMax(&fit_s, s + 1);
-  __syncthreads();
-  m.fit = fit_s;
-  m.off = off;
-  m.gv = a.svals + e0;
-  m.gc = reinterpret_cast<const IDX*>(a.cols) + e0;
-  const int32_t held = off[m.fit];
-  double* sv = reinterpret_cast<double*>(mat);
-  IDX* sc = reinterpret_cast<IDX*>(sv + held);
-  for (int32_t k = threadIdx.x; k < held; k += kPT) {
-    sv[k] = __ldg(m.gv + k);
-    sc[k] = __ldg(m.gc + k);
-  }
-  m.sv = sv;
-  m.sc = sc;
-  __syncthreads();
+  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, off, mat, a.smem - (int32_t)(mat - ps_smem));
   BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
   // r = b - A x0, z = D^-1 r
   // gathers of x and of the pairs, range-checked in the bounds-checked build
@@ -127,7 +106,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
     const double di = a.dinv ? __ldg(a.dinv + row) : 1.0;
     const double zi = a.dinv ? di * ri : ri;
     rs[i] = ri;
-    ds[i] = di;
+    if (vin) vec[4 * nr + i] = di;
     ps[i] = 0.0;
     if (ONE)
       zps[i] = make_double2(zi, 0.0);
@@ -247,6 +226,181 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   }
 }
 
+struct BicgArgs {
+  const int64_t* sptr;
+  const void* cols;
+  const double* svals;
+  int64_t n, nslices;
+  const double* b;
+  double* x;
+  const double* dinv;
+  double *phat, *shat;  // what other blocks gather
+  double* work;         // r, rhat, p, q, s, t (vstride apart) of blocks whose rows do not fit in shared memory
+  int64_t vstride;
+  GridWords* words;
+  int32_t turn, skip;
+  long long limit;
+  int32_t smem;
+  double tol2, atol2;
+  int32_t maxiter;
+  BicgResult* out;  // pinned host memory
+  int* err;
+};
+
+// BiCGStab with the steps, operands and stop rule of femk_bicgstab.cu: per iteration the direction (a barrier, the
+// others gather phat), q = A phat with <rhat, q>, s and shat with <s, s>, t = A shat with <t, s> and <t, t>, and
+// the x and r updates with <r, r> and <rhat, r>: four sums and one barrier. The chunked solver's five kernels took
+// 36.5 us an iteration at 2-D P2 131x118 (62,331 rows, vertices in no order), 19.4 us here, 10.5 of them in the five
+// waits; at P1 44x40x47 a Crank-Nicolson march of 12 steps went from 14.6 to 6.9 ms.
+template <int SET, typename IDX>
+__global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
+  extern __shared__ __align__(16) unsigned char ps_smem[];
+  constexpr int W = kPT / 32;
+  constexpr bool ONE = SET == kOneBlock;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t nsl = (int32_t)a.nslices;
+  const int G = (int)gridDim.x, bid = (int)blockIdx.x;
+  BlockMatrix<IDX> m;
+  m.s0 = block_slice(a.sptr, nsl, bid, G);
+  m.ns = block_slice(a.sptr, nsl, bid + 1, G) - m.s0;
+  const int32_t r0 = m.s0 * 32, nr = m.ns * 32;
+  // shared memory: slice offsets, the block's x, r, rhat, p, q, s, t, D^-1 (and phat, shat of one block), slices
+  int32_t* off = reinterpret_cast<int32_t*>(ps_smem);
+  const int32_t head = (4 * (m.ns + 1) + 15) & ~15;
+  const bool vin = ONE || head + 64 * nr <= a.smem;
+  double* vec = reinterpret_cast<double*>(ps_smem + head);
+  auto slot = [&](int k) { return vin ? vec + (k + 1) * nr : a.work + k * a.vstride + r0; };
+  double* xs = vin ? vec : a.x + r0;
+  double *rs = slot(0), *hs = slot(1), *ps = slot(2), *qs = slot(3), *ss = slot(4), *ts = slot(5);
+  const double* ds = vin ? vec + 7 * nr : a.dinv + r0;  // not read without a preconditioner
+  double* phat = ONE ? vec + 8 * nr : a.phat;
+  double* shat = ONE ? vec + 9 * nr : a.shat;
+  unsigned char* mat = reinterpret_cast<unsigned char*>(vec + (ONE ? 10 * nr : (vin ? 8 * nr : 0)));
+  if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
+  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, off, mat, a.smem - (int32_t)(mat - ps_smem));
+  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
+  auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
+  // body(local row, row) for every row of the block that this thread owns
+  auto rows = [&](auto&& body) {
+    for (int32_t s = warp; s < m.ns; s += W) {
+      const int32_t i = s * 32 + lane, row = r0 + i;
+      if (row < a.n) body(s, i, row);
+    }
+  };
+  double acc[2] = {0.0, 0.0};
+  rows([&](int32_t s, int32_t i, int32_t row) {
+    const double bi = __ldg(a.b + row);
+    const double ri = bi - block_row<16>(m, s, lane, row, xat);
+    rs[i] = ri;
+    hs[i] = ri;
+    ps[i] = ri;
+    qs[i] = ri;
+    if (vin) {
+      xs[i] = a.x[row];
+      vec[7 * nr + i] = a.dinv ? __ldg(a.dinv + row) : 1.0;
+    }
+    acc[0] += ri * ri;
+    acc[1] += bi * bi;
+  });
+  bool live = grid.template sum<2>(acc);
+  double rr = acc[0], rho_n = acc[0], bb = acc[1];
+  const double atol2 = fmax(a.tol2 * bb, a.atol2);
+  double rho = 1.0, alpha = 1.0, omega = 1.0;
+  int32_t k = 0, iters = 0, status = isfinite(rr) && isfinite(bb) ? FEMK_OK : FEMK_NONFINITE;
+  bool done = status != FEMK_OK || !(rr > atol2) || a.maxiter <= 0;
+  while (live && !done) {
+    const double beta = rho_n / rho * alpha / omega;
+    rows([&](int32_t, int32_t i, int32_t row) {
+      const double pi = rs[i] + beta * (ps[i] - omega * qs[i]);
+      ps[i] = pi;
+      phat[row] = a.dinv ? ds[i] * pi : pi;
+    });
+    if (!(live = grid.barrier())) break;
+    double v1[1] = {0.0};
+    rows([&](int32_t s, int32_t i, int32_t row) {
+      const double qi = block_row<16>(m, s, lane, row, [&](int32_t j) {
+        return FEMK_IN_BOUNDS(j, a.n, a.err) ? phat[j] : 0.0;
+      });
+      qs[i] = qi;
+      v1[0] += hs[i] * qi;
+    });
+    if (!(live = grid.template sum<1>(v1))) break;
+    alpha = rho_n / v1[0];
+    v1[0] = 0.0;
+    rows([&](int32_t, int32_t i, int32_t row) {
+      const double si = rs[i] - alpha * qs[i];
+      ss[i] = si;
+      shat[row] = a.dinv ? ds[i] * si : si;
+      v1[0] += si * si;
+    });
+    if (!(live = grid.template sum<1>(v1))) break;
+    const bool early = v1[0] < atol2;
+    double v2[2] = {0.0, 0.0};
+    rows([&](int32_t s, int32_t i, int32_t row) {
+      const double ti = block_row<16>(m, s, lane, row, [&](int32_t j) {
+        return FEMK_IN_BOUNDS(j, a.n, a.err) ? shat[j] : 0.0;
+      });
+      ts[i] = ti;
+      v2[0] += ti * ss[i];
+      v2[1] += ti * ti;
+    });
+    if (!(live = grid.template sum<2>(v2))) break;
+    omega = v2[0] / v2[1];
+    v2[0] = v2[1] = 0.0;
+    rows([&](int32_t, int32_t i, int32_t) {
+      const double si = ss[i];
+      const double ph = a.dinv ? ds[i] * ps[i] : ps[i];
+      double ri;
+      if (early) {
+        xs[i] = xs[i] + alpha * ph;
+        ri = si;
+      } else {
+        const double sh = a.dinv ? ds[i] * si : si;
+        xs[i] = xs[i] + (alpha * ph + omega * sh);
+        ri = si - omega * ts[i];
+      }
+      rs[i] = ri;
+      v2[0] += ri * ri;
+      v2[1] += hs[i] * ri;
+    });
+    if (!(live = grid.template sum<2>(v2))) break;
+    ++iters;
+    k = rho_n == 0.0 ? -10 : (omega == 0.0 || alpha == 0.0 ? -11 : k + 1);
+    rho = rho_n;
+    rho_n = v2[1];
+    rr = v2[0];
+    if (!isfinite(rr) || !isfinite(rho_n)) {
+      status = FEMK_NONFINITE;
+      done = true;
+    } else {
+      done = !(rr > atol2) || k >= a.maxiter || k < 0;
+    }
+  }
+  if (vin) rows([&](int32_t, int32_t i, int32_t row) { a.x[row] = xs[i]; });
+  double w2[1] = {0.0};  // the true residual of the returned x
+  if (live) live = grid.barrier();
+  if (live) {
+    rows([&](int32_t s, int32_t, int32_t row) {
+      const double wi = __ldg(a.b + row) - block_row<16>(m, s, lane, row, xat);
+      w2[0] += wi * wi;
+    });
+    live = grid.template sum<1>(w2);
+  }
+  grid.leave();
+  if (bid == 0 && threadIdx.x == 0) {
+    a.out->rr = rr;
+    a.out->ss = w2[0];
+    a.out->atol2 = atol2;
+    a.out->bb = bb;
+    a.out->k = k;
+    a.out->iters = iters;
+    a.out->status = live ? status : FEMK_TIMEOUT;
+  }
+}
+
+// Bytes of the sliced-ELL operator: what every iteration reads.
+int64_t operator_bytes(const femk_plan* p) { return p->sell_nnz * (p->sell_c16 ? 10 : 12); }
+
 // One launch of a persistent kernel: co-resident blocks (a cluster, or a cooperative grid).
 template <typename Args>
 int launch_set(const femk_plan* p, void (*kern)(Args), int set, int grid, const Args& a, cudaStream_t s) {
@@ -286,20 +440,65 @@ int prepare_kernel(void (*kern)(Args), int set, int device, std::atomic<uint64_t
 }
 
 template <int SET, typename IDX>
-int launch_pcg(const femk_plan* p, const PcgArgs& a, int grid, cudaStream_t s) {
+struct PcgKernel {
+  static constexpr auto fn = k_pcg_persist<SET, IDX>;
+};
+template <int SET, typename IDX>
+struct BicgKernel {
+  static constexpr auto fn = k_bicg_persist<SET, IDX>;
+};
+
+template <template <int, typename> class K, int SET, typename IDX, typename Args>
+int launch_kernel(const femk_plan* p, const Args& a, int grid, cudaStream_t s) {
   static std::atomic<uint64_t> ready{0};
-  FEMK_TRY(prepare_kernel(k_pcg_persist<SET, IDX>, SET, p->device, ready));
-  return launch_set(p, k_pcg_persist<SET, IDX>, SET, grid, a, s);
+  FEMK_TRY(prepare_kernel(K<SET, IDX>::fn, SET, p->device, ready));
+  return launch_set(p, K<SET, IDX>::fn, SET, grid, a, s);
 }
 
-// Bytes of the sliced-ELL operator: what every iteration reads.
-int64_t operator_bytes(const femk_plan* p) { return p->sell_nnz * (p->sell_c16 ? 10 : 12); }
+template <template <int, typename> class K, int SET, typename Args>
+int launch_columns(const femk_plan* p, const Args& a, int grid, cudaStream_t s) {
+  if (p->sell_c16) return launch_kernel<K, SET, int16_t>(p, a, grid, s);
+  return launch_kernel<K, SET, int32_t>(p, a, grid, s);
+}
+
+// The launch of kernel K for the plan. One block, with no wait for others, when all of it fits one SM
+// (one_row: bytes of vectors a row takes there). Then one cluster of up to 16 blocks: its barrier is twice as fast
+// as the grid's, until 16 SMs take longer over the rows than that gains (CG, us an iteration, cluster against
+// grid: 2-D P1 100^2, 319 slices, 4.1 / 5.7; P1 20x22x24, 378 slices, 5.8 / 7.0; 2-D P2 60^2, 458 slices, 6.3 /
+// 6.9; 2-D P2 70^2, 622 slices, 7.0 / 6.7; P1 28^3, 763 slices, 8.4 / 7.2). Then a grid of 16 slices a block, a
+// slice a warp, at most a block an SM (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148).
+template <template <int, typename> class K, typename Args>
+int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
+  a.sptr = p->sell_ptr;
+  a.cols = p->sell_c16 ? (const void*)p->sell_c16 : (const void*)p->sell_cols;
+  a.svals = p->sell_vals;
+  a.n = p->n;
+  a.nslices = p->n_slices;
+  a.vstride = p->vstride;
+  a.words = (GridWords*)p->persist_words;
+  a.turn = p->persist_turn;
+  a.skip = p->skip_arrival;
+  a.limit = p->barrier_spin;
+  a.smem = p->sell_c16 ? kPersistSmem : kPersistSmemWide;
+  a.err = p->dev_err;
+  const int64_t one = 4 * (p->n_slices + 1) + 16 + p->n_slices * 32 * one_row + operator_bytes(p);
+  if (one <= a.smem) return launch_columns<K, kOneBlock>(p, a, 1, s);
+  if (p->n_slices <= 32 * kMaxCluster) {
+    int grid = 2;
+    while (grid < kMaxCluster && grid * 16 < p->n_slices) grid *= 2;
+    return launch_columns<K, kOneCluster>(p, a, grid, s);
+  }
+  const int grid = (int)std::min<int64_t>(std::min(p->n_sm, kMaxBlocks), (p->n_slices + 15) / 16);
+  FEMK_TRY((launch_columns<K, kGrid>(p, a, grid, s)));
+  p->persist_turn ^= 1;
+  return FEMK_OK;
+}
 
 // One allocation for all of the solver's global memory: the pairs, the vectors of blocks whose rows do not fit
 // in shared memory, and the grid's words.
 int ensure_persist(femk_plan* p) {
   if (!p->persist_ws) {
-    const size_t vec = sizeof(double) * 6 * (size_t)p->vstride;
+    const size_t vec = sizeof(double) * 5 * (size_t)p->vstride;
     char* ws = nullptr;
     FEMK_CUDA_TRY(cudaMalloc(&ws, vec + sizeof(GridWords)));
     p->persist_ws = ws;
@@ -329,22 +528,11 @@ int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double
   PersistOut* out = (PersistOut*)p->persist_out;
   out->status = FEMK_TIMEOUT;
   PcgArgs a{};
-  a.sptr = p->sell_ptr;
-  a.cols = p->sell_c16 ? (const void*)p->sell_c16 : (const void*)p->sell_cols;
-  a.svals = p->sell_vals;
-  a.n = p->n;
-  a.nslices = p->n_slices;
   a.b = b;
   a.x = x;
   a.dinv = dinv;
   a.zp = (double2*)p->persist_ws;
   a.work = (double*)p->persist_ws + 2 * p->vstride;
-  a.vstride = p->vstride;
-  a.words = (GridWords*)p->persist_words;
-  a.turn = p->persist_turn;
-  a.skip = p->skip_arrival;
-  a.limit = p->barrier_spin;
-  a.smem = p->sell_c16 ? kPersistSmem : kPersistSmemWide;
   a.tol2 = tol * tol;
   a.atol2 = atol * atol;
   a.maxiter = maxiter;
@@ -352,33 +540,7 @@ int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double
   ProfData* pd = (ProfData*)p->prof;
   a.timed = pd != nullptr;
   a.out = out;
-  a.err = p->dev_err;
-  // One block, with no wait for others, when all of it fits one SM. Then one cluster of up to 16 blocks: its
-  // barrier is twice as fast as the grid's, until 16 SMs take longer over the rows than that gains (us an
-  // iteration, cluster against grid: 2-D P1 100^2, 319 slices, 4.1 / 5.7; P1 20x22x24, 378 slices, 5.8 / 7.0;
-  // 2-D P2 60^2, 458 slices, 6.3 / 6.9; 2-D P2 70^2, 622 slices, 7.0 / 6.7; P1 28^3, 763 slices, 8.4 / 7.2).
-  // 16 slices a block: a slice a warp (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148).
-  const int64_t one = 4 * (p->n_slices + 1) + 16 + p->n_slices * 32 * 56 + operator_bytes(p);
-  int set = kGrid, grid = (int)std::min<int64_t>(std::min(p->n_sm, kMaxBlocks), (p->n_slices + 15) / 16);
-  if (one <= a.smem) {
-    set = kOneBlock, grid = 1;
-  } else if (p->n_slices <= 32 * kMaxCluster) {
-    set = kOneCluster, grid = 2;
-    while (grid < kMaxCluster && grid * 16 < p->n_slices) grid *= 2;
-  }
-  const bool c16 = p->sell_c16 != nullptr;
-  switch (set) {
-    case kOneBlock:
-      FEMK_TRY((c16 ? launch_pcg<kOneBlock, int16_t>(p, a, grid, s) : launch_pcg<kOneBlock, int32_t>(p, a, grid, s)));
-      break;
-    case kOneCluster:
-      FEMK_TRY((c16 ? launch_pcg<kOneCluster, int16_t>(p, a, grid, s) : launch_pcg<kOneCluster, int32_t>(p, a, grid, s)));
-      break;
-    default:
-      FEMK_TRY((c16 ? launch_pcg<kGrid, int16_t>(p, a, grid, s) : launch_pcg<kGrid, int32_t>(p, a, grid, s)));
-      break;
-  }
-  if (set == kGrid) p->persist_turn ^= 1;
+  FEMK_TRY(launch_persist<PcgKernel>(p, a, 56, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   if (iters_out) *iters_out = out->iter;
   if (relres_out) *relres_out = std::sqrt(out->ww) / (std::sqrt(out->bb) + 1e-30);
@@ -405,6 +567,30 @@ int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double
     set_error("femk_pcg: iteration cap reached above tolerance");
     return FEMK_NOT_CONVERGED;
   }
+  return FEMK_OK;
+}
+
+bool bicg_persist_fits(const femk_plan* p) {
+  return p->persist_ok && p->coop && operator_bytes(p) <= 80000000;
+}
+
+int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, double* ws, double tol, double atol,
+                 int32_t maxiter, cudaStream_t s, BicgResult* out) {
+  FEMK_TRY(ensure_persist(p));
+  out->status = FEMK_TIMEOUT;
+  BicgArgs a{};
+  a.b = b;
+  a.x = x;
+  a.dinv = dinv;
+  a.phat = ws;
+  a.shat = ws + p->vstride;
+  a.work = ws + 2 * p->vstride;
+  a.tol2 = tol * tol;
+  a.atol2 = atol * atol;
+  a.maxiter = maxiter;
+  a.out = out;
+  FEMK_TRY(launch_persist<BicgKernel>(p, a, 80, s));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   return FEMK_OK;
 }
 

@@ -64,6 +64,20 @@ struct BlockSum {
   int skip;            // testing: the block that never arrives (-1: none)
   unsigned int phase;  // sums done
 
+  // one thread of the block: its writes and, after a __syncthreads, its block's are released, the others' acquired
+  __device__ __forceinline__ int arrive() {
+    unsigned int* c = &words->counter[turn][0];
+    const unsigned int want = gridDim.x * phase;  // wraps with the counter
+    if ((int)blockIdx.x != skip) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
+    const long long t0 = clock64();
+    unsigned int seen, polls = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(c) : "memory");
+      if ((int)(seen - want) >= 0) return 1;
+      if ((++polls & 63u) == 0u && clock64() - t0 > limit) return 0;
+    }
+  }
+
   template <int NV>
   __device__ __forceinline__ bool sum(double (&v)[NV]) {
     constexpr int W = THREADS / 32;
@@ -107,20 +121,7 @@ struct BlockSum {
       if (lane == 0) {
 #pragma unroll
         for (int j = 0; j < NV; ++j) __stcg(&words->part[par][j][blockIdx.x], t[j]);
-        unsigned int* c = &words->counter[turn][0];
-        const unsigned int want = (unsigned int)G * phase;  // wraps with the counter
-        if (!((int)blockIdx.x == skip))
-          asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
-        const long long t0 = clock64();
-        unsigned int seen, polls = 0;
-        for (;;) {
-          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(c) : "memory");
-          if ((int)(seen - want) >= 0) break;
-          if ((++polls & 63u) == 0u && clock64() - t0 > limit) {
-            ok = 0;
-            break;
-          }
-        }
+        ok = arrive();
       }
     }
     ok = __syncthreads_and(ok);
@@ -136,6 +137,21 @@ struct BlockSum {
 #pragma unroll
     for (int j = 0; j < NV; ++j) v[j] = warp_sum(lane < groups ? tot[par][j][lane] : 0.0);
     return ok != 0;
+  }
+
+  // the barrier alone: what any block wrote before it is visible to all after it
+  __device__ __forceinline__ bool barrier() {
+    if (SET != kGrid) {
+      if (SET == kOneBlock)
+        __syncthreads();
+      else
+        cluster_sync();
+      return true;
+    }
+    ++phase;
+    __syncthreads();
+    const int ok = threadIdx.x == 0 ? arrive() : 1;
+    return __syncthreads_and(ok) != 0;
   }
 
   // before the kernel returns: no block of a cluster leaves while another may store into its shared memory
@@ -192,6 +208,35 @@ __device__ __forceinline__ double lane_row(const double* vb, const IDX* cb, int3
       if (k0 + u < w) acc += v[u] * g(c[u]);
   }
   return acc;
+}
+
+// The block's share, its first slices copied into `mat` (room bytes of shared memory; off: ns + 1 words of shared
+// memory). The whole block calls this.
+template <int THREADS, typename IDX>
+__device__ __forceinline__ void hold_slices(BlockMatrix<IDX>& m, const int64_t* __restrict__ sptr, const void* cols,
+                                            const double* svals, int32_t* off, unsigned char* mat, int32_t room) {
+  __shared__ int32_t fit_s;
+  const int64_t e0 = __ldg(sptr + m.s0);
+  for (int32_t s = threadIdx.x; s <= m.ns; s += THREADS) off[s] = (int32_t)(__ldg(sptr + m.s0 + s) - e0);
+  if (threadIdx.x == 0) fit_s = 0;
+  __syncthreads();
+  for (int32_t s = threadIdx.x; s < m.ns; s += THREADS)
+    if ((int64_t)off[s + 1] * (8 + (int)sizeof(IDX)) <= room) atomicMax(&fit_s, s + 1);
+  __syncthreads();
+  m.fit = fit_s;
+  m.off = off;
+  m.gv = svals + e0;
+  m.gc = reinterpret_cast<const IDX*>(cols) + e0;
+  const int32_t held = off[m.fit];
+  double* sv = reinterpret_cast<double*>(mat);
+  IDX* sc = reinterpret_cast<IDX*>(sv + held);
+  for (int32_t k = threadIdx.x; k < held; k += THREADS) {
+    sv[k] = __ldg(m.gv + k);
+    sc[k] = __ldg(m.gc + k);
+  }
+  m.sv = sv;
+  m.sc = sc;
+  __syncthreads();
 }
 
 template <int B, typename IDX, typename G>

@@ -124,3 +124,58 @@ def test_a_grid_wait_that_runs_out_is_a_status():
             plan.pcg(vals, b, None, inv)
     x, it, rel, st = FemPlan(pts, cells, 1).pcg(vals, b, None, inv)
     assert st == 0 and rel <= 2e-8
+
+
+@pytest.mark.parametrize("dim,n,order,shuffled", SYSTEMS)
+@pytest.mark.parametrize("precond", [True, False])
+def test_bicgstab_matches_the_chunked_solver(dim, n, order, shuffled, precond):
+    """BiCGStab's count moves with the order of its sums, so the solutions are held to each other: both meet a
+    relative residual of 1e-11, which bounds their distance by twice that times the condition number (below 1e5
+    here, without a preconditioner too): 2e-6."""
+    one, chunked, vals, b, inv = _plans(dim, n, order, shuffled)
+    inv = inv if precond else None
+    g = torch.Generator(device="cuda").manual_seed(2)
+    start = torch.randn(one.n, dtype=torch.float64, device="cuda", generator=g) * b.abs().max()
+    for x0 in (torch.zeros_like(b), start):
+        x, it, rel, st = one.bicgstab(vals, b, x0.clone(), inv, tol=1e-11)
+        y, _, _, sty = chunked.bicgstab(vals, b, x0.clone(), inv, tol=1e-11)
+        assert st == sty == 0
+        assert abs(rel - (torch.linalg.norm(b - one.spmv(vals, x)) / torch.linalg.norm(b)).item()) <= 1e-12
+        assert (torch.linalg.norm(x - y) / torch.linalg.norm(y)).item() <= 2e-6
+        again, it2, rel2, _ = one.bicgstab(vals, b, x0.clone(), inv, tol=1e-11)
+        assert it2 == it and rel2 == rel and torch.equal(again, x)
+
+
+@pytest.mark.parametrize("dim,n,order", [(3, (3, 3, 3), 1), (3, (14, 14, 14), 1), (3, (33, 35, 31), 1)])
+def test_bicgstab_status_paths_match_the_chunked_solver(dim, n, order):
+    from jno_b200 import _lib
+
+    one, chunked, vals, b, inv = _plans(dim, n, order, False)
+    for maxiter in (0, 1, 3):
+        got = [p.bicgstab(vals, b, None, inv, 1e-12, maxiter=maxiter) for p in (one, chunked)]
+        assert got[0][3] == got[1][3] and got[0][1] == got[1][1] == maxiter
+        assert torch.allclose(got[0][0], got[1][0], rtol=0, atol=1e-11 * max(1e-300, got[1][0].abs().max().item()))
+    bad = b.clone()
+    bad[one.n // 2] = float("nan")
+    for p in (one, chunked):
+        with pytest.raises(_lib.FemkError, match="non-finite"):
+            p.bicgstab(vals, bad, None, inv)
+
+
+@pytest.mark.parametrize("dim,n,order", [(2, (19, 23), 1), (3, (14, 13, 15), 1), (3, (33, 35, 31), 1), (3, (9, 8, 7), 2)])
+def test_theta_march_matches_the_chunked_solver(dim, n, order):
+    """Every step to 1e-12 of its right-hand side; the step systems' condition numbers are below 1e3 at this dt:
+    1e-8 of the state's size covers the steps together."""
+    from jno_b200.plan import FemPlan
+
+    pts, cells = _mesh(dim, n, order, False)
+    logk = torch.as_tensor(om.logk_field(len(cells), 1016), device="cuda")
+    states = []
+    for options in (None, {"ring64": 14}):
+        plan = FemPlan(pts, cells, order, options=options)
+        S, R, q = plan.assemble_theta(logk, theta=0.5, dt=1e-3)
+        u = plan.lumped_mass() / plan.lumped_mass().abs().max()
+        u, _, worst = plan.theta_march(S, R, q, u, 5, tol=1e-12)
+        assert worst <= 1e-11
+        states.append(u)
+    assert (states[0] - states[1]).abs().max() <= 1e-8 * states[1].abs().max()
