@@ -148,8 +148,7 @@ __global__ void __launch_bounds__(kThreads) k_bicg_sell(const int64_t* __restric
     if (row >= n) continue;
     const int64_t b0 = __ldg(sptr + sl);
     const int32_t w = (int32_t)((__ldg(sptr + sl + 1) - b0) >> 5);
-    epi(row, sell_row<double, IDX, 16>(vals + b0 + lane, cols + b0 + lane, w, (int32_t)row,
-                                                        GatherX<double>{x}));
+    epi(row, sell_row<double, IDX, 16>(vals + b0 + lane, cols + b0 + lane, w, (int32_t)row, GatherX<double>{x}));
   }
   finish<KIND, kThreads>(st, acc, partials);
 }
@@ -173,6 +172,27 @@ __global__ void __launch_bounds__(kBulkW * 32) k_bicg_bulk(const int64_t* __rest
       FEMK_TIMEOUT, cptr);
   if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
   finish<KIND, kBulkW * 32>(st, acc, partials);
+}
+
+// The same on slices of any width with 32-bit column tables.
+template <int KIND>
+__global__ void __launch_bounds__(kWideWarps * 32, 8) k_bicg_wide(const int64_t* __restrict__ sptr,
+                                                              const double* __restrict__ vals,
+                                                              const int64_t* __restrict__ tptr,
+                                                              const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n,
+                                                              int64_t nslices, const double* __restrict__ x,
+                                                              const double* __restrict__ b, Vecs v,
+                                                              double* __restrict__ partials, BicgState* st) {
+  extern __shared__ __align__(128) unsigned char bulk_smem[];
+  if (kind_skips<KIND>(st)) return;
+  const int wib = threadIdx.x >> 5;
+  double acc[Epi<KIND>::NV] = {};
+  const bool ok = sell_wide_rows<double>(bulk_smem + wib * WideRing<double>::kWarpBytes, sptr, vals, tptr, tab, runs, n,
+                                         nslices, (int64_t)blockIdx.x * kWideWarps + wib,
+                                         (int64_t)gridDim.x * kWideWarps, GatherX<double>{x}, Epi<KIND>{b, v, acc},
+                                         &st->status, FEMK_TIMEOUT);
+  if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
+  finish<KIND, kWideWarps * 32>(st, acc, partials);
 }
 
 // (1) beta = rho' / rho * alpha / omega;  p = r + beta (p - omega q);  phat = D^-1 p
@@ -291,6 +311,19 @@ int launch_spmv(const femk_plan* p, const double* x, const double* b, const Vecs
                                        : launch_bulk_kind<KIND, 32>(p, x, b, v, st, s, prime);
     if (ok) return FEMK_OK;
   }
+  if (p->sell_ct && p->bulk_cfg) {
+    auto kern = k_bicg_wide<KIND>;
+    constexpr int kSmem = kWideWarps * WideRing<double>::kWarpBytes;
+    static int per_sm = -1;
+    if (per_sm < 0) per_sm = wide_blocks((const void*)kern, kSmem);
+    if (per_sm > 0) {
+      if (!prime)
+        kern<<<counted_launch() + p->n_sm * std::min(per_sm, 16), kWideWarps * 32, kSmem, s>>>(
+            p->sell_ptr, p->sell_vals, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, x, b, v, p->partials, st);
+      FEMK_CUDA_TRY(cudaGetLastError());
+      return FEMK_OK;
+    }
+  }
   if (p->sell_c16 && p->sell64_c16) {
     auto kern = k_bicg_sell<KIND, int16_t>;
     const int grid = wave_grid(kern, kThreads, p);
@@ -380,9 +413,9 @@ __global__ void k_bicg_setup(BicgState* st, double tol2, double atol_sq, int32_t
   st->done = 0;
 }
 
-// One BiCGStab solve on the plan's prepared sliced-ELL operator: x holds x0 on entry. Ends with the
-// true-residual SpMV (kResid) and returns the final state in *out (host).
-int solve_prepared(femk_plan* p, const double* b, double* x, const double* dinv, double tol, double atol,
+// One BiCGStab solve on the plan's prepared sliced-ELL operator, all vectors in the solver's row order: x holds x0
+// on entry. Ends with the true-residual SpMV (kResid) and returns the final state in *out (host).
+int solve_in_order(femk_plan* p, const double* b, double* x, const double* dinv, double tol, double atol,
                    int32_t maxiter, cudaStream_t ws, BicgState* out) {
   const Vecs v = vecs_of(p);
   BicgState* st = (BicgState*)p->bicg_state;
@@ -428,6 +461,18 @@ int solve_prepared(femk_plan* p, const double* b, double* x, const double* dinv,
   FEMK_CUDA_TRY(cudaMemcpyAsync(host, st, sizeof(BicgState), cudaMemcpyDeviceToHost, ws));
   FEMK_CUDA_TRY(cudaStreamSynchronize(ws));
   *out = host[0];
+  return FEMK_OK;
+}
+
+// The same with the caller's vectors (DOF order).
+int solve_prepared(femk_plan* p, const double* b, double* x, const double* dinv, double tol, double atol,
+                   int32_t maxiter, cudaStream_t ws, BicgState* out) {
+  if (!p->perm) return solve_in_order(p, b, x, dinv, tol, atol, maxiter, ws, out);
+  double* xs = x;
+  FEMK_TRY(permute_in(p, &b, &xs, &dinv, ws));
+  FEMK_TRY(solve_in_order(p, b, xs, dinv, tol, atol, maxiter, ws, out));
+  FEMK_TRY(permute_out(p, xs, x, ws));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(ws));
   return FEMK_OK;
 }
 

@@ -301,4 +301,166 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
   return ok;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Slices of any width with 32-bit column tables (femk_order.cu): what 3-D P2 rows (up to 65 entries) need. A warp
+// takes a slice in pieces of at most kPiece entries, each streamed into its one stage: the values, and the piece of
+// the slice's table: the offsets of its runs of rows, or of every entry. One stage a warp and 4 warps a block, as the
+// 16-entry ring: more warps hide the gathers better than a deeper ring.
+// ---------------------------------------------------------------------------------------------
+constexpr int kWideWarps = 4;
+constexpr int kPiece = 16;
+
+struct WideDir {
+  int64_t b0, t0;         // first value, first table word
+  int32_t w, runs, first; // entries a row; runs of rows (0: full offsets) and where the later ones start
+};
+
+template <typename V>
+struct WideRing {
+  static constexpr int kVal = 32 * kPiece * (int)sizeof(V);
+  static constexpr int kCol = 32 * kPiece * 4;  // full offsets (those of up to 4 runs take less)
+  static constexpr int kDir = 16;
+  static constexpr int kHead = 128 + kDir * (int)sizeof(WideDir);
+  static constexpr int kWarpBytes = kHead + kVal + kCol;
+  static_assert(kHead % 128 == 0, "stage alignment");
+};
+
+// Every slice of this warp (g, g + NW, ...): epi(row, row sum), sums in entry order. False if a wait timed out
+// (*err is set to errval).
+template <typename V, typename G, typename Epi>
+__device__ __forceinline__ bool sell_wide_rows(unsigned char* wsmem, const int64_t* __restrict__ sptr,
+                                               const V* __restrict__ vals, const int64_t* __restrict__ tptr,
+                                               const int32_t* __restrict__ tab, const int32_t* __restrict__ runs,
+                                               int64_t n, int64_t nslices64, int64_t g64, int64_t NW64, const G& gx,
+                                               Epi&& epi, int* err, int errval) {
+  using R = WideRing<V>;
+  const int lane = threadIdx.x & 31;
+  const int32_t nslices = (int32_t)nslices64, g = (int32_t)g64, NW = (int32_t)NW64;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(wsmem);
+  WideDir* dir = reinterpret_cast<WideDir*>(wsmem + 128);
+  unsigned char* st = wsmem + R::kHead;
+  const V* sv = reinterpret_cast<const V*>(st) + lane;
+  const int32_t* sb = reinterpret_cast<const int32_t*>(st + R::kVal);
+  uint64_t pol = 0;
+  if (lane == 0) {
+    pol = l2_evict_first();
+    mbar_init(bar, 1);
+    mbar_fence_init();
+  }
+  int32_t dbase = 0;
+  auto fill_dir = [&](int32_t base) {  // slices of ordinals [base, base + kDir), one a lane
+    if (lane < R::kDir) {
+      const int32_t sl = g + (base + lane) * NW;
+      if (sl < nslices) {
+        const int64_t b0 = __ldg(sptr + sl), t0 = __ldg(tptr + sl);
+        const int32_t w = (int32_t)((__ldg(sptr + sl + 1) - b0) >> 5), first = __ldg(runs + sl);
+        const int32_t words = (int32_t)(__ldg(tptr + sl + 1) - t0), head = (w + 3) & ~3;
+        dir[lane] = WideDir{b0, t0, w, first < 0 || head == 0 ? 0 : words / head, first};
+      }
+    }
+    __syncwarp();
+  };
+  fill_dir(0);
+  // lane 0: stream entries [k0, k0 + kc) of slice d into the stage
+  auto issue = [&](const WideDir& d, int32_t k0, int32_t kc) {
+    const uint32_t vb = (uint32_t)(32 * kc * (int)sizeof(V));
+    const uint32_t cb = (uint32_t)(4 * (d.runs > 0 ? d.runs * ((kc + 3) & ~3) : 32 * kc));
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(bar, vb + cb);  // with no bytes this arrival alone completes the phase
+    if (kc > 0) {
+      bulk_g2s(st, vals + d.b0 + 32 * (int64_t)k0, vb, bar, pol);
+      bulk_g2s(st + R::kVal, tab + d.t0 + (int64_t)(d.runs > 0 ? d.runs : 32) * k0, cb, bar, pol);
+    }
+  };
+  if (lane == 0 && g < nslices) issue(dir[0], 0, min(kPiece, dir[0].w));
+  uint32_t parity = 0;
+  bool ok = true;
+  int32_t j = 0;
+  for (int32_t sl = g; sl < nslices && ok; sl += NW, ++j) {
+    const WideDir d = dir[j - dbase];
+    const int32_t row = sl * 32 + lane;
+    const bool live = row < n;
+    int run = 0;  // of this lane's row
+    if (d.runs > 1)
+      run = (lane >= (d.first & 255)) + (lane >= ((d.first >> 8) & 255)) + (lane >= ((d.first >> 16) & 255));
+    V acc = V(0);
+    for (int32_t k0 = 0;;) {
+      const int32_t kc = min(kPiece, d.w - k0);
+      if (!mbar_wait_all(bar, parity)) {
+        ok = false;
+        break;
+      }
+      parity ^= 1u;
+      // K entries (the piece's, rounded up to 4): those past kc gather the row itself and count nothing, so
+      // no load hangs on a branch
+      auto sum = [&](auto KC, auto&& offset) {
+        constexpr int K = decltype(KC)::value;
+        V xg[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) xg[k] = gx(k < K - 3 || k < kc ? row + offset(k) : row);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const V t = fma(sv[k * 32], xg[k], acc);
+          acc = k < K - 3 || k < kc ? t : acc;
+        }
+      };
+      auto sized = [&](auto&& offset) {
+        using std::integral_constant;
+        if (kc > 12)
+          sum(integral_constant<int, 16>{}, offset);
+        else if (kc > 8)
+          sum(integral_constant<int, 12>{}, offset);
+        else if (kc > 4)
+          sum(integral_constant<int, 8>{}, offset);
+        else
+          sum(integral_constant<int, 4>{}, offset);
+      };
+      if (live) {
+        if (d.runs > 0) {
+          const int32_t* c = sb + run * ((kc + 3) & ~3);
+          sized([&](int k) { return c[k]; });
+        } else {
+          const int32_t* c = sb + lane;
+          sized([&](int k) { return c[32 * k]; });
+        }
+      }
+      __syncwarp();  // every lane is done with the stage
+      k0 += kc;
+      if (k0 < d.w) {
+        if (lane == 0) issue(d, k0, min(kPiece, d.w - k0));
+        continue;
+      }
+      if (sl + NW < nslices) {
+        if (j + 1 >= dbase + R::kDir) {
+          dbase = j + 1;
+          fill_dir(dbase);
+        }
+        if (lane == 0) issue(dir[j + 1 - dbase], 0, min(kPiece, dir[j + 1 - dbase].w));
+      }
+      break;
+    }
+    __syncwarp();
+    if (ok && live) epi((int64_t)row, acc);
+  }
+  if (!ok) {
+    if (lane == 0) {
+      atomicExch(err, errval);
+      mbar_wait(bar, parity);  // the one copy in flight lands (bounded) before the block may exit
+    }
+    __syncwarp();
+  }
+  return ok;
+}
+
+// blocks of kWideWarps warps with smem bytes of shared memory that fit an SM; 0 when they do not run
+inline int wide_blocks(const void* kern, int smem) {
+  int b = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, kWideWarps * 32, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return b;
+}
+
 }  // namespace femk

@@ -256,6 +256,42 @@ __global__ void __launch_bounds__(WPB * 32) k_sell_bulk(const int64_t* __restric
   }
 }
 
+// The CG step on slices of any width with 32-bit column tables (3-D P2 rows; femk_bulk.cuh, sell_wide_rows).
+template <int WPB>
+__global__ void __launch_bounds__(WPB * 32, 8) k_sell_wide(const int64_t* __restrict__ sptr, const double* __restrict__ svals,
+                                                       const int64_t* __restrict__ tptr,
+                                                       const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n, int64_t nslices,
+                                                       const double* __restrict__ x, double* __restrict__ y,
+                                                       double* __restrict__ partials, CgState* st) {
+  extern __shared__ __align__(128) unsigned char bulk_smem[];
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->xpend = 0;  // the last x update is applied
+  if (st->done) return;
+  const int wib = threadIdx.x >> 5;
+  double acc[1] = {0.0};
+  const bool ok = sell_wide_rows<double>(
+      bulk_smem + wib * WideRing<double>::kWarpBytes, sptr, svals, tptr, tab, runs, n, nslices,
+      (int64_t)blockIdx.x * WPB + wib, (int64_t)gridDim.x * WPB, checked(GatherX<double>{x}, n, &st->status),
+      [&](int64_t row, double sv) {
+        y[row] = sv;
+        acc[0] += __ldg(x + row) * sv;
+      },
+      &st->status, FEMK_TIMEOUT);
+  if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
+  block_reduce_store<1, WPB * 32>(acc, partials);
+  double tot[1];
+  if (!grid_finish<1, WPB * 32>(partials, &st->ticket, tot)) return;
+  if (threadIdx.x != 0) return;
+  st->pq = tot[0];
+  st->alpha = st->gamma / tot[0];
+  if (!isfinite(tot[0])) {
+    st->status = FEMK_NONFINITE;
+    st->done = 1;
+  } else if (!(tot[0] > 0.0)) {
+    st->status = FEMK_BREAKDOWN;
+    st->done = 1;
+  }
+}
+
 template <typename T>
 __global__ void k_sell_gather(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr, int64_t n,
                               int64_t nslices, const double* __restrict__ vals, int64_t nnz, int32_t cap,
@@ -265,6 +301,17 @@ __global__ void k_sell_gather(const int64_t* __restrict__ sptr, const int32_t* _
   sell_transpose_warp<T>(sg_buf + (int64_t)wib * cap, cap, sptr, indptr, n, nslices, vals, nnz, out,
                          (int64_t)blockIdx.x * wpb + wib, (int64_t)gridDim.x * wpb,
                          [](double v, int64_t, int64_t) { return (T)v; }, err);
+}
+
+template <typename T>
+__global__ void k_sell_gather_order(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr,
+                                    const int32_t* __restrict__ perm, const uint8_t* __restrict__ src, int64_t n,
+                                    int64_t nslices, const double* __restrict__ vals, int64_t nnz, T* __restrict__ out,
+                                    int* __restrict__ err) {
+  const int wpb = blockDim.x >> 5;
+  sell_order_warp<T>(sptr, indptr, perm, src, n, nslices, vals, nnz, out,
+                     (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5), (int64_t)gridDim.x * wpb,
+                     [](double v, int64_t, int64_t) { return (T)v; }, err);
 }
 
 // x += alpha p; r -= alpha q; z = D^-1 r; <r, z>, <r, r>; stop test; beta.
@@ -906,12 +953,27 @@ bool launch_sell_bulk(const femk_plan* p, const double* x, double* y, CgState* s
 #undef FEMK_BULK_CFG
 }
 
+// The same on 32-bit column tables (plans whose offsets do not fit 16 bits but have tables).
+bool launch_sell_wide(const femk_plan* p, const double* x, double* y, CgState* st, cudaStream_t s,
+                      bool prime = false) {
+  if (!p->sell_ct || !p->bulk_cfg) return false;
+  auto kern = k_sell_wide<kWideWarps>;
+  constexpr int kSmem = kWideWarps * WideRing<double>::kWarpBytes;
+  static int per_sm = -1;
+  if (per_sm < 0) per_sm = wide_blocks((const void*)kern, kSmem);
+  if (per_sm <= 0) return false;
+  if (prime) return true;
+  kern<<<::femk::counted_launch() + p->n_sm * std::min(per_sm, 16), kWideWarps * 32, kSmem, s>>>(
+      p->sell_ptr, p->sell_vals, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, x, y, p->partials, st);
+  return true;
+}
+
 // The operator of a solve: the sliced-ELL copy (values gathered by prepare_sell) or the CSR.
 template <int MODE>
 int launch_op(const femk_plan* p, bool sell, const double* vals, const double* x, double* y, const double* b,
               const double* dinv, double* z, double* pout, CgState* st, double tol2, double atol2, cudaStream_t s) {
   if (!sell) return launch_csr<MODE>(p, vals, x, y, b, dinv, z, pout, st, tol2, atol2, s);
-  if (MODE == kCgStep && launch_sell_bulk(p, x, y, st, s)) {
+  if (MODE == kCgStep && (launch_sell_bulk(p, x, y, st, s) || launch_sell_wide(p, x, y, st, s))) {
     FEMK_CUDA_TRY(cudaGetLastError());
     return FEMK_OK;
   }
@@ -962,14 +1024,8 @@ int launch_op(const femk_plan* p, bool sell, const double* vals, const double* x
 }
 
 int prepare_sell(femk_plan* p, const double* vals, cudaStream_t s) {
-  if (!p->sell_vals) FEMK_CUDA_TRY(cudaMalloc(&p->sell_vals, sizeof(double) * (p->sell_nnz + 1)));
-  const int32_t cap = 32 * (p->max_row > 0 ? p->max_row : 1);
-  const size_t smem = sizeof(double) * 4 * (size_t)cap;
-  FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_gather<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_sell_gather<double><<<::femk::counted_launch() + blocks_for(p->n_slices, 4, p->n_sm * 16), 128, smem, s>>>(
-      p->sell_ptr, p->indptr, p->n, p->n_slices, vals, p->nnz, cap, p->sell_vals, p->dev_err);
-  FEMK_CUDA_TRY(cudaGetLastError());
-  return FEMK_OK;
+  FEMK_TRY(ensure_sell_values(p, false));
+  return launch_sell_values(p, vals, false, s);
 }
 
 struct MatFree {
@@ -1114,6 +1170,7 @@ int ensure_chunk_graph(femk_plan* p, const double* vals, double* x, const double
   (void)wave_grid(k_pupdate_x<true>, kThreads, p);
   (void)wave_grid(k_pupdate_x<false>, kThreads, p);
   if (sell) (void)launch_sell_bulk(p, nullptr, nullptr, nullptr, nullptr, true);
+  if (sell) (void)launch_sell_wide(p, nullptr, nullptr, nullptr, nullptr, true);
   cudaGraph_t g = nullptr;
   set_capturing(true);
   cudaError_t e = cudaStreamBeginCapture(p->cg_stream, cudaStreamCaptureModeThreadLocal);
@@ -1316,6 +1373,15 @@ int launch_sell_values(const femk_plan* p, const double* vals, bool fp32, cudaSt
   const int32_t cap = 32 * (p->max_row > 0 ? p->max_row : 1);
   const size_t smem = sizeof(double) * 4 * (size_t)cap;
   const int grid = blocks_for(p->n_slices, 4, p->n_sm * 16);
+  if (p->perm) {
+    k_sell_gather_order<double><<<::femk::counted_launch() + grid, 128, 0, s>>>(
+        p->sell_ptr, p->indptr, p->perm, p->sell_src, p->n, p->n_slices, vals, p->nnz, p->sell_vals, p->dev_err);
+    if (fp32)
+      k_sell_gather_order<float><<<::femk::counted_launch() + grid, 128, 0, s>>>(
+          p->sell_ptr, p->indptr, p->perm, p->sell_src, p->n, p->n_slices, vals, p->nnz, p->sell_vals32, p->dev_err);
+    FEMK_CUDA_TRY(cudaGetLastError());
+    return FEMK_OK;
+  }
   k_sell_gather<double><<<::femk::counted_launch() + grid, 128, smem, s>>>(p->sell_ptr, p->indptr, p->n, p->n_slices,
                                                                            vals, p->nnz, cap, p->sell_vals, p->dev_err);
   if (fp32)
@@ -1389,8 +1455,16 @@ extern "C" int femk_spmv_prepared(const femk_plan* p, const double* x, double* y
   clear_error();
   FEMK_CHECK_ARG(p && x && y, "femk_spmv_prepared: NULL argument");
   FEMK_CHECK_ARG(p->sell_vals, "femk_spmv_prepared: call femk_prepare_operator first");
-  FEMK_TRY(launch_op<kPlain>(p, true, nullptr, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, 0.0,
-                             (cudaStream_t)stream));
+  cudaStream_t s = (cudaStream_t)stream;
+  if (p->perm) {
+    double* xs = const_cast<double*>(x);  // read only
+    FEMK_TRY(permute_in(const_cast<femk_plan*>(p), nullptr, &xs, nullptr, s));
+    double* ys = p->perm_ws;
+    FEMK_TRY(launch_op<kPlain>(p, true, nullptr, xs, ys, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, 0.0, s));
+    FEMK_TRY(permute_out(p, ys, y, s));
+    return check_bounds(p, s, "femk_spmv_prepared");
+  }
+  FEMK_TRY(launch_op<kPlain>(p, true, nullptr, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, 0.0, s));
   return check_bounds(p, (cudaStream_t)stream, "femk_spmv_prepared");
 }
 
@@ -1425,9 +1499,17 @@ extern "C" int femk_pcg(const femk_plan* p, const double* vals, const double* b,
   clear_error();
   FEMK_CHECK_ARG(p && vals && b && x, "femk_pcg: NULL argument");
   FEMK_CHECK_ARG(tol >= 0.0 && atol >= 0.0, "femk_pcg: negative tolerance");
-  if (pcg_persist_fits(p))
-    return pcg_persist(p, vals, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, (cudaStream_t)stream);
-  return pcg_run(p, vals, nullptr, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, (cudaStream_t)stream);
+  cudaStream_t s = (cudaStream_t)stream;
+  double* xs = x;
+  if (p->perm) FEMK_TRY(permute_in(const_cast<femk_plan*>(p), &b, &xs, &dinv, s));
+  const int rc = pcg_persist_fits(p)
+                     ? pcg_persist(p, vals, b, xs, dinv, tol, atol, maxiter, iters_out, relres_out, s)
+                     : pcg_run(p, vals, nullptr, b, xs, dinv, tol, atol, maxiter, iters_out, relres_out, s);
+  if (p->perm) {  // x holds what the solver left, whatever its status
+    FEMK_TRY(permute_out(p, xs, x, s));
+    FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  }
+  return rc;
 }
 
 extern "C" int femk_pcg_matfree(const femk_plan* p, const double* param, int mode, double scale, const double* b,

@@ -182,6 +182,17 @@ struct femk_plan {
   int64_t* sell_cuptr = nullptr;  // i64[n_slices+1] first table entry of each slice
   int16_t* sell_cu = nullptr;     // i16[sell_cu_len]
   int64_t sell_cu_len = 0;
+  // 32-bit column tables of the bulk-copy product of wide rows (sell_wide_rows), where int16 offsets do not fit
+  int64_t* sell_ctptr = nullptr;  // i64[n_slices+1] first word of each slice
+  int32_t* sell_ct = nullptr;     // i32[sell_ct_len]
+  int64_t sell_ct_len = 0;
+  int32_t* sell_runs = nullptr;   // i32[n_slices] first rows of a slice's second to fourth run (a byte each), -1: full
+  // the solver's row order (femk_order.cu), NULL: the DOF order
+  void* perm_base = nullptr;    // the allocation that holds sell_ctptr, perm, pos and sell_runs
+  int32_t* perm = nullptr;      // i32[n] DOF of each solver row
+  int32_t* pos = nullptr;       // i32[n] solver row of each DOF
+  uint8_t* sell_src = nullptr;  // u8[sell_nnz] place of each entry in its CSR row (255: padding)
+  double* perm_ws = nullptr;    // f64[3 vstride] b, x and D^-1 of a solve in the solver's order
   int use_sell = 1;
   int l2_mode = 0;               // L2 eviction hints of the FP64 CG kernels (the l2_hints plan option)
   int sell64_c16 = 1;            // FP64 sliced-ELL streams int16 column offsets when available
@@ -281,6 +292,15 @@ int check_bounds(const femk_plan* p, cudaStream_t s, const char* what);
 int scan_exclusive_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
 
 int ensure_workspace(femk_plan* p);
+
+// The sliced-ELL copy of the pattern in the solver's row order (femk_order.cu). natural_order rebuilds it in the
+// DOF order, for solvers whose problems own runs of DOFs. permute_in copies b, x and dinv (each may be NULL) into
+// plan-owned vectors in the solver's order and redirects the pointers to those; permute_out copies back. Both only
+// for plans with a row order of their own (p->perm).
+int build_sell(femk_plan* p, cudaStream_t s);
+int natural_order(femk_plan* p, cudaStream_t s);
+int permute_in(femk_plan* p, const double** b, double** x, const double** dinv, cudaStream_t s);
+int permute_out(const femk_plan* p, const double* xs, double* x, cudaStream_t s);
 
 // The sliced-ELL value copies of a caller's CSR values (femk_cg.cu): ensure_sell_values allocates
 // sell_vals (and, fp32, sell_vals32) and sets the copy kernels' shared-memory size (not during a

@@ -134,10 +134,11 @@ __global__ void k_fill_f(float* __restrict__ v, int64_t n, float val) {
 
 // S = D^-1/2 from the Jacobi inverse: FP32 (the fold x += S e) and FP64 (s64, forming A^); D itself
 // (FP32, for <r, D r>)
-__global__ void k_scaling(const double* __restrict__ dinv, int64_t n, float* __restrict__ sc, float* __restrict__ dd,
-                          double* __restrict__ s64) {
+// (all in the solver's row order; dinv in the DOF order, as x, b and the CSR are)
+__global__ void k_scaling(const double* __restrict__ dinv, const int32_t* __restrict__ perm, int64_t n,
+                          float* __restrict__ sc, float* __restrict__ dd, double* __restrict__ s64) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double di = dinv[i];
+    const double di = dinv[perm ? perm[i] : i];
     const double si = sqrt(di);
     sc[i] = (float)si;
     dd[i] = (float)(1.0 / di);
@@ -159,6 +160,25 @@ __global__ void k_gather_scaled(const int64_t* __restrict__ sptr, const int32_t*
       sg_buf + (int64_t)wib * cap, cap, sptr, indptr, n, nslices, vals, nnz, out, (int64_t)blockIdx.x * wpb + wib,
       (int64_t)gridDim.x * wpb,
       [&](double v, int64_t row, int64_t j) {
+        const int64_t col = sizeof(IDX) == 2 ? row + (int64_t)__ldcs(cols + j) : (int64_t)__ldcs(cols + j);
+        return (float)(v * __ldg(s64 + row) * __ldg(s64 + col));
+      },
+      err);
+}
+
+// the same for a plan with a row order of its own
+template <typename IDX>
+__global__ void k_gather_scaled_order(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr,
+                                      const int32_t* __restrict__ perm, const uint8_t* __restrict__ src,
+                                      const IDX* __restrict__ cols, int64_t n, int64_t nslices,
+                                      const double* __restrict__ vals, int64_t nnz, const double* __restrict__ s64,
+                                      float* __restrict__ out, int* __restrict__ err) {
+  const int wpb = blockDim.x >> 5;
+  sell_order_warp<float>(
+      sptr, indptr, perm, src, n, nslices, vals, nnz, out, (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5),
+      (int64_t)gridDim.x * wpb,
+      [&](double v, int64_t row, int64_t j) {
+        if (row >= n) return 0.0f;
         const int64_t col = sizeof(IDX) == 2 ? row + (int64_t)__ldcs(cols + j) : (int64_t)__ldcs(cols + j);
         return (float)(v * __ldg(s64 + row) * __ldg(s64 + col));
       },
@@ -306,6 +326,29 @@ __global__ void __launch_bounds__(WPB * 32) k_step32_bulk(const int64_t* __restr
   step_finish<REFRESH, WPB * 32>(st, tot[0], partials + kPartialsA, ga, odd);
 }
 
+// K_B on slices of any width with 32-bit column tables (3-D P2 rows; femk_bulk.cuh, sell_wide_rows).
+template <bool REFRESH>
+__global__ void __launch_bounds__(kWideWarps * 32, 8) k_step32_wide(const int64_t* __restrict__ sptr,
+                                                                const float* __restrict__ vals,
+                                                                const int64_t* __restrict__ tptr,
+                                                                const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n,
+                                                                int64_t nslices, const float* __restrict__ r,
+                                                                float* __restrict__ w, double* __restrict__ partials,
+                                                                int ga, MixedState* st, int odd) {
+  extern __shared__ __align__(128) unsigned char bulk_smem[];
+  if (step_skip(st, REFRESH)) return;
+  const int wib = threadIdx.x >> 5;
+  StepEpi epi{r, w, 0.f};
+  const bool ok = sell_wide_rows<float>(bulk_smem + wib * WideRing<float>::kWarpBytes, sptr, vals, tptr, tab, runs, n,
+                                        nslices, (int64_t)blockIdx.x * kWideWarps + wib,
+                                        (int64_t)gridDim.x * kWideWarps, checked(GatherX<float>{r}, n, &st->status),
+                                        epi, &st->status, FEMK_TIMEOUT);
+  if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
+  double v[1] = {(double)epi.a}, tot[1];
+  if (!reduce_finish<1, kWideWarps * 32>(v, partials, &st->ticket, tot)) return;
+  step_finish<REFRESH, kWideWarps * 32>(st, tot[0], partials + kPartialsA, ga, odd);
+}
+
 // K_B on the CSR copy (plans without a sliced-ELL layout)
 template <int L, int U, typename IDX, bool REFRESH>
 __global__ void __launch_bounds__(kThreads) k_step32(const int32_t* __restrict__ indptr, const IDX* __restrict__ cols,
@@ -403,23 +446,25 @@ __global__ void __launch_bounds__(kThreads) k_mixed_update(int64_t n, const floa
 
 // x += S (e + alpha_pend p); e = 0 (only at a requested update; the owed term of an even last step
 // is paid here)
-__global__ void k_fold(int64_t n, double* __restrict__ x, float* __restrict__ e, const float* __restrict__ p,
-                       const float* __restrict__ sc, const MixedState* st) {
+__global__ void k_fold(int64_t n, double* __restrict__ x, const int32_t* __restrict__ perm, float* __restrict__ e,
+                       const float* __restrict__ p, const float* __restrict__ sc, const MixedState* st) {
   if (st->done || st->need_update != 1) return;
   const float ap = (float)st->alpha_pend;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += (double)sc[i] * (double)fmaf(ap, p[i], e[i]);
+    x[perm ? perm[i] : i] += (double)sc[i] * (double)fmaf(ap, p[i], e[i]);
     e[i] = 0.f;
   }
 }
 
-// r64 = b - A64 x; r^ = fp32(S r64); <r^, r^>, <r64, r64> (+ <b, b> at init, + <p, s>, <r^, s> after)
+// r64 = b - A64 x; r^ = fp32(S r64); <r^, r^>, <r64, r64> (+ <b, b> at init, + <p, s>, <r^, s> after). On the CSR in
+// the DOF order; r^, p and s are in the solver's (row pos[i], or i).
 template <int L, int U, bool INIT>
 __global__ void __launch_bounds__(kThreads) k_true_resid(const int32_t* __restrict__ indptr,
                                                         const int32_t* __restrict__ indices,
                                                         const double* __restrict__ vals, int64_t n,
                                                         const double* __restrict__ x, const double* __restrict__ b,
-                                                        const double* __restrict__ dinv, float* __restrict__ r,
+                                                        const double* __restrict__ dinv,
+                                                        const int32_t* __restrict__ pos, float* __restrict__ r,
                                                         const float* __restrict__ p, const float* __restrict__ s,
                                                         double* __restrict__ partials, MixedState* st, double tol2,
                                                         double atol2) {
@@ -440,14 +485,15 @@ __global__ void __launch_bounds__(kThreads) k_true_resid(const int32_t* __restri
       const double bi = b[row];
       const double r64 = bi - sv[k];
       const float rf = (float)(sqrt(dinv[row]) * r64);
-      r[row] = rf;
+      const int64_t at = pos ? pos[row] : row;
+      r[at] = rf;
       a[0] += (double)rf * (double)rf;
       a[1] += r64 * r64;
       if (INIT) {
         a[2] += bi * bi;
       } else {
-        const float si = s[row];
-        a[3] += (double)p[row] * (double)si;
+        const float si = s[at];
+        a[3] += (double)p[at] * (double)si;
         a[4] += (double)rf * (double)si;
       }
     }
@@ -490,7 +536,7 @@ void launch_true_resid(const femk_plan* p, const double* vals, const double* x, 
     constexpr int L = decltype(Lc)::value, U = decltype(Uc)::value;
     const int grid = wave_grid(k_true_resid<L, U, INIT>, kThreads, p);
     k_true_resid<L, U, INIT><<<::femk::counted_launch() + grid, kThreads, 0, s>>>(
-        p->indptr, p->indices, vals, p->n, x, b, dinv, r, pv, sv, p->partials, st, tol2, atol2);
+        p->indptr, p->indices, vals, p->n, x, b, dinv, p->pos, r, pv, sv, p->partials, st, tol2, atol2);
   });
 }
 
@@ -547,10 +593,27 @@ bool launch_step32_bulk(const femk_plan* p, const float* r, float* w, MixedState
 #undef FEMK_BULK_CFG
 }
 
+template <bool REFRESH>
+bool launch_step32_wide(const femk_plan* p, const float* r, float* w, MixedState* st, cudaStream_t s,
+                        bool prime = false, int odd = 0) {
+  if (!p->sell_ct || !p->sell_vals32 || !p->bulk32_cfg) return false;
+  auto kern = k_step32_wide<REFRESH>;
+  constexpr int kSmem = kWideWarps * WideRing<float>::kWarpBytes;
+  static int per_sm = -1;
+  if (per_sm < 0) per_sm = wide_blocks((const void*)kern, kSmem);
+  if (per_sm <= 0) return false;
+  if (prime) return true;
+  kern<<<::femk::counted_launch() + p->n_sm * std::min(per_sm, 16), kWideWarps * 32, kSmem, s>>>(
+      p->sell_ptr, p->sell_vals32, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, r, w, p->partials, update_grid(p), st,
+      odd);
+  return true;
+}
+
 // K_B in the plan's layout; odd: the parity of the step (normal steps; 0 for a refresh)
 template <bool REFRESH>
 void launch_step32(const femk_plan* p, const float* r, float* w, MixedState* st, cudaStream_t s, int odd = 0) {
   if (launch_step32_bulk<REFRESH>(p, r, w, st, s, false, odd)) return;
+  if (launch_step32_wide<REFRESH>(p, r, w, st, s, false, odd)) return;
   const int ga = update_grid(p);
   if (p->sell_vals32) {
     if (p->sell_c16) {
@@ -594,6 +657,8 @@ void prime_mixed(const femk_plan* p) {
   (void)wave_grid(k_step32_sell<int32_t, true>, kThreads, p);
   (void)launch_step32_bulk<false>(p, nullptr, nullptr, nullptr, nullptr, true);
   (void)launch_step32_bulk<true>(p, nullptr, nullptr, nullptr, nullptr, true);
+  (void)launch_step32_wide<false>(p, nullptr, nullptr, nullptr, nullptr, true);
+  (void)launch_step32_wide<true>(p, nullptr, nullptr, nullptr, nullptr, true);
   (void)update_grid(p);
   (void)wave_grid(k_fold, 256, p);
 }
@@ -630,7 +695,7 @@ int enqueue_mixed_chunk(const femk_plan* p, const double* vals, const double* b,
                                                          m.st);
     launch_step32<false>(p, m.r, m.w, m.st, s, odd);
   }
-  k_fold<<<::femk::counted_launch() + wave_grid(k_fold, 256, p), 256, 0, s>>>(n, x, m.e, m.pv, m.sc, m.st);
+  k_fold<<<::femk::counted_launch() + wave_grid(k_fold, 256, p), 256, 0, s>>>(n, x, p->perm, m.e, m.pv, m.sc, m.st);
   launch_true_resid<false>(p, vals, x, b, dinv, m.r, m.pv, m.s, m.st, 0.0, 0.0, s);
   launch_step32<true>(p, m.r, m.w, m.st, s);
   FEMK_CUDA_TRY(cudaGetLastError());
@@ -728,12 +793,21 @@ extern "C" int femk_pcg_mixed(const femk_plan* pc, const double* vals, const dou
   else prime_mixed(p);
   const int g1 = p->n_sm * 8;
   double* s64 = p->work;  // the FP64 CG workspace is free during a mixed solve
-  k_scaling<<<::femk::counted_launch() + g1, 256, 0, ws>>>(dinv64, n, m.sc, m.dd, s64);
+  k_scaling<<<::femk::counted_launch() + g1, 256, 0, ws>>>(dinv64, p->perm, n, m.sc, m.dd, s64);
   if (p->sell_vals32) {
     const int gg = blocks_for(p->n_slices, 4, p->n_sm * 16);
     const int32_t cap = 32 * (p->max_row > 0 ? p->max_row : 1);
     const size_t smem = sizeof(double) * 4 * (size_t)cap;
-    if (p->sell_c16) {
+    if (p->perm) {
+      if (p->sell_c16)
+        k_gather_scaled_order<int16_t><<<::femk::counted_launch() + gg, 128, 0, ws>>>(
+            p->sell_ptr, p->indptr, p->perm, p->sell_src, p->sell_c16, n, p->n_slices, vals, p->nnz, s64,
+            p->sell_vals32, p->dev_err);
+      else
+        k_gather_scaled_order<int32_t><<<::femk::counted_launch() + gg, 128, 0, ws>>>(
+            p->sell_ptr, p->indptr, p->perm, p->sell_src, p->sell_cols, n, p->n_slices, vals, p->nnz, s64,
+            p->sell_vals32, p->dev_err);
+    } else if (p->sell_c16) {
       FEMK_CUDA_TRY(cudaFuncSetAttribute(k_gather_scaled<int16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k_gather_scaled<int16_t><<<::femk::counted_launch() + gg, 128, smem, ws>>>(
           p->sell_ptr, p->indptr, p->sell_c16, n, p->n_slices, vals, p->nnz, cap, s64, p->sell_vals32, p->dev_err);

@@ -1,0 +1,540 @@
+// The solver's copy of the operator (sliced ELL, SELL-32): its row order, its slices and its column tables.
+//
+// Row order. P1 plans keep the DOF order. A P2 plan numbers its edge midpoints as the cells first meet them, so
+// consecutive rows belong to different kinds of edges: rows of unequal length share a slice (12 % padding at
+// P2 64^3), and no two neighbouring rows have columns at the same offsets, so every entry carries a 4-byte column
+// and every gather of a slice touches up to 32 sectors. When the edges fall into few classes by the distance of
+// their end vertices' numbers (a lattice has 7 in 3-D, 3 in 2-D), the solver's rows are the vertices and then
+// the edges class by class, each in the order of the lower end: neighbouring rows of a class then have the same
+// length and the same column offsets along a mesh line. The solvers permute b, x and D^-1 on entry and x on
+// exit; nothing outside them sees the order. B200, us a product: P2 64^3 in FP32 99.5 -> 50.5 (544 -> 250 MB), P2
+// 37x45x41 in FP64 39.8 -> 26.8 (215 -> 132 MB): 5.0 TB/s of the measured 6.5.
+//
+// Column tables. With int16 columns (femk_bulk.cuh reads those) a slice whose rows share one offset sequence
+// stores it once. In the solver's order a slice mostly has one or two such runs of rows (one mesh line, or the end of
+// one and the start of the next), whose 32-bit offsets it stores once each (sell_wide_rows reads these).
+#include <algorithm>
+#include <climits>
+
+#include "femk_element.cuh"
+#include "femk_internal.cuh"
+#include "femk_bulk.cuh"
+#include "femk_spmv.cuh"
+
+namespace femk {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kMaxClasses = 16;
+
+template <typename T>
+int dev_alloc(T** p, int64_t count) {
+  FEMK_CUDA_TRY(cudaMalloc((void**)p, sizeof(T) * (count > 0 ? count : 1)));
+  return FEMK_OK;
+}
+
+struct Temp {
+  void* p = nullptr;
+  ~Temp() {
+    if (p) cudaFree(p);
+  }
+};
+
+int grid_for(const femk_plan* p, int64_t threads) { return blocks_for(threads, kThreads, p->n_sm * 64); }
+
+// ---------------------------------------------------------------------------------------------
+// row order
+// ---------------------------------------------------------------------------------------------
+// lower and upper end vertex of every edge midpoint (every cell writes the same)
+template <int ND>
+__global__ void k_edge_ends(const int32_t* __restrict__ cells, int64_t ntet, int64_t nvert, int2* __restrict__ ends) {
+  constexpr int NV = Cell<ND>::NV, NE = ND - NV;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ntet * NE; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = t / NE;
+    const int e = (int)(t % NE);
+    const int32_t a = cells[c * ND + cell_edge_a<NV>(e)], b = cells[c * ND + cell_edge_b<NV>(e)];
+    ends[cells[c * ND + NV + e] - nvert] = make_int2(min(a, b), max(a, b));
+  }
+}
+
+// the distinct distances upper - lower (at most kMaxClasses; cls[kMaxClasses] is raised when there are more)
+__global__ void k_edge_classes(const int2* __restrict__ ends, int64_t nedge, int32_t* __restrict__ cls) {
+  __shared__ int32_t seen[kMaxClasses];  // distances that the block has met in cls
+  if (threadIdx.x < kMaxClasses) seen[threadIdx.x] = 0;
+  __syncthreads();
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nedge; e += (int64_t)gridDim.x * blockDim.x) {
+    const int2 v = ends[e];
+    const int32_t d = v.y - v.x;
+    bool found = false;
+    for (int k = 0; k < kMaxClasses && !found; ++k) found = seen[k] == d;
+    if (found) continue;
+    if (*(volatile int32_t*)(cls + kMaxClasses)) return;  // there are too many already
+    for (int k = 0; k < kMaxClasses && !found; ++k) {
+      int32_t c = *(volatile int32_t*)(cls + k);
+      if (c == 0) c = atomicCAS(cls + k, 0, d);  // 0: this thread took the place
+      if ((found = c == 0 || c == d)) seen[k] = d;
+    }
+    if (!found) {
+      cls[kMaxClasses] = 1;
+      return;
+    }
+  }
+}
+
+__device__ __forceinline__ int class_of(const int32_t* __restrict__ cls, int nc, int32_t d) {
+  int k = 0;
+  while (k < nc - 1 && cls[k] != d) ++k;
+  return k;
+}
+
+__global__ void k_class_flags(const int2* __restrict__ ends, int64_t nedge, const int32_t* __restrict__ cls, int nc,
+                              int64_t nvert, int64_t* __restrict__ flag) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nedge; e += (int64_t)gridDim.x * blockDim.x) {
+    const int2 v = ends[e];
+    flag[class_of(cls, nc, v.y - v.x) * nvert + v.x] = 1;  // (class, lower end) names one edge
+  }
+}
+
+__global__ void k_order(const int2* __restrict__ ends, int64_t nedge, const int32_t* __restrict__ cls, int nc,
+                        int64_t nvert, const int64_t* __restrict__ rank, int32_t* __restrict__ perm,
+                        int32_t* __restrict__ pos) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nvert + nedge;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    int64_t at = t;
+    if (t >= nvert) {
+      const int2 v = ends[t - nvert];
+      at = nvert + rank[class_of(cls, nc, v.y - v.x) * nvert + v.x];
+    }
+    perm[at] = (int32_t)t;
+    pos[t] = (int32_t)at;
+  }
+}
+
+// perm / pos of a P2 plan whose edges fall into few classes; leaves them NULL otherwise
+int build_order(femk_plan* p, cudaStream_t s) {
+  if (p->order != 2 || !p->use_sell) return FEMK_OK;
+  const int64_t nedge = p->n - p->nvert;
+  if (nedge < 1) return FEMK_OK;
+  Temp first;  // edge ends, then the classes
+  FEMK_CUDA_TRY(cudaMalloc(&first.p, sizeof(int2) * nedge + sizeof(int32_t) * (kMaxClasses + 1)));
+  int2* ends = (int2*)first.p;
+  int32_t* cls = (int32_t*)(ends + nedge);
+  FEMK_CUDA_TRY(cudaMemsetAsync(cls, 0, sizeof(int32_t) * (kMaxClasses + 1), s));
+  if (p->nd == 10)
+    k_edge_ends<10><<<counted_launch() + grid_for(p, p->ntet * 6), kThreads, 0, s>>>(p->cells, p->ntet, p->nvert,
+                                                                                  ends);
+  else
+    k_edge_ends<6><<<counted_launch() + grid_for(p, p->ntet * 3), kThreads, 0, s>>>(p->cells, p->ntet, p->nvert,
+                                                                                 ends);
+  k_edge_classes<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(ends, nedge, cls);
+  FEMK_CUDA_TRY(cudaGetLastError());
+  int32_t h[kMaxClasses + 1];
+  FEMK_CUDA_TRY(cudaMemcpyAsync(h, cls, sizeof(h), cudaMemcpyDeviceToHost, s));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  if (h[kMaxClasses]) return FEMK_OK;
+  int nc = 0;
+  while (nc < kMaxClasses && h[nc]) ++nc;
+  std::sort(h, h + nc);  // they were found in no fixed order
+  FEMK_CUDA_TRY(cudaMemcpyAsync(cls, h, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
+  Temp second;  // a flag for every (class, lower end), then their exclusive scan
+  const int64_t m = nc * p->nvert;
+  FEMK_CUDA_TRY(cudaMalloc(&second.p, sizeof(int64_t) * 2 * (m + 1)));
+  int64_t* flag = (int64_t*)second.p;
+  int64_t* rank = flag + m + 1;
+  FEMK_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int64_t) * (m + 1), s));
+  k_class_flags<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(ends, nedge, cls, nc, p->nvert, flag);
+  FEMK_TRY(scan_exclusive_i64(flag, rank, m, s));
+  // one allocation (an allocation takes 0.3 ms): table starts, the two orders, run starts
+  const int64_t ns = (p->n + 31) / 32;
+  FEMK_CUDA_TRY(cudaMalloc(&p->perm_base, sizeof(int64_t) * (ns + 1) + sizeof(int32_t) * (2 * p->n + ns)));
+  p->perm = (int32_t*)((int64_t*)p->perm_base + ns + 1);
+  p->pos = p->perm + p->n;
+  k_order<<<counted_launch() + grid_for(p, p->n), kThreads, 0, s>>>(ends, nedge, cls, nc, p->nvert, rank, p->perm,
+                                                                    p->pos);
+  FEMK_CUDA_TRY(cudaGetLastError());
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));  // temporaries are freed on return
+  return FEMK_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// slices
+// ---------------------------------------------------------------------------------------------
+// Width of each 32-row slice (its longest row) and its entry count.
+__global__ void k_sell_width(const int32_t* __restrict__ indptr, const int32_t* __restrict__ perm, int64_t n,
+                             int64_t nslices, int64_t* __restrict__ len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
+    int64_t row = sl * 32 + lane;
+    const bool live = row < n;
+    if (live && perm) row = perm[row];
+    int w = live ? indptr[row + 1] - indptr[row] : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
+    if (lane == 0) len[sl] = (int64_t)w * 32;
+  }
+}
+
+__global__ void k_sell_fill(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
+                            int64_t nslices, const int64_t* __restrict__ sptr, int32_t* __restrict__ cols,
+                            int16_t* __restrict__ c16) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
+    const int64_t row = sl * 32 + lane;
+    const int64_t w = (sptr[sl + 1] - sptr[sl]) / 32;
+    const int32_t beg = row < n ? indptr[row] : 0;
+    const int32_t len = row < n ? indptr[row + 1] - beg : 0;
+    const int64_t self = row < n ? row : n - 1;
+    for (int64_t k = 0; k < w; ++k) {
+      const int64_t j = sptr[sl] + k * 32 + lane;
+      const bool real = k < len;
+      const int32_t col = real ? indices[beg + k] : (int32_t)self;
+      cols[j] = col;
+      if (c16) c16[j] = (int16_t)(col - self);
+    }
+  }
+}
+
+// The same in the solver's row order, with the column tables of sell_wide_rows. A warp takes a slice, a lane a row:
+// the row's columns as solver rows, sorted. Going down the slice, rows whose offsets (column - row) are all among
+// those of a longer row, or hold all of them, form a run and share that longest row's offsets, an entry for each
+// (value 0 where a row has none): rows along a mesh line, its ends included. A slice with up to kRuns runs stores
+// one offset sequence a run, piece by piece of kPiece entries, each padded to 4 words; a slice with more stores
+// every entry's offset. No shared offset leads outside [0, n).
+// PASS 0: words[s], the table words of slice s. PASS 1: columns, places in the CSR row, tables and run starts.
+constexpr int kRowMax = 255;  // place of an entry that a row does not have (rows hold fewer entries)
+constexpr int kRuns = 4;
+
+template <int PASS>
+__global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+                             const int32_t* __restrict__ perm, const int32_t* __restrict__ pos, int64_t n,
+                             int64_t nslices, const int64_t* __restrict__ sptr, int32_t cap,
+                             int64_t* __restrict__ words, int32_t* __restrict__ cols, uint8_t* __restrict__ src,
+                             const int64_t* __restrict__ tptr, int32_t* __restrict__ tab, int32_t* __restrict__ runs) {
+  extern __shared__ long long order_buf[];  // 32 cap words a warp: (offset << 8) | place, entry k of lane l at 32 k + l
+  const int lane = threadIdx.x & 31;
+  long long* buf = order_buf + (int64_t)(threadIdx.x >> 5) * 32 * cap;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
+    const int64_t b0 = sptr[sl];
+    const int32_t w = (int32_t)((sptr[sl + 1] - b0) >> 5), head = (w + 3) & ~3;
+    const int32_t row = (int32_t)(sl * 32) + lane;
+    const bool live = row < n;
+    const int32_t dof = live ? perm[row] : 0;
+    const int32_t beg = live ? indptr[dof] : 0;
+    const int32_t len = live ? indptr[dof + 1] - beg : 0;
+    for (int32_t k = 0; k < len; ++k) {  // insertion sort by offset
+      const long long v = ((long long)(pos[indices[beg + k]] - row) << 8) | k;
+      int32_t q = k;
+      for (; q > 0 && buf[32 * (q - 1) + lane] > v; --q) buf[32 * q + lane] = buf[32 * (q - 1) + lane];
+      buf[32 * q + lane] = v;
+    }
+    __syncwarp();
+    auto off = [&](int l, int32_t k) { return (int32_t)(buf[32 * k + l] >> 8); };
+    // whether every offset of lane `a` is one of lane `b` (all lanes ask and get the same answer)
+    auto within = [&](int a, int32_t na, int b, int32_t nb) {
+      bool in = true;
+      for (int32_t k = lane; k < na; k += 32) {
+        const int32_t v = off(a, k);
+        int32_t lo = 0, hi = nb;
+        while (lo < hi) {
+          const int32_t mid = (lo + hi) >> 1;
+          if (off(b, mid) < v)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        in = in && lo < nb && off(b, lo) == v;
+      }
+      return __all_sync(0xffffffffu, in) != 0;
+    };
+    int nruns = 1, rep[kRuns] = {0, 0, 0, 0}, start[kRuns] = {0, 32, 32, 32};
+    for (int l = 1; l < 32 && nruns > 0; ++l) {
+      const int32_t nl = __shfl_sync(0xffffffffu, len, l);
+      int cur = rep[0];
+#pragma unroll
+      for (int q = 1; q < kRuns; ++q)
+        if (q < nruns) cur = rep[q];
+      const int32_t nr = __shfl_sync(0xffffffffu, len, cur);
+      if (nl == 0 || within(l, nl, cur, nr)) continue;  // rows past n are in any run
+      if (within(cur, nr, l, nl)) {
+#pragma unroll
+        for (int q = 0; q < kRuns; ++q)
+          if (q == nruns - 1) rep[q] = l;
+        continue;
+      }
+      if (nruns == kRuns) {
+        nruns = 0;
+        break;
+      }
+#pragma unroll
+      for (int q = 1; q < kRuns; ++q)
+        if (q == nruns) {
+          rep[q] = l;
+          start[q] = l;
+        }
+      ++nruns;
+    }
+    int mine = 0, lead = rep[0];
+#pragma unroll
+    for (int q = 1; q < kRuns; ++q)
+      if (q < nruns && lane >= start[q]) {
+        mine = q;
+        lead = rep[q];
+      }
+    const int32_t nlead = __shfl_sync(0xffffffffu, len, lead);
+    const bool inside = !live || nlead == 0 || (row + off(lead, 0) >= 0 && row + off(lead, nlead - 1) < n);
+    if (!__all_sync(0xffffffffu, inside)) nruns = 0;
+    if (PASS == 0) {
+      if (lane == 0) words[sl] = nruns > 0 ? nruns * head : 32 * w;
+      __syncwarp();
+      continue;
+    }
+    // entries: a run's rows in the lead's slots, or in their own order
+    int32_t* t = tab ? tab + tptr[sl] : nullptr;
+    for (int32_t k = 0, q = 0; k < w; ++k) {
+      const int64_t j = b0 + 32 * (int64_t)k + lane;
+      const bool have = q < len && (nruns == 0 || off(lane, q) == off(lead, k));
+      const int32_t o = have ? off(lane, q) : 0;
+      cols[j] = live ? row + o : (int32_t)(n - 1);
+      src[j] = have ? (uint8_t)(buf[32 * q + lane] & 255) : (uint8_t)kRowMax;
+      if (t && nruns == 0) t[32 * k + lane] = o;
+      q += have;
+    }
+    int32_t nrep[kRuns];
+#pragma unroll
+    for (int q = 0; q < kRuns; ++q) nrep[q] = __shfl_sync(0xffffffffu, len, rep[q]);
+    if (t && nruns > 0) {  // piece p of run q starts at word nruns * kPiece * p + q * (the piece's padded entries)
+      for (int32_t k = lane; k < head; k += 32) {
+        const int32_t k0 = k / kPiece * kPiece, pk = min(kPiece, head - k0);
+#pragma unroll
+        for (int q = 0; q < kRuns; ++q) {
+          if (q >= nruns) continue;
+          t[nruns * k0 + q * pk + (k - k0)] = k < nrep[q] ? off(rep[q], k) : 0;
+        }
+      }
+    }
+    if (runs && lane == 0) runs[sl] = nruns > 0 ? start[1] | (start[2] << 8) | (start[3] << 16) : -1;
+    __syncwarp();
+  }
+}
+
+// int16 column offsets of the slices; *bad is raised when one does not fit
+__global__ void k_sell_c16(const int64_t* __restrict__ sptr, const int32_t* __restrict__ cols, int64_t n,
+                           int64_t nslices, int16_t* __restrict__ c16, int* __restrict__ bad) {
+  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < nslices * 32;
+       row += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b0 = sptr[row >> 5] + (row & 31), w = (sptr[(row >> 5) + 1] - sptr[row >> 5]) >> 5;
+    const int64_t self = row < n ? row : n - 1;
+    for (int64_t k = 0; k < w; ++k) {
+      const int64_t d = cols[b0 + 32 * k] - self;
+      if (d < -32768 || d > 32767) *bad = 1;
+      c16[b0 + 32 * k] = (int16_t)d;
+    }
+  }
+}
+
+// Per-slice column table of the bulk-copy SpMV: a slice whose 32 rows share one column-offset
+// sequence (every row of an interior stretch of a structured mesh line) stores it once
+// (w offsets, padded to 8 = 16 bytes); any other slice keeps its 32*w per-entry offsets.
+// len[s] = entries of slice s's table; the table of slice s starts at cptr[s] (a multiple of 8).
+__global__ void k_sell_uni_len(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
+                               int64_t* __restrict__ len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
+    const int64_t b0 = sptr[sl];
+    const int64_t w = (sptr[sl + 1] - b0) / 32;
+    bool uni = true;
+    for (int64_t k = 0; k < w && uni; ++k) {
+      const int16_t c = c16[b0 + 32 * k + lane];
+      uni = __all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0));
+    }
+    if (lane == 0) len[sl] = uni ? (w + 7) / 8 * 8 : 32 * w;
+  }
+}
+
+__global__ void k_sell_uni_fill(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
+                                const int64_t* __restrict__ cptr, int16_t* __restrict__ cu) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
+    const int64_t b0 = sptr[sl];
+    const int64_t w = (sptr[sl + 1] - b0) / 32;
+    const int64_t c0 = cptr[sl], len = cptr[sl + 1] - c0;
+    if (len == 32 * w) {
+      for (int64_t j = lane; j < len; j += 32) cu[c0 + j] = c16[b0 + j];
+    } else {
+      for (int64_t k = lane; k < len; k += 32) cu[c0 + k] = k < w ? c16[b0 + 32 * k] : (int16_t)0;
+    }
+  }
+}
+
+int build_uniform_columns(femk_plan* p, cudaStream_t s) {
+  if (!p->sell_uni) return FEMK_OK;
+  Temp len;
+  FEMK_CUDA_TRY(cudaMalloc(&len.p, sizeof(int64_t) * (p->n_slices + 1)));
+  FEMK_TRY(dev_alloc(&p->sell_cuptr, p->n_slices + 1));
+  const int sgrid = blocks_for(p->n_slices * 32, kThreads, p->n_sm * 64);
+  k_sell_uni_len<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
+                                                                       (int64_t*)len.p);
+  FEMK_TRY(scan_exclusive_i64((const int64_t*)len.p, p->sell_cuptr, p->n_slices, s));
+  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_cu_len, p->sell_cuptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost,
+                                s));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  FEMK_TRY(dev_alloc(&p->sell_cu, p->sell_cu_len));
+  k_sell_uni_fill<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
+                                                                        p->sell_cuptr, p->sell_cu);
+  FEMK_CUDA_TRY(cudaGetLastError());
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  return FEMK_OK;
+}
+
+int build_slices(femk_plan* p, cudaStream_t s) {
+  const int64_t n = p->n;
+  p->n_slices = (n + 31) / 32;
+  Temp slen;
+  FEMK_CUDA_TRY(cudaMalloc(&slen.p, sizeof(int64_t) * (p->n_slices + 1)));
+  FEMK_TRY(dev_alloc(&p->sell_ptr, p->n_slices + 1));
+  const int sgrid = grid_for(p, p->n_slices * 32);
+  k_sell_width<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->perm, n, p->n_slices, (int64_t*)slen.p);
+  FEMK_TRY(scan_exclusive_i64((const int64_t*)slen.p, p->sell_ptr, p->n_slices, s));
+  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_nnz, p->sell_ptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  if (p->sell_nnz >= INT32_MAX) {
+    p->use_sell = 0;
+    cudaFree(p->perm_base);
+    p->perm_base = nullptr;
+    p->perm = p->pos = nullptr;
+    return FEMK_OK;
+  }
+  FEMK_TRY(dev_alloc(&p->sell_cols, p->sell_nnz));
+  if (!p->perm) {
+    if (p->cols16) FEMK_TRY(dev_alloc(&p->sell_c16, p->sell_nnz));
+    k_sell_fill<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->indices, n, p->n_slices, p->sell_ptr,
+                                                              p->sell_cols, p->sell_c16);
+  } else {
+    FEMK_TRY(dev_alloc(&p->sell_src, p->sell_nnz));
+    const bool table = n > 65536 && p->sell_uni;
+    const int threads = 64, smem = threads * p->max_row * (int)sizeof(long long);
+    const int ogrid = blocks_for(p->n_slices * 32, threads, p->n_sm * 64);
+    if (table) {
+      FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      k_sell_order<0><<<counted_launch() + ogrid, threads, smem, s>>>(
+          p->indptr, p->indices, p->perm, p->pos, n, p->n_slices, p->sell_ptr, p->max_row, (int64_t*)slen.p, nullptr,
+          nullptr, nullptr, nullptr, nullptr);
+      p->sell_ctptr = (int64_t*)p->perm_base;
+      FEMK_TRY(scan_exclusive_i64((const int64_t*)slen.p, p->sell_ctptr, p->n_slices, s));
+      FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_ct_len, p->sell_ctptr + p->n_slices, sizeof(int64_t),
+                                    cudaMemcpyDeviceToHost, s));
+      FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+      FEMK_TRY(dev_alloc(&p->sell_ct, p->sell_ct_len));
+      p->sell_runs = p->pos + n;
+    }
+    FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_sell_order<1><<<counted_launch() + ogrid, threads, smem, s>>>(
+        p->indptr, p->indices, p->perm, p->pos, n, p->n_slices, p->sell_ptr, p->max_row, nullptr, p->sell_cols,
+        p->sell_src, p->sell_ctptr, p->sell_ct, p->sell_runs);
+    if (n <= 65536) {  // larger systems have offsets past 16 bits for certain: the last class is n / 8 rows away
+      Temp bad;
+      int h = 0;
+      FEMK_CUDA_TRY(cudaMalloc(&bad.p, sizeof(int)));
+      FEMK_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
+      FEMK_TRY(dev_alloc(&p->sell_c16, p->sell_nnz));
+      k_sell_c16<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_cols, n, p->n_slices, p->sell_c16,
+                                                               (int*)bad.p);
+      FEMK_CUDA_TRY(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+      FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+      if (h) {
+        cudaFree(p->sell_c16);
+        p->sell_c16 = nullptr;
+      }
+    }
+  }
+  FEMK_CUDA_TRY(cudaGetLastError());
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  return p->sell_c16 ? build_uniform_columns(p, s) : FEMK_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// values and vectors in the solver's order
+// ---------------------------------------------------------------------------------------------
+__global__ void k_permute_in(const int32_t* __restrict__ perm, int64_t n, const double* __restrict__ b,
+                             const double* __restrict__ x, const double* __restrict__ d, double* __restrict__ bs,
+                             double* __restrict__ xs, double* __restrict__ ds) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t j = perm[i];
+    if (b) bs[i] = b[j];
+    if (x) xs[i] = x[j];
+    if (d) ds[i] = d[j];
+  }
+}
+
+__global__ void k_permute_out(const int32_t* __restrict__ perm, int64_t n, const double* __restrict__ xs,
+                              double* __restrict__ x) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    x[perm[i]] = xs[i];
+}
+
+}  // namespace
+
+int build_sell(femk_plan* p, cudaStream_t s) {
+  FEMK_TRY(build_order(p, s));
+  return build_slices(p, s);
+}
+
+int natural_order(femk_plan* p, cudaStream_t s) {
+  if (!p->perm) return FEMK_OK;
+  FEMK_CUDA_TRY(cudaDeviceSynchronize());  // nothing may still read what is freed here
+  auto drop = [](auto*& q) {
+    if (q) cudaFree(q);
+    q = nullptr;
+  };
+  cudaFree(p->perm_base);
+  p->perm_base = nullptr;
+  p->perm = p->pos = p->sell_runs = nullptr;
+  p->sell_ctptr = nullptr;
+  drop(p->sell_src);
+  drop(p->sell_ptr);
+  drop(p->sell_cols);
+  drop(p->sell_c16);
+  drop(p->sell_cuptr);
+  drop(p->sell_cu);
+  drop(p->sell_ct);
+  drop(p->sell_vals);
+  drop(p->sell_vals32);
+  for (cudaGraphExec_t* e : {&p->cg_exec, &p->mx_exec, &p->bicg_exec})
+    if (*e) {
+      cudaGraphExecDestroy(*e);
+      *e = nullptr;
+    }
+  return build_slices(p, s);
+}
+
+int permute_in(femk_plan* p, const double** b, double** x, const double** dinv, cudaStream_t s) {
+  if (!p->perm_ws) FEMK_TRY(dev_alloc(&p->perm_ws, 3 * p->vstride));
+  double* bs = p->perm_ws;
+  double* xs = bs + p->vstride;
+  double* ds = xs + p->vstride;
+  k_permute_in<<<counted_launch() + blocks_for(p->n, kThreads, p->n_sm * 8), kThreads, 0, s>>>(
+      p->perm, p->n, b ? *b : nullptr, x ? *x : nullptr, dinv ? *dinv : nullptr, bs, xs, ds);
+  FEMK_CUDA_TRY(cudaGetLastError());
+  if (b) *b = bs;
+  if (x) *x = xs;
+  if (dinv && *dinv) *dinv = ds;
+  return FEMK_OK;
+}
+
+int permute_out(const femk_plan* p, const double* xs, double* x, cudaStream_t s) {
+  k_permute_out<<<counted_launch() + blocks_for(p->n, kThreads, p->n_sm * 8), kThreads, 0, s>>>(p->perm, p->n, xs, x);
+  FEMK_CUDA_TRY(cudaGetLastError());
+  return FEMK_OK;
+}
+
+}  // namespace femk

@@ -165,14 +165,10 @@ __global__ void k_p2_cells(const int32_t* __restrict__ tets, int64_t ntet, int64
   }
 }
 
-__device__ __forceinline__ int warp_min_i32(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // Row pattern by repeated warp-wide minimum extraction over the candidate dofs of a row's
-// incident elements: no sort, deterministic, each row's columns ascending.
+// incident elements: no sort, deterministic, each row's columns ascending. Up to 32 kHeld candidates
+// (a P2 vertex of the Kuhn lattice has 240) are read once into registers: reading them again for
+// every minimum took 5.5 ms of a P2 37x45x41 plan, this 2.0 ms.
 template <int ND>
 __global__ void k_row_pattern(const int32_t* __restrict__ cells, const int32_t* __restrict__ inc_ptr,
                               const int32_t* __restrict__ inc, int64_t n, const int64_t* __restrict__ rowptr,
@@ -186,14 +182,30 @@ __global__ void k_row_pattern(const int32_t* __restrict__ cells, const int32_t* 
     int prev = -1;
     int32_t count = 0;
     const int64_t out = cols ? rowptr[row] : 0;
+    constexpr int kHeld = 10;
+    const bool held = m <= 32 * kHeld;
+    int have[kHeld];
+    if (held) {
+#pragma unroll
+      for (int u = 0; u < kHeld; ++u) {
+        const int32_t idx = lane + 32 * u;
+        have[u] = INT_MAX;
+        if (idx < m) have[u] = cells[(int64_t)inc[beg + idx / ND] * ND + idx % ND];
+      }
+    }
     while (true) {
       int best = INT_MAX;
-      for (int32_t idx = lane; idx < m; idx += 32) {
+      if (held) {
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u)
+          if (have[u] > prev && have[u] < best) best = have[u];
+      }
+      for (int32_t idx = held ? m : lane; idx < m; idx += 32) {
         const int32_t c = inc[beg + idx / ND];
         const int v = cells[(int64_t)c * ND + idx % ND];
         if (v > prev && v < best) best = v;
       }
-      best = warp_min_i32(best);
+      best = __reduce_min_sync(0xffffffffu, best);
       if (best == INT_MAX) break;
       if (cols && lane == 0) cols[out + count] = best;
       ++count;
@@ -308,55 +320,19 @@ __global__ void k_block_span(const int32_t* __restrict__ indptr, int64_t n, int 
   }
 }
 
-// Width of each 32-row slice (its longest row) and its entry count.
-__global__ void k_sell_width(const int32_t* __restrict__ indptr, int64_t n, int64_t nslices, int64_t* __restrict__ len) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t row = sl * 32 + lane;
-    int w = row < n ? indptr[row + 1] - indptr[row] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
-    if (lane == 0) len[sl] = (int64_t)w * 32;
-  }
-}
-
-__global__ void k_sell_fill(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
-                            int64_t nslices, const int64_t* __restrict__ sptr, int32_t* __restrict__ cols,
-                            int16_t* __restrict__ c16) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t row = sl * 32 + lane;
-    const int64_t w = (sptr[sl + 1] - sptr[sl]) / 32;
-    const int32_t beg = row < n ? indptr[row] : 0;
-    const int32_t len = row < n ? indptr[row + 1] - beg : 0;
-    const int64_t self = row < n ? row : n - 1;
-    for (int64_t k = 0; k < w; ++k) {
-      const int64_t j = sptr[sl] + k * 32 + lane;
-      const bool real = k < len;
-      const int32_t col = real ? indices[beg + k] : (int32_t)self;
-      cols[j] = col;
-      if (c16) c16[j] = (int16_t)(col - self);
-    }
+// whether a row's columns (ascending) lie past int16 offsets
+__global__ void k_cols16_fit(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
+                             int* __restrict__ bad) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t beg = indptr[i], end = indptr[i + 1];
+    if (beg < end && (indices[beg] - i < -32768 || indices[end - 1] - i > 32767)) *bad = 1;
   }
 }
 
 __global__ void k_cols16(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t n,
-                         int16_t* __restrict__ c16, int* __restrict__ bad) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    for (int32_t k = indptr[i]; k < indptr[i + 1]; ++k) {
-      const int64_t d = (int64_t)indices[k] - i;
-      if (d < -32768 || d > 32767) {
-        atomicOr(bad, 1);
-        c16[k] = 0;
-      } else {
-        c16[k] = (int16_t)d;
-      }
-    }
-  }
+                         int16_t* __restrict__ c16) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    for (int32_t k = indptr[i]; k < indptr[i + 1]; ++k) c16[k] = (int16_t)(indices[k] - i);
 }
 
 // coordinates with dim components per vertex -> 3 per vertex (z = 0 in 2-D) in a (and b)
@@ -422,8 +398,6 @@ int build_incidence(const int32_t* cells, int64_t ntet, int64_t n, int32_t** ptr
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));  // temporaries are freed on return
   return FEMK_OK;
 }
-
-int build_uniform_columns(femk_plan* p, cudaStream_t s);
 
 template <int ND>
 int build_pattern(femk_plan* p, int* d_err, int* h_err, cudaStream_t s) {
@@ -496,93 +470,17 @@ int build_pattern(femk_plan* p, int* d_err, int* h_err, cudaStream_t s) {
   Temp bad;
   bad.p = d_bad;
   FEMK_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
-  FEMK_TRY(dev_alloc(&p->cols16, nnz, s));
-  k_cols16<<<::femk::counted_launch() + blocks_for(n, kThreads, 65535 * 4), kThreads, 0, s>>>(p->indptr, p->indices, n, p->cols16, d_bad);
+  k_cols16_fit<<<::femk::counted_launch() + blocks_for(n, kThreads, 65535 * 4), kThreads, 0, s>>>(
+      p->indptr, p->indices, n, d_bad);
   int hbad = 0;
   FEMK_TRY(read_err(d_bad, s, &hbad));
-  if (hbad) {
-    cudaFree(p->cols16);
-    p->cols16 = nullptr;
+  if (!hbad) {
+    FEMK_TRY(dev_alloc(&p->cols16, nnz, s));
+    k_cols16<<<::femk::counted_launch() + blocks_for(n, kThreads, 65535 * 4), kThreads, 0, s>>>(p->indptr, p->indices,
+                                                                                                n, p->cols16);
   }
   // sliced-ELL copy of the pattern for the solver
-  p->n_slices = (n + 31) / 32;
-  Temp slen;
-  FEMK_CUDA_TRY(cudaMalloc(&slen.p, sizeof(int64_t) * (p->n_slices + 1)));
-  FEMK_TRY(dev_alloc(&p->sell_ptr, p->n_slices + 1, s));
-  const int sgrid = blocks_for(p->n_slices * 32, kThreads, p->n_sm * 64);
-  k_sell_width<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, n, p->n_slices, (int64_t*)slen.p);
-  FEMK_TRY(scan_exclusive_i64((const int64_t*)slen.p, p->sell_ptr, p->n_slices, s));
-  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_nnz, p->sell_ptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  if (p->sell_nnz >= INT32_MAX) {
-    p->use_sell = 0;
-    return FEMK_OK;
-  }
-  FEMK_TRY(dev_alloc(&p->sell_cols, p->sell_nnz, s));
-  if (p->cols16) FEMK_TRY(dev_alloc(&p->sell_c16, p->sell_nnz, s));
-  k_sell_fill<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->indices, n, p->n_slices, p->sell_ptr,
-                                                                    p->sell_cols, p->sell_c16);
-  FEMK_CUDA_TRY(cudaGetLastError());
-  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  return build_uniform_columns(p, s);
-}
-
-// Per-slice column table of the bulk-copy SpMV: a slice whose 32 rows share one column-offset
-// sequence (every row of an interior stretch of a structured mesh line) stores it once
-// (w offsets, padded to 8 = 16 bytes); any other slice keeps its 32*w per-entry offsets.
-// len[s] = entries of slice s's table; the table of slice s starts at cptr[s] (a multiple of 8).
-__global__ void k_sell_uni_len(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
-                               int64_t* __restrict__ len) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t b0 = sptr[sl];
-    const int64_t w = (sptr[sl + 1] - b0) / 32;
-    bool uni = true;
-    for (int64_t k = 0; k < w && uni; ++k) {
-      const int16_t c = c16[b0 + 32 * k + lane];
-      uni = __all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0));
-    }
-    if (lane == 0) len[sl] = uni ? (w + 7) / 8 * 8 : 32 * w;
-  }
-}
-
-__global__ void k_sell_uni_fill(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
-                                const int64_t* __restrict__ cptr, int16_t* __restrict__ cu) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t b0 = sptr[sl];
-    const int64_t w = (sptr[sl + 1] - b0) / 32;
-    const int64_t c0 = cptr[sl], len = cptr[sl + 1] - c0;
-    if (len == 32 * w) {
-      for (int64_t j = lane; j < len; j += 32) cu[c0 + j] = c16[b0 + j];
-    } else {
-      for (int64_t k = lane; k < len; k += 32) cu[c0 + k] = k < w ? c16[b0 + 32 * k] : (int16_t)0;
-    }
-  }
-}
-
-int build_uniform_columns(femk_plan* p, cudaStream_t s) {
-  if (!p->sell_c16 || !p->sell_uni) return FEMK_OK;
-  Temp len;
-  FEMK_CUDA_TRY(cudaMalloc(&len.p, sizeof(int64_t) * (p->n_slices + 1)));
-  FEMK_TRY(dev_alloc(&p->sell_cuptr, p->n_slices + 1, s));
-  const int sgrid = blocks_for(p->n_slices * 32, kThreads, p->n_sm * 64);
-  k_sell_uni_len<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
-                                                                       (int64_t*)len.p);
-  FEMK_TRY(scan_exclusive_i64((const int64_t*)len.p, p->sell_cuptr, p->n_slices, s));
-  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_cu_len, p->sell_cuptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                s));
-  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  FEMK_TRY(dev_alloc(&p->sell_cu, p->sell_cu_len, s));
-  k_sell_uni_fill<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
-                                                                        p->sell_cuptr, p->sell_cu);
-  FEMK_CUDA_TRY(cudaGetLastError());
-  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  return FEMK_OK;
+  return build_sell(p, s);
 }
 
 // Assembly stream of the parametric assembly (femk_assemble): the geometry of a mesh does not change
@@ -839,7 +737,8 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
                   p->sell_ptr, p->sell_cols, p->sell_c16,  p->sell_vals, p->sell_vals32,
                   p->bar,      p->batch_ws,  p->bicg_ws,   p->bicg_state, p->sell_cuptr, p->sell_cu,
                   p->coef_tmp, p->theta_ws, p->cmp_ws, p->gm_ws, p->dev_err, p->astr_ptr, p->astr_elem,
-                  p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn, p->persist_ws};
+                  p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn, p->persist_ws,
+                  p->perm_base, p->sell_src, p->sell_ct, p->perm_ws};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (p->state_host) cudaFreeHost(p->state_host);

@@ -57,6 +57,37 @@ __device__ __forceinline__ void sell_transpose_warp(double* wbuf, int32_t cap, c
   }
 }
 
+// The same for a plan with a row order of its own (femk_order.cu): lane l of a slice reads the CSR row of its DOF,
+// entry k from place src of it (255: padding).
+template <typename T, typename F>
+__device__ __forceinline__ void sell_order_warp(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr,
+                                                const int32_t* __restrict__ perm, const uint8_t* __restrict__ src,
+                                                int64_t n, int64_t nslices, const double* __restrict__ vals,
+                                                int64_t nnz, T* __restrict__ out, int64_t g, int64_t NW, F f,
+                                                int* err) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t sl = g; sl < nslices; sl += NW) {
+    const int64_t row = sl * 32 + lane;
+    const int32_t beg = row < n ? __ldg(indptr + __ldg(perm + row)) : 0;
+    const int64_t b0 = __ldg(sptr + sl) + lane;
+    const int32_t w = (int32_t)((__ldg(sptr + sl + 1) - __ldg(sptr + sl)) >> 5);
+    for (int32_t k0 = 0; k0 < w; k0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int32_t q = k0 + u < w && row < n ? (int32_t)__ldg(src + b0 + 32 * (k0 + u)) : 255;
+        v[u] = q != 255 && FEMK_IN_BOUNDS(beg + q, nnz, err) ? __ldg(vals + beg + q) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (k0 + u < w) {
+          const int64_t j = b0 + 32 * (k0 + u);
+          out[j] = f(v[u], row, j);
+        }
+    }
+  }
+}
+
 // gather functors: x[j], or the CG direction z[j] + beta p[j] formed on the fly
 template <typename V>
 struct GatherX {
