@@ -444,12 +444,34 @@ __global__ void __launch_bounds__(kThreads) k_pupdate(int64_t n, double* __restr
 // Every value is formed by the same floating-point operations as in k_update + k_pupdate. The
 // iteration that meets the stop test still owes its x update: k_update_r raises st->xpend, the
 // direction kernel applies x (and p only while the solve runs), and the next CG-step SpMV clears it.
-template <bool H>
+// SUM: <p, q> comes as npq block shares in pq, which every block adds up in the same order before it starts.
+template <bool H, bool SUM = false>
 __global__ void __launch_bounds__(kThreads) k_update_r(int64_t n, double* __restrict__ r, const double* __restrict__ q,
                                                       const double* __restrict__ dinv, double* __restrict__ partials,
-                                                      CgState* st) {
+                                                      CgState* st, const double* __restrict__ pq, int npq) {
   if (st->done) return;
-  const double alpha = st->alpha;
+  double alpha = st->alpha;
+  if (SUM) {
+    __shared__ double share[kThreads / 32];
+    double t = 0.0;
+    for (int b = threadIdx.x; b < npq; b += kThreads) t += __ldg(pq + b);
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) share[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) t += share[w];
+    alpha = st->gamma / t;  // gamma changes once every block has passed here (the last block's finish)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      st->pq = t;
+      st->alpha = alpha;
+      if (!(t > 0.0) || !isfinite(t)) {
+        st->status = isfinite(t) ? FEMK_BREAKDOWN : FEMK_NONFINITE;
+        st->done = 1;
+      }
+    }
+    if (!(t > 0.0) || !isfinite(t)) return;
+  }
   double acc[2] = {0.0, 0.0};
   const int64_t tid = blockIdx.x * (int64_t)kThreads + threadIdx.x;
   const int64_t nt = (int64_t)gridDim.x * kThreads;
@@ -517,10 +539,11 @@ __global__ void __launch_bounds__(kThreads) k_update_r(int64_t n, double* __rest
   }
 }
 
-template <bool H>
+// ZERO: q = 0 as well, for the matrix-free step that adds into it
+template <bool H, bool ZERO = false>
 __global__ void __launch_bounds__(kThreads) k_pupdate_x(int64_t n, double* __restrict__ x, double* __restrict__ p,
                                                        const double* __restrict__ r, const double* __restrict__ dinv,
-                                                       const CgState* st) {
+                                                       double* __restrict__ q, const CgState* st) {
   if (!st->xpend) return;
   const bool dir = !st->done;
   const double alpha = st->alpha, beta = st->beta;
@@ -546,12 +569,14 @@ __global__ void __launch_bounds__(kThreads) k_pupdate_x(int64_t n, double* __res
       const double2 da = dinv ? ld(d2 + i) : make_double2(1.0, 1.0);
       st2(x2 + i, make_double2(fma(alpha, pa.x, xa.x), fma(alpha, pa.y, xa.y)));
       st2(p2 + i, make_double2(fma(beta, pa.x, da.x * ra.x), fma(beta, pa.y, da.y * ra.y)));
+      if (ZERO) st2(reinterpret_cast<double2*>(q) + i, make_double2(0.0, 0.0));
     }
     if ((n & 1) && tid == 0) {
       const int64_t i = n - 1;
       const double pi = p[i];
       x[i] = fma(alpha, pi, x[i]);
       p[i] = fma(beta, pi, (dinv ? dinv[i] : 1.0) * r[i]);
+      if (ZERO) q[i] = 0.0;
     }
   } else {
     for (int64_t i = tid; i < n2; i += nt) {
@@ -566,17 +591,56 @@ __global__ void __launch_bounds__(kThreads) k_pupdate_x(int64_t n, double* __res
 // matrix-free operator: y = A x, A the Dirichlet-eliminated stiffness, recomputed per element from
 // the vertex coordinates (thread per element, FP64 atomics into y). mcells is the connectivity with
 // each Dirichlet DOF d stored as -1 - d, so one load gives the DOF and its mask: a Dirichlet DOF
-// contributes x = 0 and receives nothing (its row is the identity, k_dirichlet_identity).
+// contributes x = 0 and receives nothing; its row is the identity, which the same launch writes. y is zero on entry.
+//
+// In the CG loop (DOT) the launch also forms its blocks' shares of <p, A p>: every element adds
+// x_e . k_e K_hat_e x_e, a non-negative term of the sum, every Dirichlet DOF x_d^2. k_update_r adds them up: a
+// last-block sum here would wait, before its ticket, for the atomics of every block (46 against 41 us at P1
+// 92x104x87, P2 36x40x38 25 against 17). So a CG step is this launch, k_update_r and k_pupdate_x, which zeroes q for
+// the next one: separate kernels for zeroing, the Dirichlet rows and the dot product took 12.3 us and three gaps
+// of the 79 us an iteration at P1 92x104x87.
 // ---------------------------------------------------------------------------------------------
-// (P2 tetrahedra: 6 resident blocks per SM fit the product in 80 registers without spills)
-template <int ND>
-__global__ void __launch_bounds__(128, ND == 10 ? 6 : 8) k_matfree(const double* __restrict__ xyz,
-                                                                   const int32_t* __restrict__ mcells,
-                                                 int64_t ntet, const double* __restrict__ param, int mode, double scale,
-                                                 const double* __restrict__ x, double* __restrict__ y,
-                                                 const CgState* st) {
+struct MatfreeArgs {
+  const double* xyz;
+  const int32_t* conn;   // masked connectivity (k_matfree) or corners of the Kuhn blocks (k_matfree_kuhn)
+  int64_t count;         // elements or blocks
+  const double* param;
+  int mode;
+  double scale;
+  const double* x;
+  double* y;
+  const int32_t* dlist;  // Dirichlet DOFs
+  int64_t ndir;
+  double* partials;
+  CgState* st;
+};
+
+// The Dirichlet rows, and with DOT the block's share of <x, A x>; acc0: the thread's share over its elements.
+template <bool DOT>
+__device__ __forceinline__ void matfree_finish(const MatfreeArgs& a, double acc0) {
+  double acc[1] = {acc0};
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < a.ndir; t += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t d = __ldg(a.dlist + t);
+    const double xd = __ldg(a.x + d);
+    a.y[d] = xd;
+    acc[0] += xd * xd;
+  }
+  if (DOT) block_reduce_store<1, 128>(acc, a.partials);
+}
+
+// (P2 tetrahedra: 6 resident blocks per SM fit the plain product in 80 registers without spills; with the dot product
+// 4 blocks of 116 take 18.2 us at 36x40x38, 5 with spills 19.5, 6 20.6)
+template <int ND, bool DOT>
+__global__ void __launch_bounds__(128, ND == 10 ? (DOT ? 4 : 6) : (ND == 6 ? 7 : 8)) k_matfree(MatfreeArgs a) {
   constexpr int NV = Cell<ND>::NV;
-  if (st && st->done) return;
+  if (DOT && blockIdx.x == 0 && threadIdx.x == 0) a.st->xpend = 0;  // the last x update is applied
+  if (DOT && a.st->done) return;
+  const double* __restrict__ xyz = a.xyz;
+  const int32_t* __restrict__ mcells = a.conn;
+  const double* __restrict__ x = a.x;
+  double* __restrict__ y = a.y;
+  const int64_t ntet = a.count;
+  double acc = 0.0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ntet; c += (int64_t)gridDim.x * blockDim.x) {
     int32_t dof[ND];
     double xe[ND];
@@ -588,14 +652,14 @@ __global__ void __launch_bounds__(128, ND == 10 ? 6 : 8) k_matfree(const double*
       dof[3] = d4.w;
     } else {
 #pragma unroll
-      for (int a = 0; a < ND; ++a) dof[a] = __ldg(mcells + c * ND + a);
+      for (int i = 0; i < ND; ++i) dof[i] = __ldg(mcells + c * ND + i);
     }
 #pragma unroll
-    for (int a = 0; a < ND; ++a) xe[a] = dof[a] >= 0 ? __ldg(x + dof[a]) : 0.0;
+    for (int i = 0; i < ND; ++i) xe[i] = dof[i] >= 0 ? __ldg(x + dof[i]) : 0.0;
     int32_t v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = dof[i] >= 0 ? dof[i] : -1 - dof[i];
-    const double k = coef_of(param, mode, scale, c);
+    const double k = coef_of(a.param, a.mode, a.scale, c);
     double ye[ND];
     if constexpr (!Cell<ND>::P2) {
       double P[NV][3];
@@ -612,9 +676,13 @@ __global__ void __launch_bounds__(128, ND == 10 ? 6 : 8) k_matfree(const double*
       khat_apply<ND>(VG, xe, ye);
     }
 #pragma unroll
-    for (int a = 0; a < ND; ++a)
-      if (dof[a] >= 0) atomicAdd(y + dof[a], k * ye[a]);
+    for (int i = 0; i < ND; ++i)
+      if (dof[i] >= 0) {
+        atomicAdd(y + dof[i], k * ye[i]);
+        if (DOT) acc += xe[i] * (k * ye[i]);
+      }
   }
+  matfree_finish<DOT>(a, acc);
 }
 
 // Kuhn blocks: six consecutive tetrahedra that split one hexahedron, tet e of a block being the
@@ -659,15 +727,20 @@ __global__ void k_kuhn_corners(const int32_t* __restrict__ mcells, int64_t nhex,
 // y += A x over whole Kuhn blocks: one thread loads a hexahedron's 8 corners, their coordinates and
 // x once (six separate elements load 24 of each), applies the six element operators (p1_apply, the
 // local indices compile-time constants) and adds into the 8 corners with 8 atomics in place of 24.
-__global__ void __launch_bounds__(128) k_matfree_kuhn(const double* __restrict__ xyz,
-                                                      const int32_t* __restrict__ corners, int64_t nhex,
-                                                      const double* __restrict__ param, int mode, double scale,
-                                                      const double* __restrict__ x, double* __restrict__ y,
-                                                      const CgState* st) {
-  if (st && st->done) return;
-  for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < nhex; h += (int64_t)gridDim.x * blockDim.x) {
-    const int4 c0 = __ldg(reinterpret_cast<const int4*>(corners) + 2 * h);
-    const int4 c1 = __ldg(reinterpret_cast<const int4*>(corners) + 2 * h + 1);
+// 4 blocks an SM (128 registers, 36 bytes spilled with the dot product): 43.9 us at 92x104x87, 3 and 5 blocks 54 and
+// 51. Slower too: the six tetrahedra as a ring around the diagonal, sharing cross products (46 us at best: its
+// chain is longer and it holds more); handing shared corners to the next lane in place of 4 atomics (+1.5 us);
+// two threads a hexahedron with three tetrahedra each (55 us).
+template <bool DOT>
+__global__ void __launch_bounds__(128, 4) k_matfree_kuhn(MatfreeArgs a) {
+  if (DOT && blockIdx.x == 0 && threadIdx.x == 0) a.st->xpend = 0;  // the last x update is applied
+  if (DOT && a.st->done) return;
+  const double* __restrict__ xyz = a.xyz;
+  const double* __restrict__ x = a.x;
+  double acc = 0.0;
+  for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < a.count; h += (int64_t)gridDim.x * blockDim.x) {
+    const int4 c0 = __ldg(reinterpret_cast<const int4*>(a.conn) + 2 * h);
+    const int4 c1 = __ldg(reinterpret_cast<const int4*>(a.conn) + 2 * h + 1);
     const int32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
     double X[8][3], xv[8], ys[8];
 #pragma unroll
@@ -688,14 +761,17 @@ __global__ void __launch_bounds__(128) k_matfree_kuhn(const double* __restrict__
         xe[i] = xv[kuhn_corner(e, i)];
       }
       p1_apply(P, xe, ye);
-      const double k = coef_of(param, mode, scale, 6 * h + e);
+      const double k = coef_of(a.param, a.mode, a.scale, 6 * h + e);
 #pragma unroll
       for (int i = 0; i < 4; ++i) ys[kuhn_corner(e, i)] += k * ye[i];
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (c[u] >= 0) atomicAdd(y + c[u], ys[u]);
+    for (int u = 0; u < 8; ++u) {
+      if (DOT) acc += xv[u] * ys[u];
+      if (c[u] >= 0) atomicAdd(a.y + c[u], ys[u]);
+    }
   }
+  matfree_finish<DOT>(a, acc);
 }
 
 // the masked connectivity of the matrix-free operator
@@ -704,15 +780,6 @@ __global__ void k_mask_cells(const int32_t* __restrict__ cells, int64_t len, con
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < len; t += (int64_t)gridDim.x * blockDim.x) {
     const int32_t d = cells[t];
     mcells[t] = dmask[d] ? -1 - d : d;
-  }
-}
-
-__global__ void k_dirichlet_identity(const int32_t* __restrict__ dlist, int64_t nd, const double* __restrict__ x,
-                                     double* __restrict__ y, const CgState* st) {
-  if (st && st->done) return;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nd; t += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t d = dlist[t];
-    y[d] = x[d];
   }
 }
 
@@ -735,31 +802,29 @@ __global__ void k_matfree_diag(const double* __restrict__ xyz, const int32_t* __
   }
 }
 
-// The rest of a CG step for the matrix-free operator: <p, q> (q already holds A p)
-__global__ void __launch_bounds__(kThreads) k_dot_pq(int64_t n, const double* __restrict__ p, const double* __restrict__ q,
-                                                    double* __restrict__ partials, CgState* st) {
+// <p, q> and alpha from the product's block shares, for the vector kernels of unaligned caller vectors
+__global__ void __launch_bounds__(kThreads) k_sum_pq(const double* __restrict__ pq, int npq, CgState* st) {
   if (st->done) return;
-  double acc[1] = {0.0};
-  for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads)
-    acc[0] += p[i] * q[i];
-  block_reduce_store<1>(acc, partials);
-  double tot[1];
-  if (!grid_finish<1>(partials, &st->ticket, tot)) return;
+  __shared__ double share[kThreads / 32];
+  double t = 0.0;
+  for (int b = threadIdx.x; b < npq; b += kThreads) t += pq[b];
+  t = warp_sum(t);
+  if ((threadIdx.x & 31) == 0) share[threadIdx.x >> 5] = t;
+  __syncthreads();
   if (threadIdx.x != 0) return;
-  st->pq = tot[0];
-  st->alpha = st->gamma / tot[0];
-  if (!isfinite(tot[0])) {
-    st->status = FEMK_NONFINITE;
-    st->done = 1;
-  } else if (!(tot[0] > 0.0)) {
-    st->status = FEMK_BREAKDOWN;
+  double sum = 0.0;
+  for (int w = 0; w < kThreads / 32; ++w) sum += share[w];
+  st->pq = sum;
+  st->alpha = st->gamma / sum;
+  if (!(sum > 0.0) || !isfinite(sum)) {
+    st->status = isfinite(sum) ? FEMK_BREAKDOWN : FEMK_NONFINITE;
     st->done = 1;
   }
 }
 
-// r = b - y (y = A x), z = D^-1 r, p = z and the init dots (matrix-free init)
+// r = b - y (y = A x), z = D^-1 r, p = z and the init dots (matrix-free init); y is zeroed for the first step
 __global__ void __launch_bounds__(kThreads) k_init_from_ax(int64_t n, const double* __restrict__ b,
-                                                          const double* __restrict__ ax, const double* __restrict__ dinv,
+                                                          double* __restrict__ ax, const double* __restrict__ dinv,
                                                           double* __restrict__ r, double* __restrict__ z,
                                                           double* __restrict__ p, double* __restrict__ partials,
                                                           CgState* st, double tol2, double atol2) {
@@ -767,6 +832,7 @@ __global__ void __launch_bounds__(kThreads) k_init_from_ax(int64_t n, const doub
   for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
     const double bi = b[i];
     const double ri = bi - ax[i];
+    ax[i] = 0.0;
     const double zi = dinv ? dinv[i] * ri : ri;
     r[i] = ri;
     z[i] = zi;
@@ -861,16 +927,22 @@ bool split_ok(const femk_plan* p, const double* x, const double* dinv) {
   return p->cg_split && aligned16(x) && (dinv == nullptr || aligned16(dinv));
 }
 
+// npq: block shares of <p, q> left by the matrix-free product past kPqShares (0: st->alpha is formed already)
+constexpr int64_t kPqShares = 16384;
 void launch_update_r(const femk_plan* p, double* r, const double* q, const double* dinv, CgState* st,
-                     cudaStream_t s) {
-  auto kern = p->l2_mode != 0 ? k_update_r<true> : k_update_r<false>;
-  kern<<<::femk::counted_launch() + vec_grid(kern, kThreads, p), kThreads, 0, s>>>(p->n, r, q, dinv, p->partials, st);
+                     cudaStream_t s, int npq = 0) {
+  auto kern = npq ? (p->l2_mode != 0 ? k_update_r<true, true> : k_update_r<false, true>)
+                  : (p->l2_mode != 0 ? k_update_r<true> : k_update_r<false>);
+  kern<<<::femk::counted_launch() + vec_grid(kern, kThreads, p), kThreads, 0, s>>>(p->n, r, q, dinv, p->partials, st,
+                                                                                  p->partials + kPqShares, npq);
 }
 
-void launch_pupdate_x(const femk_plan* p, double* x, double* pv, const double* r, const double* dinv,
+// zero_q: q = 0 too (NULL: not)
+void launch_pupdate_x(const femk_plan* p, double* x, double* pv, const double* r, const double* dinv, double* zero_q,
                       const CgState* st, cudaStream_t s) {
-  auto kern = p->l2_mode != 0 ? k_pupdate_x<true> : k_pupdate_x<false>;
-  kern<<<::femk::counted_launch() + vec_grid(kern, kThreads, p), kThreads, 0, s>>>(p->n, x, pv, r, dinv, st);
+  auto kern = zero_q ? (p->l2_mode != 0 ? k_pupdate_x<true, true> : k_pupdate_x<false, true>)
+                     : (p->l2_mode != 0 ? k_pupdate_x<true> : k_pupdate_x<false>);
+  kern<<<::femk::counted_launch() + vec_grid(kern, kThreads, p), kThreads, 0, s>>>(p->n, x, pv, r, dinv, zero_q, st);
 }
 
 template <int MODE>
@@ -1034,13 +1106,11 @@ struct MatFree {
   double scale;
 };
 
-__global__ void k_zero(double* __restrict__ y, int64_t n, const CgState* st) {
-  if (st && st->done) return;
+__global__ void k_zero(double* __restrict__ y, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = 0.0;
 }
 
-// y = A x for the matrix-free operator; with st != NULL every launch is a no-op once st->done.
 // the masked connectivity, built on first use (the Dirichlet set of a plan is fixed), and on a P1
 // tetrahedral plan the Kuhn-block check (once, with a synchronous read of its flag)
 int ensure_mcells(const femk_plan* pc, cudaStream_t s) {
@@ -1081,22 +1151,30 @@ int ensure_mcells(const femk_plan* pc, cudaStream_t s) {
   return FEMK_OK;
 }
 
-int launch_matfree(const femk_plan* p, const MatFree& m, const double* x, double* y, cudaStream_t s,
-                   const CgState* st = nullptr) {
-  FEMK_TRY(ensure_mcells(p, s));
-  k_zero<<<::femk::counted_launch() + p->n_sm * 8, 256, 0, s>>>(y, p->n, st);
-  const int grid = blocks_for(p->ntet, 128, p->n_sm * 16);
+// DOT: *shares block shares of <x, A x> in p->partials + kPqShares
+template <bool DOT>
+int launch_matfree_product(const femk_plan* p, const MatFree& m, const double* x, double* y, CgState* st,
+                           cudaStream_t s, int* shares = nullptr) {
+  MatfreeArgs a{p->xyz, p->kuhn ? p->kuhn : p->mcells, p->kuhn ? p->ntet / 6 : p->ntet, m.param, m.mode, m.scale, x, y,
+                p->dlist, p->n_dir, p->partials + kPqShares, st};
+  auto launch = [&](auto kern) {
+    const int grid = blocks_for(std::max(a.count, a.ndir), 128, p->n_sm * 16);
+    if (DOT) *shares = grid;
+    kern<<<::femk::counted_launch() + grid, 128, 0, s>>>(a);
+  };
   if (p->kuhn)
-    k_matfree_kuhn<<<::femk::counted_launch() + blocks_for(p->ntet / 6, 128, p->n_sm * 16), 128, 0, s>>>(
-        p->xyz, p->kuhn, p->ntet / 6, m.param, m.mode, m.scale, x, y, st);
+    launch(k_matfree_kuhn<DOT>);
   else
-    FEMK_BY_ND(p->nd, k_matfree<ND><<<::femk::counted_launch() + grid, 128, 0, s>>>(p->xyz, p->mcells, p->ntet, m.param, m.mode, m.scale, x, y, st));
+    FEMK_BY_ND(p->nd, launch(k_matfree<ND, DOT>));
   FEMK_CUDA_TRY(cudaGetLastError());
-  if (p->n_dir > 0) {
-    k_dirichlet_identity<<<::femk::counted_launch() + blocks_for(p->n_dir, 256, 65535), 256, 0, s>>>(p->dlist, p->n_dir, x, y, st);
-    FEMK_CUDA_TRY(cudaGetLastError());
-  }
   return FEMK_OK;
+}
+
+// y = A x
+int launch_matfree(const femk_plan* p, const MatFree& m, const double* x, double* y, cudaStream_t s) {
+  FEMK_TRY(ensure_mcells(p, s));
+  k_zero<<<::femk::counted_launch() + p->n_sm * 8, 256, 0, s>>>(y, p->n);
+  return launch_matfree_product<false>(p, m, x, y, nullptr, s);
 }
 
 // One chunk of CG iterations on stream ws: the step SpMV and the two vector kernels per iteration.
@@ -1120,12 +1198,76 @@ int enqueue_chunk(const femk_plan* p, const double* vals, double* x, const doubl
       launch_update(p, x, r, z, P0, q, dinv, p->partials, st, ws);
     if (pd) cudaEventRecord(pd->ev[it][2], ws);
     if (split)
-      launch_pupdate_x(p, x, P0, r, dinv, st, ws);
+      launch_pupdate_x(p, x, P0, r, dinv, nullptr, st, ws);
     else
       launch_pupdate(p, P0, z, st, ws);
     if (pd) cudaEventRecord(pd->ev[it][3], ws);
   }
   FEMK_CUDA_TRY(cudaGetLastError());
+  return FEMK_OK;
+}
+
+// A chunk of the matrix-free CG: the product with <p, q>, the r update, the x and p update (which zeroes q).
+int enqueue_matfree_chunk(const femk_plan* p, const MatFree& m, double* x, const double* dinv, int64_t iters,
+                          cudaStream_t ws) {
+  const int64_t vs = p->vstride;
+  double* r = p->work;
+  double* z = r + vs;
+  double* pv = z + vs;
+  double* q = pv + vs;
+  CgState* st = p->state;
+  const bool split = split_ok(p, x, dinv);
+  for (int64_t it = 0; it < iters; ++it) {
+    int shares = 0;
+    FEMK_TRY(launch_matfree_product<true>(p, m, pv, q, st, ws, &shares));
+    if (split) {
+      launch_update_r(p, r, q, dinv, st, ws, shares);
+      launch_pupdate_x(p, x, pv, r, dinv, q, st, ws);
+    } else {
+      k_sum_pq<<<::femk::counted_launch() + 1, kThreads, 0, ws>>>(p->partials + kPqShares, shares, st);
+      launch_update(p, x, r, z, pv, q, dinv, p->partials, st, ws);
+      launch_pupdate(p, pv, z, st, ws);
+      k_zero<<<::femk::counted_launch() + p->n_sm * 8, 256, 0, ws>>>(q, p->n);
+    }
+  }
+  FEMK_CUDA_TRY(cudaGetLastError());
+  return FEMK_OK;
+}
+
+// Captures what `enqueue` puts on the plan's stream into *exec (an update of the graph that is there, if it fits).
+template <typename F>
+int capture_chunk(femk_plan* p, cudaGraphExec_t* exec, F&& enqueue) {
+  cudaGraph_t g = nullptr;
+  set_capturing(true);
+  cudaError_t e = cudaStreamBeginCapture(p->cg_stream, cudaStreamCaptureModeThreadLocal);
+  int st = e == cudaSuccess ? enqueue() : FEMK_ECUDA;
+  const cudaError_t e2 = cudaStreamEndCapture(p->cg_stream, &g);
+  set_capturing(false);
+  if (e != cudaSuccess || e2 != cudaSuccess || st != FEMK_OK) {
+    if (g) cudaGraphDestroy(g);
+    set_error(std::string("femk_pcg: graph capture failed: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
+    return st != FEMK_OK ? st : FEMK_ECUDA;
+  }
+  bool updated = false;
+  if (*exec) {
+    cudaGraphExecUpdateResultInfo info;
+    updated = cudaGraphExecUpdate(*exec, g, &info) == cudaSuccess;
+    if (!updated) {
+      cudaGetLastError();
+      cudaGraphExecDestroy(*exec);
+      *exec = nullptr;
+    }
+  }
+  if (!updated) {
+    const cudaError_t e3 = cudaGraphInstantiate(exec, g, 0);
+    if (e3 != cudaSuccess) {
+      cudaGraphDestroy(g);
+      *exec = nullptr;
+      set_error(std::string("femk_pcg: graph instantiation failed: ") + cudaGetErrorString(e3));
+      return FEMK_ECUDA;
+    }
+  }
+  cudaGraphDestroy(g);
   return FEMK_OK;
 }
 
@@ -1171,39 +1313,27 @@ int ensure_chunk_graph(femk_plan* p, const double* vals, double* x, const double
   (void)wave_grid(k_pupdate_x<false>, kThreads, p);
   if (sell) (void)launch_sell_bulk(p, nullptr, nullptr, nullptr, nullptr, true);
   if (sell) (void)launch_sell_wide(p, nullptr, nullptr, nullptr, nullptr, true);
-  cudaGraph_t g = nullptr;
-  set_capturing(true);
-  cudaError_t e = cudaStreamBeginCapture(p->cg_stream, cudaStreamCaptureModeThreadLocal);
-  int st = e == cudaSuccess ? enqueue_chunk(p, vals, x, dinv, sell, kChunk, p->cg_stream) : FEMK_ECUDA;
-  const cudaError_t e2 = cudaStreamEndCapture(p->cg_stream, &g);
-  set_capturing(false);
-  if (e != cudaSuccess || e2 != cudaSuccess || st != FEMK_OK) {
-    if (g) cudaGraphDestroy(g);
-    set_error(std::string("femk_pcg: graph capture failed: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
-    return st != FEMK_OK ? st : FEMK_ECUDA;
-  }
-  bool updated = false;
-  if (p->cg_exec) {
-    cudaGraphExecUpdateResultInfo info;
-    updated = cudaGraphExecUpdate(p->cg_exec, g, &info) == cudaSuccess;
-    if (!updated) {
-      cudaGetLastError();
-      cudaGraphExecDestroy(p->cg_exec);
-      p->cg_exec = nullptr;
-    }
-  }
-  if (!updated) {
-    const cudaError_t e3 = cudaGraphInstantiate(&p->cg_exec, g, 0);
-    if (e3 != cudaSuccess) {
-      cudaGraphDestroy(g);
-      p->cg_exec = nullptr;
-      set_error(std::string("femk_pcg: graph instantiation failed: ") + cudaGetErrorString(e3));
-      return FEMK_ECUDA;
-    }
-  }
-  cudaGraphDestroy(g);
+  FEMK_TRY(capture_chunk(p, &p->cg_exec, [&] { return enqueue_chunk(p, vals, x, dinv, sell, kChunk, p->cg_stream); }));
   for (int i = 0; i < 5; ++i) p->cg_key[i] = key[i];
   p->cg_nodes = 3 * kChunk;
+  return FEMK_OK;
+}
+
+// The same for the matrix-free step (aligned caller vectors): keyed by the coefficient, x and D^-1.
+int ensure_matfree_graph(femk_plan* p, const MatFree& m, double* x, const double* dinv) {
+  const void* key[3] = {m.param, x, dinv};
+  bool same = p->mf_exec != nullptr && p->mf_mode == m.mode && p->mf_scale == m.scale;
+  for (int i = 0; i < 3; ++i) same = same && key[i] == p->mf_key[i];
+  if (same) return FEMK_OK;
+  (void)wave_grid(k_update_r<true, true>, kThreads, p);
+  (void)wave_grid(k_update_r<false, true>, kThreads, p);
+  (void)wave_grid(k_pupdate_x<true, true>, kThreads, p);
+  (void)wave_grid(k_pupdate_x<false, true>, kThreads, p);
+  FEMK_TRY(capture_chunk(p, &p->mf_exec,
+                         [&] { return enqueue_matfree_chunk(p, m, x, dinv, kChunk, p->cg_stream); }));
+  for (int i = 0; i < 3; ++i) p->mf_key[i] = key[i];
+  p->mf_mode = m.mode;
+  p->mf_scale = m.scale;
   return FEMK_OK;
 }
 
@@ -1227,7 +1357,7 @@ int pcg_run(const femk_plan* pc, const double* vals, const MatFree* mf, const do
   double* q = pv + vs;
   CgState* st = p->state;
   ProfData* pd = !mf ? (ProfData*)p->prof : nullptr;
-  const bool graph = !mf && p->cg_graph && !pd;
+  const bool graph = p->cg_graph && !pd && (!mf || split_ok(p, x, dinv));
   const bool sell = !mf && p->use_sell && p->sell_cols;
   // all solver work runs on the plan's stream, ordered after the caller's stream and before
   // whatever the caller enqueues next
@@ -1236,7 +1366,8 @@ int pcg_run(const femk_plan* pc, const double* vals, const MatFree* mf, const do
   FEMK_CUDA_TRY(cudaStreamWaitEvent(ws, p->cg_ev[2], 0));
   // the sliced-ELL values buffer must exist before a graph that reads it is captured
   if (sell) FEMK_TRY(prepare_sell(p, vals, ws));
-  if (graph) FEMK_TRY(ensure_chunk_graph(p, vals, x, dinv, sell));
+  if (mf) FEMK_TRY(ensure_mcells(p, ws));
+  if (graph) FEMK_TRY((mf ? ensure_matfree_graph(p, *mf, x, dinv) : ensure_chunk_graph(p, vals, x, dinv, sell)));
   CgState init{};
   init.maxiter = maxiter;
   init.precond = dinv ? 1 : 0;
@@ -1257,19 +1388,12 @@ int pcg_run(const femk_plan* pc, const double* vals, const MatFree* mf, const do
   bool have_prev = false;
   while (true) {
     if (graph) {
-      FEMK_CUDA_TRY(cudaGraphLaunch(p->cg_exec, ws));
-      count_launches(p->cg_nodes);
+      FEMK_CUDA_TRY(cudaGraphLaunch(mf ? p->mf_exec : p->cg_exec, ws));
+      count_launches(mf ? 3 * kChunk : p->cg_nodes);
       enq += kChunk;  // iterations past convergence or maxiter return at entry
     } else if (mf) {
       const int64_t todo = std::min<int64_t>(kChunk, (int64_t)maxiter - enq);
-      for (int64_t it = 0; it < todo; ++it) {
-        FEMK_TRY(launch_matfree(p, *mf, pv, q, ws, st));
-        k_dot_pq<<<::femk::counted_launch() + wave_grid(k_dot_pq, kThreads, p), kThreads, 0, ws>>>(n, pv, q,
-                                                                                                  p->partials, st);
-        launch_update(p, x, r, z, pv, q, dinv, p->partials, st, ws);
-        launch_pupdate(p, pv, z, st, ws);
-      }
-      FEMK_CUDA_TRY(cudaGetLastError());
+      FEMK_TRY(enqueue_matfree_chunk(p, *mf, x, dinv, todo, ws));
       enq += todo;
     } else {
       const int64_t todo = std::min<int64_t>(kChunk, (int64_t)maxiter - enq);

@@ -224,6 +224,11 @@ struct femk_plan {
   cudaGraphExec_t cg_exec = nullptr;
   const void* cg_key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int cg_nodes = 0;
+  // the same for the matrix-free steps
+  cudaGraphExec_t mf_exec = nullptr;
+  const void* mf_key[3] = {nullptr, nullptr, nullptr};
+  int mf_mode = 0;
+  double mf_scale = 0.0;
   // the same for the mixed-precision solver
   cudaStream_t mx_stream = nullptr;
   cudaEvent_t mx_ev[3] = {nullptr, nullptr, nullptr};

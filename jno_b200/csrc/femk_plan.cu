@@ -744,6 +744,7 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
   if (p->state_host) cudaFreeHost(p->state_host);
   if (p->persist_out) cudaFreeHost(p->persist_out);
   if (p->cg_exec) cudaGraphExecDestroy(p->cg_exec);
+  if (p->mf_exec) cudaGraphExecDestroy(p->mf_exec);
   for (cudaEvent_t e : p->cg_ev)
     if (e) cudaEventDestroy(e);
   if (p->cg_stream) cudaStreamDestroy(p->cg_stream);
