@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(kBulkW * 32) k_bicg_bulk(const int64_t* __rest
                                                           const double* __restrict__ vals, int64_t n, int64_t nslices,
                                                           const double* __restrict__ x, const double* __restrict__ b,
                                                           Vecs v, double* __restrict__ partials, BicgState* st,
-                                                          const int64_t* __restrict__ cptr) {
+                                                          const int64_t* __restrict__ cptr,
+                                                          const int32_t* __restrict__ runs) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
   using R = BulkRing<double, int16_t, WMAX, kBulkS>;
   if (kind_skips<KIND>(st)) return;
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(kBulkW * 32) k_bicg_bulk(const int64_t* __rest
   const bool ok = sell_bulk_rows<double, int16_t, WMAX, kBulkS>(
       bulk_smem + wib * R::kWarpBytes, sptr, cols, vals, n, nslices, (int64_t)blockIdx.x * kBulkW + wib,
       (int64_t)gridDim.x * kBulkW, GatherXL<double>{x, l2_evict_last()}, Epi<KIND>{b, v, acc}, &st->status,
-      FEMK_TIMEOUT, cptr);
+      FEMK_TIMEOUT, cptr, runs);
   if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
   finish<KIND, kBulkW * 32>(st, acc, partials);
 }
@@ -292,7 +293,7 @@ bool launch_bulk_kind(const femk_plan* p, const double* x, const double* b, cons
   const bool tab = p->sell_cu != nullptr;
   kern<<<counted_launch() + p->n_sm * std::min(per_sm, 16), kBulkW * 32, kSmem, s>>>(
       p->sell_ptr, tab ? p->sell_cu : p->sell_c16, p->sell_vals, p->n, p->n_slices, x, b, v, p->partials, st,
-      tab ? p->sell_cuptr : nullptr);
+      tab ? p->sell_cuptr : nullptr, tab ? p->sell_runs : nullptr);
   return true;
 }
 

@@ -96,13 +96,14 @@ __device__ __forceinline__ void bulk_g2s_plain(void* dst, const void* src, uint3
 }
 
 // Where the copies of one slice come from: values at vals + b0 (32 w entries), columns at cols + c0
-// (cn entries; cn < 32 w marks a shared-offset table).
+// (cn entries), in runs of rows that share their offsets (first: where the later runs start, a byte each)
+// or one an entry (first < 0).
 struct SliceDir {
   int64_t b0, c0;
-  int32_t w, cn;
+  int32_t w, cn, first, pad;
 };
 
-// Shared memory one warp needs: S mbarriers + S widths (128 B), a directory of the
+// Shared memory one warp needs: S mbarriers, widths and run starts (128 B), a directory of the
 // warp's next kDir slices, then S stages of [32*WMAX values][32*WMAX columns].
 template <typename V, typename IDX, int WMAX, int S>
 struct BulkRing {
@@ -135,18 +136,21 @@ __device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity) {
 // fit in 32 bits (the plan's column indices are int32), so the loop runs on 32-bit indices.
 //
 // cptr == NULL: cols holds one column (or offset) per stored entry, like vals. cptr != NULL: cols is
-// the per-slice column table (int16 offsets): slice s's table starts at cptr[s] and holds either w
-// offsets shared by all 32 rows (padded to 8) or the 32*w per-entry offsets.
+// the per-slice column table (int16 offsets): slice s's table starts at cptr[s] and holds the w offsets
+// of each of its runs of rows (padded to 8 a run; runs[s] as femk_order.cu leaves it) or the 32*w
+// per-entry offsets.
 template <typename V, typename IDX, int WMAX, int S, typename G, typename Epi>
 __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64_t* __restrict__ sptr,
                                                const IDX* __restrict__ cols, const V* __restrict__ vals, int64_t n,
                                                int64_t nslices64, int64_t g64, int64_t NW64, const G& gx, Epi&& epi,
-                                               int* err, int errval, const int64_t* __restrict__ cptr = nullptr) {
+                                               int* err, int errval, const int64_t* __restrict__ cptr = nullptr,
+                                               const int32_t* __restrict__ runs = nullptr) {
   using R = BulkRing<V, IDX, WMAX, S>;
   const int lane = threadIdx.x & 31;
   const int32_t nslices = (int32_t)nslices64, g = (int32_t)g64, NW = (int32_t)NW64;
   uint64_t* bar = reinterpret_cast<uint64_t*>(wsmem);
-  int32_t* wid = reinterpret_cast<int32_t*>(wsmem + 8 * S);  // slice width per stage; negative: shared offsets
+  int32_t* wid = reinterpret_cast<int32_t*>(wsmem + 8 * S);  // slice width per stage
+  int32_t* rst = wid + S;                                    // run starts per stage (-1: per-entry columns)
   SliceDir* dir = reinterpret_cast<SliceDir*>(wsmem + 128);
   unsigned char* stages = wsmem + R::kHead;
   uint64_t pol = 0;
@@ -166,12 +170,13 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
         const int64_t b0 = __ldg(sptr + sl);
         const int32_t w = (int32_t)((__ldg(sptr + sl + 1) - b0) >> 5);
         int64_t c0 = b0;
-        int32_t cn = 32 * w;
+        int32_t cn = 32 * w, first = -1;
         if (cptr) {
           c0 = __ldg(cptr + sl);
           cn = (int32_t)(__ldg(cptr + sl + 1) - c0);
+          first = __ldg(runs + sl);
         }
-        dir[lane] = SliceDir{b0, c0, w, cn};
+        dir[lane] = SliceDir{b0, c0, w, cn, first, 0};
       }
     }
     __syncwarp();
@@ -180,7 +185,8 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
   // lane 0: stream the slice of ordinal j (in the directory) into stage `s`
   auto issue = [&](int32_t j, int s) {
     const SliceDir d = dir[j - dbase];
-    wid[s] = d.cn == 32 * d.w ? d.w : -d.w;
+    wid[s] = d.w;
+    rst[s] = d.first;
     const uint32_t vb = (uint32_t)(32 * d.w * (int)sizeof(V));
     const uint32_t cb = (uint32_t)(d.cn * (int)sizeof(IDX));
     unsigned char* st = stages + s * R::kStage;
@@ -209,10 +215,11 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
       ok = false;
       break;
     }
-    const int32_t ws = wid[s];
-    const int32_t w = ws < 0 ? -ws : ws;
+    const int32_t w = wid[s], first = rst[s];
     const V* sv = reinterpret_cast<const V*>(stages + s * R::kStage) + lane;
     const IDX* sc = reinterpret_cast<const IDX*>(stages + s * R::kStage + R::kVal);
+    if (first >= 0)  // this lane's run
+      sc += ((w + 7) & ~7) * ((lane >= (first & 255)) + (lane >= ((first >> 8) & 255)) + (lane >= (first >> 16)));
     const int32_t row = sl * 32 + lane;
     const bool live = row < n;  // rows past n in the last slice gather nothing
     V acc = V(0);
@@ -225,8 +232,8 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
       const IDX* cb = U ? sc : sc + lane;
       V xg[K];
       if constexpr (U && sizeof(IDX) == 2 && sizeof(V) == 4) {
-        // FP32 rows, shared offsets: broadcast 16-byte loads of 8 offsets each (the table is padded
-        // to 8, and the stage's column area starts 128-byte aligned). Measured on one B200 at P1
+        // FP32 rows, shared offsets: 16-byte loads of 8 offsets each, one address a run (a run's table is
+        // padded to 8, and the stage's column area starts 128-byte aligned). Measured on one B200 at P1
         // 128^3: the mixed solve 25.87 -> 25.24 ms, while the same loads slowed the FP64 solve
         // 35.78 -> 38.51 ms, so FP64 rows keep the per-entry loads.
         constexpr int NQ = (K + 7) / 8;
@@ -253,14 +260,14 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
     };
     if (live) {
       using std::integral_constant;
-      const bool u = ws < 0;
+      const bool u = first >= 0;
       if (w == WMAX) {
         u ? run(integral_constant<int, WMAX>{}, std::true_type{}) : run(integral_constant<int, WMAX>{}, std::false_type{});
       } else if (w == WMAX - 1) {
         u ? run(integral_constant<int, WMAX - 1>{}, std::true_type{})
           : run(integral_constant<int, WMAX - 1>{}, std::false_type{});
       } else {
-        const int cstride = u ? 1 : 32;  // shared offsets: every lane reads entry k (a broadcast)
+        const int cstride = u ? 1 : 32;  // shared offsets: the lanes of a run read one entry k
         const int clane = u ? 0 : lane;
         V xg[WMAX];
 #pragma unroll

@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(WPB * 32) k_sell_bulk(const int64_t* __restric
                                                        const double* __restrict__ svals, int64_t n, int64_t nslices,
                                                        const double* __restrict__ x, double* __restrict__ y,
                                                        double* __restrict__ partials, CgState* st, int* err,
-                                                       const int64_t* __restrict__ cptr) {
+                                                       const int64_t* __restrict__ cptr,
+                                                       const int32_t* __restrict__ runs) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
   constexpr int kWarpBytes = BulkRing<double, IDX, WMAX, S>::kWarpBytes;
   if (MODE == kCgStep) {
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(WPB * 32) k_sell_bulk(const int64_t* __restric
         y[row] = sv;
         if (MODE == kCgStep) acc[0] += __ldg(x + row) * sv;
       },
-      errp, FEMK_TIMEOUT, cptr);
+      errp, FEMK_TIMEOUT, cptr, runs);
   if (MODE == kPlain) return;
   if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
   block_reduce_store<1, WPB * 32>(acc, partials);
@@ -295,12 +296,12 @@ __global__ void __launch_bounds__(WPB * 32, 8) k_sell_wide(const int64_t* __rest
 template <typename T>
 __global__ void k_sell_gather(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr, int64_t n,
                               int64_t nslices, const double* __restrict__ vals, int64_t nnz, int32_t cap,
-                              T* __restrict__ out, int* __restrict__ err) {
+                              T* __restrict__ out, int* __restrict__ err, const uint8_t* __restrict__ src) {
   extern __shared__ double sg_buf[];
   const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   sell_transpose_warp<T>(sg_buf + (int64_t)wib * cap, cap, sptr, indptr, n, nslices, vals, nnz, out,
                          (int64_t)blockIdx.x * wpb + wib, (int64_t)gridDim.x * wpb,
-                         [](double v, int64_t, int64_t) { return (T)v; }, err);
+                         [](double v, int64_t, int64_t) { return (T)v; }, err, src);
 }
 
 template <typename T>
@@ -989,10 +990,11 @@ bool launch_sell_bulk_cfg(const femk_plan* p, const double* x, double* y, CgStat
   if (per_sm <= 0) return false;
   if (prime) return true;
   const int grid = p->n_sm * std::min(per_sm, 16);
-  const bool tab = p->sell_cu != nullptr;  // per-slice column tables (shared-offset slices stored once)
+  const bool tab = p->sell_cu != nullptr;  // per-slice column tables
   kern<<<::femk::counted_launch() + grid, WPB * 32, kSmem, s>>>(
       (const int64_t*)p->sell_ptr, (const int16_t*)(tab ? p->sell_cu : p->sell_c16), (const double*)p->sell_vals,
-      p->n, p->n_slices, x, y, p->partials, st, (int*)nullptr, (const int64_t*)(tab ? p->sell_cuptr : nullptr));
+      p->n, p->n_slices, x, y, p->partials, st, (int*)nullptr, (const int64_t*)(tab ? p->sell_cuptr : nullptr),
+      (const int32_t*)(tab ? p->sell_runs : nullptr));
   return true;
 }
 
@@ -1507,10 +1509,12 @@ int launch_sell_values(const femk_plan* p, const double* vals, bool fp32, cudaSt
     return FEMK_OK;
   }
   k_sell_gather<double><<<::femk::counted_launch() + grid, 128, smem, s>>>(p->sell_ptr, p->indptr, p->n, p->n_slices,
-                                                                           vals, p->nnz, cap, p->sell_vals, p->dev_err);
+                                                                           vals, p->nnz, cap, p->sell_vals, p->dev_err,
+                                                                           p->sell_src);
   if (fp32)
     k_sell_gather<float><<<::femk::counted_launch() + grid, 128, smem, s>>>(p->sell_ptr, p->indptr, p->n, p->n_slices,
-                                                                            vals, p->nnz, cap, p->sell_vals32, p->dev_err);
+                                                                            vals, p->nnz, cap, p->sell_vals32, p->dev_err,
+                                                                            p->sell_src);
   FEMK_CUDA_TRY(cudaGetLastError());
   return FEMK_OK;
 }

@@ -172,23 +172,23 @@ struct femk_plan {
   // sliced-ELL solver layout (SELL-32), built with the pattern
   int64_t n_slices = 0, sell_nnz = 0;
   int64_t* sell_ptr = nullptr;   // i64[n_slices+1] first entry of each slice
-  int32_t* sell_cols = nullptr;  // i32[sell_nnz]
+  int32_t* sell_cols = nullptr;  // i32[sell_nnz] (with sell_c16 and sell_src in one allocation)
   int16_t* sell_c16 = nullptr;   // i16[sell_nnz] col - row, when the bandwidth fits
   double* sell_vals = nullptr;   // f64[sell_nnz] values gathered for the current solve
   float* sell_vals32 = nullptr;  // f32[sell_nnz] FP32 values for the mixed-precision inner solve
-  // per-slice column tables of the bulk-copy SpMV (int16 offsets): a slice whose rows share one
-  // offset sequence stores it once (padded to 8), any other slice its 32*w per-entry offsets
+  // column tables (femk_order.cu): a slice with up to 4 runs of rows of the same column offsets stores each run's
+  // once, any other slice its 32*w per-entry offsets. 16-bit offsets for the bulk-copy ring ...
   int sell_uni = 1;
+  void* sell_base = nullptr;      // the allocation of sell_ptr, the table starts, sell_runs, perm and pos
+  int32_t* sell_runs = nullptr;   // i32[n_slices] first rows of a slice's second to fourth run (a byte each), -1: per entry
   int64_t* sell_cuptr = nullptr;  // i64[n_slices+1] first table entry of each slice
   int16_t* sell_cu = nullptr;     // i16[sell_cu_len]
   int64_t sell_cu_len = 0;
-  // 32-bit column tables of the bulk-copy product of wide rows (sell_wide_rows), where int16 offsets do not fit
+  // ... 32-bit ones for the product of wide rows (sell_wide_rows), where 16 bits do not fit
   int64_t* sell_ctptr = nullptr;  // i64[n_slices+1] first word of each slice
   int32_t* sell_ct = nullptr;     // i32[sell_ct_len]
   int64_t sell_ct_len = 0;
-  int32_t* sell_runs = nullptr;   // i32[n_slices] first rows of a slice's second to fourth run (a byte each), -1: full
   // the solver's row order (femk_order.cu), NULL: the DOF order
-  void* perm_base = nullptr;    // the allocation that holds sell_ctptr, perm, pos and sell_runs
   int32_t* perm = nullptr;      // i32[n] DOF of each solver row
   int32_t* pos = nullptr;       // i32[n] solver row of each DOF
   uint8_t* sell_src = nullptr;  // u8[sell_nnz] place of each entry in its CSR row (255: padding)

@@ -153,7 +153,7 @@ template <typename IDX>
 __global__ void k_gather_scaled(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr,
                                 const IDX* __restrict__ cols, int64_t n, int64_t nslices, const double* __restrict__ vals,
                                 int64_t nnz, int32_t cap, const double* __restrict__ s64, float* __restrict__ out,
-                                int* __restrict__ err) {
+                                int* __restrict__ err, const uint8_t* __restrict__ src) {
   extern __shared__ double sg_buf[];
   const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   sell_transpose_warp<float>(
@@ -163,7 +163,7 @@ __global__ void k_gather_scaled(const int64_t* __restrict__ sptr, const int32_t*
         const int64_t col = sizeof(IDX) == 2 ? row + (int64_t)__ldcs(cols + j) : (int64_t)__ldcs(cols + j);
         return (float)(v * __ldg(s64 + row) * __ldg(s64 + col));
       },
-      err);
+      err, src);
 }
 
 // the same for a plan with a row order of its own
@@ -311,7 +311,8 @@ __global__ void __launch_bounds__(WPB * 32) k_step32_bulk(const int64_t* __restr
                                                          const float* __restrict__ vals, int64_t n, int64_t nslices,
                                                          const float* __restrict__ r, float* __restrict__ w,
                                                          double* __restrict__ partials, int ga, MixedState* st,
-                                                         const int64_t* __restrict__ cptr, int odd) {
+                                                         const int64_t* __restrict__ cptr,
+                                                         const int32_t* __restrict__ runs, int odd) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
   constexpr int kWarpBytes = BulkRing<float, int16_t, WMAX, S>::kWarpBytes;
   if (step_skip(st, REFRESH)) return;
@@ -319,7 +320,8 @@ __global__ void __launch_bounds__(WPB * 32) k_step32_bulk(const int64_t* __restr
   StepEpi epi{r, w, 0.f};
   const bool ok = sell_bulk_rows<float, int16_t, WMAX, S>(
       bulk_smem + wib * kWarpBytes, sptr, cols, vals, n, nslices, (int64_t)blockIdx.x * WPB + wib,
-      (int64_t)gridDim.x * WPB, checked(GatherX<float>{r}, n, &st->status), epi, &st->status, FEMK_TIMEOUT, cptr);
+      (int64_t)gridDim.x * WPB, checked(GatherX<float>{r}, n, &st->status), epi, &st->status, FEMK_TIMEOUT, cptr,
+      runs);
   if (!ok && (threadIdx.x & 31) == 0) st->done = 1;
   double v[1] = {(double)epi.a}, tot[1];
   if (!reduce_finish<1, WPB * 32>(v, partials, &st->ticket, tot)) return;
@@ -559,10 +561,11 @@ bool launch_step32_bulk_cfg(const femk_plan* p, const float* r, float* w, MixedS
   if (per_sm <= 0) return false;
   if (prime) return true;
   const int grid = p->n_sm * std::min(per_sm, 16);
-  const bool tab = p->sell_cu != nullptr;  // per-slice column tables (shared-offset slices stored once)
+  const bool tab = p->sell_cu != nullptr;  // per-slice column tables
   kern<<<::femk::counted_launch() + grid, WPB * 32, kSmem, s>>>(
       (const int64_t*)p->sell_ptr, (const int16_t*)(tab ? p->sell_cu : p->sell_c16), (const float*)p->sell_vals32,
-      p->n, p->n_slices, r, w, p->partials, update_grid(p), st, (const int64_t*)(tab ? p->sell_cuptr : nullptr), odd);
+      p->n, p->n_slices, r, w, p->partials, update_grid(p), st, (const int64_t*)(tab ? p->sell_cuptr : nullptr),
+      (const int32_t*)(tab ? p->sell_runs : nullptr), odd);
   return true;
 }
 
@@ -810,11 +813,13 @@ extern "C" int femk_pcg_mixed(const femk_plan* pc, const double* vals, const dou
     } else if (p->sell_c16) {
       FEMK_CUDA_TRY(cudaFuncSetAttribute(k_gather_scaled<int16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k_gather_scaled<int16_t><<<::femk::counted_launch() + gg, 128, smem, ws>>>(
-          p->sell_ptr, p->indptr, p->sell_c16, n, p->n_slices, vals, p->nnz, cap, s64, p->sell_vals32, p->dev_err);
+          p->sell_ptr, p->indptr, p->sell_c16, n, p->n_slices, vals, p->nnz, cap, s64, p->sell_vals32, p->dev_err,
+          p->sell_src);
     } else {
       FEMK_CUDA_TRY(cudaFuncSetAttribute(k_gather_scaled<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k_gather_scaled<int32_t><<<::femk::counted_launch() + gg, 128, smem, ws>>>(
-          p->sell_ptr, p->indptr, p->sell_cols, n, p->n_slices, vals, p->nnz, cap, s64, p->sell_vals32, p->dev_err);
+          p->sell_ptr, p->indptr, p->sell_cols, n, p->n_slices, vals, p->nnz, cap, s64, p->sell_vals32, p->dev_err,
+          p->sell_src);
     }
   } else {
     k_scale_csr<<<::femk::counted_launch() + g1, 256, 0, ws>>>(p->indptr, p->indices, n, vals, s64, p->vals32);

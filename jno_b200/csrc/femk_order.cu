@@ -10,9 +10,12 @@
 // exit; nothing outside them sees the order. B200, us a product: P2 64^3 in FP32 99.5 -> 50.5 (544 -> 250 MB), P2
 // 37x45x41 in FP64 39.8 -> 26.8 (215 -> 132 MB): 5.0 TB/s of the measured 6.5.
 //
-// Column tables. With int16 columns (femk_bulk.cuh reads those) a slice whose rows share one offset sequence
-// stores it once. In the solver's order a slice mostly has one or two such runs of rows (one mesh line, or the end of
-// one and the start of the next), whose 32-bit offsets it stores once each (sell_wide_rows reads these).
+// Column tables. A slice mostly has one or two runs of rows with the same column offsets (one mesh line, or the end of
+// one and the start of the next), which it stores once a run: 16-bit offsets where those fit (P1 lattices; the
+// 16-entry ring of femk_bulk.cuh reads them), 32-bit ones otherwise (P2 in the order above; sell_wide_rows). With one
+// offset sequence a slice at most, the 28 % of P1 128^3's slices that hold a line's end kept 2 bytes an entry:
+// 18 of the 309 MB of a product (53.9 -> 51.8 us a CG step), and nearly every slice did where lines are shorter than
+// two slices.
 #include <algorithm>
 #include <climits>
 
@@ -110,47 +113,52 @@ __global__ void k_order(const int2* __restrict__ ends, int64_t nedge, const int3
   }
 }
 
-// perm / pos of a P2 plan whose edges fall into few classes; leaves them NULL otherwise
-int build_order(femk_plan* p, cudaStream_t s) {
-  if (p->order != 2 || !p->use_sell) return FEMK_OK;
+struct Order {
+  Temp ends_base;
+  int2* ends = nullptr;
+  int32_t* cls = nullptr;
+  int classes = 0;  // 0: the DOF order
+};
+
+// the edge classes of a P2 plan, when there are few
+int find_order(const femk_plan* p, Order* o, cudaStream_t s) {
   const int64_t nedge = p->n - p->nvert;
-  if (nedge < 1) return FEMK_OK;
-  Temp first;  // edge ends, then the classes
-  FEMK_CUDA_TRY(cudaMalloc(&first.p, sizeof(int2) * nedge + sizeof(int32_t) * (kMaxClasses + 1)));
-  int2* ends = (int2*)first.p;
-  int32_t* cls = (int32_t*)(ends + nedge);
-  FEMK_CUDA_TRY(cudaMemsetAsync(cls, 0, sizeof(int32_t) * (kMaxClasses + 1), s));
+  if (p->order != 2 || !p->use_sell || nedge < 1) return FEMK_OK;
+  FEMK_CUDA_TRY(cudaMalloc(&o->ends_base.p, sizeof(int2) * nedge + sizeof(int32_t) * (kMaxClasses + 1)));
+  o->ends = (int2*)o->ends_base.p;
+  o->cls = (int32_t*)(o->ends + nedge);
+  FEMK_CUDA_TRY(cudaMemsetAsync(o->cls, 0, sizeof(int32_t) * (kMaxClasses + 1), s));
   if (p->nd == 10)
     k_edge_ends<10><<<counted_launch() + grid_for(p, p->ntet * 6), kThreads, 0, s>>>(p->cells, p->ntet, p->nvert,
-                                                                                  ends);
+                                                                                  o->ends);
   else
     k_edge_ends<6><<<counted_launch() + grid_for(p, p->ntet * 3), kThreads, 0, s>>>(p->cells, p->ntet, p->nvert,
-                                                                                 ends);
-  k_edge_classes<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(ends, nedge, cls);
+                                                                                 o->ends);
+  k_edge_classes<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(o->ends, nedge, o->cls);
   FEMK_CUDA_TRY(cudaGetLastError());
   int32_t h[kMaxClasses + 1];
-  FEMK_CUDA_TRY(cudaMemcpyAsync(h, cls, sizeof(h), cudaMemcpyDeviceToHost, s));
+  FEMK_CUDA_TRY(cudaMemcpyAsync(h, o->cls, sizeof(h), cudaMemcpyDeviceToHost, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   if (h[kMaxClasses]) return FEMK_OK;
-  int nc = 0;
-  while (nc < kMaxClasses && h[nc]) ++nc;
-  std::sort(h, h + nc);  // they were found in no fixed order
-  FEMK_CUDA_TRY(cudaMemcpyAsync(cls, h, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, s));
-  Temp second;  // a flag for every (class, lower end), then their exclusive scan
-  const int64_t m = nc * p->nvert;
-  FEMK_CUDA_TRY(cudaMalloc(&second.p, sizeof(int64_t) * 2 * (m + 1)));
-  int64_t* flag = (int64_t*)second.p;
+  while (o->classes < kMaxClasses && h[o->classes]) ++o->classes;
+  std::sort(h, h + o->classes);  // they were found in no fixed order
+  FEMK_CUDA_TRY(cudaMemcpyAsync(o->cls, h, sizeof(int32_t) * o->classes, cudaMemcpyHostToDevice, s));
+  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
+  return FEMK_OK;
+}
+
+int fill_order(femk_plan* p, const Order& o, cudaStream_t s) {
+  const int64_t nedge = p->n - p->nvert, m = o.classes * p->nvert;
+  Temp base;  // a flag for every (class, lower end), then their exclusive scan
+  FEMK_CUDA_TRY(cudaMalloc(&base.p, sizeof(int64_t) * 2 * (m + 1)));
+  int64_t* flag = (int64_t*)base.p;
   int64_t* rank = flag + m + 1;
   FEMK_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int64_t) * (m + 1), s));
-  k_class_flags<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(ends, nedge, cls, nc, p->nvert, flag);
+  k_class_flags<<<counted_launch() + grid_for(p, nedge), kThreads, 0, s>>>(o.ends, nedge, o.cls, o.classes, p->nvert,
+                                                                           flag);
   FEMK_TRY(scan_exclusive_i64(flag, rank, m, s));
-  // one allocation (an allocation takes 0.3 ms): table starts, the two orders, run starts
-  const int64_t ns = (p->n + 31) / 32;
-  FEMK_CUDA_TRY(cudaMalloc(&p->perm_base, sizeof(int64_t) * (ns + 1) + sizeof(int32_t) * (2 * p->n + ns)));
-  p->perm = (int32_t*)((int64_t*)p->perm_base + ns + 1);
-  p->pos = p->perm + p->n;
-  k_order<<<counted_launch() + grid_for(p, p->n), kThreads, 0, s>>>(ends, nedge, cls, nc, p->nvert, rank, p->perm,
-                                                                    p->pos);
+  k_order<<<counted_launch() + grid_for(p, p->n), kThreads, 0, s>>>(o.ends, nedge, o.cls, o.classes, p->nvert, rank,
+                                                                    p->perm, p->pos);
   FEMK_CUDA_TRY(cudaGetLastError());
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));  // temporaries are freed on return
   return FEMK_OK;
@@ -198,22 +206,25 @@ __global__ void k_sell_fill(const int32_t* __restrict__ indptr, const int32_t* _
   }
 }
 
-// The same in the solver's row order, with the column tables of sell_wide_rows. A warp takes a slice, a lane a row:
-// the row's columns as solver rows, sorted. Going down the slice, rows whose offsets (column - row) are all among
+// The same with column tables, in the solver's row order (perm, pos; NULL: the DOF order). A warp takes a slice, a lane
+// a row: the row's columns as solver rows, sorted. Going down the slice, rows whose offsets (column - row) are all among
 // those of a longer row, or hold all of them, form a run and share that longest row's offsets, an entry for each
 // (value 0 where a row has none): rows along a mesh line, its ends included. A slice with up to kRuns runs stores
-// one offset sequence a run, piece by piece of kPiece entries, each padded to 4 words; a slice with more stores
-// every entry's offset. No shared offset leads outside [0, n).
-// PASS 0: words[s], the table words of slice s. PASS 1: columns, places in the CSR row, tables and run starts.
+// one offset sequence a run (16-bit offsets: run by run, each padded to 8; 32-bit ones: piece by piece of kPiece
+// entries, each padded to 4); a slice with more stores every entry's offset. No shared offset leads outside [0, n).
+// PASS 0: words[s], the table entries of slice s. PASS 1: columns (and 16-bit offsets), places in the CSR row, tables
+// and run starts.
 constexpr int kRowMax = 255;  // place of an entry that a row does not have (rows hold fewer entries)
 constexpr int kRuns = 4;
 
-template <int PASS>
+template <int PASS, typename T>
 __global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                              const int32_t* __restrict__ perm, const int32_t* __restrict__ pos, int64_t n,
                              int64_t nslices, const int64_t* __restrict__ sptr, int32_t cap,
-                             int64_t* __restrict__ words, int32_t* __restrict__ cols, uint8_t* __restrict__ src,
-                             const int64_t* __restrict__ tptr, int32_t* __restrict__ tab, int32_t* __restrict__ runs) {
+                             int64_t* __restrict__ words, int32_t* __restrict__ cols, int16_t* __restrict__ c16,
+                             uint8_t* __restrict__ src, const int64_t* __restrict__ tptr, T* __restrict__ tab,
+                             int32_t* __restrict__ runs) {
+  constexpr int kPad = sizeof(T) == 2 ? 8 : 4;
   extern __shared__ long long order_buf[];  // 32 cap words a warp: (offset << 8) | place, entry k of lane l at 32 k + l
   const int lane = threadIdx.x & 31;
   long long* buf = order_buf + (int64_t)(threadIdx.x >> 5) * 32 * cap;
@@ -221,14 +232,15 @@ __global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* 
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t sl = warp; sl < nslices; sl += nwarps) {
     const int64_t b0 = sptr[sl];
-    const int32_t w = (int32_t)((sptr[sl + 1] - b0) >> 5), head = (w + 3) & ~3;
+    const int32_t w = (int32_t)((sptr[sl + 1] - b0) >> 5), head = (w + kPad - 1) & ~(kPad - 1);
     const int32_t row = (int32_t)(sl * 32) + lane;
     const bool live = row < n;
-    const int32_t dof = live ? perm[row] : 0;
+    const int32_t dof = live ? (perm ? perm[row] : row) : 0;
     const int32_t beg = live ? indptr[dof] : 0;
     const int32_t len = live ? indptr[dof + 1] - beg : 0;
     for (int32_t k = 0; k < len; ++k) {  // insertion sort by offset
-      const long long v = ((long long)(pos[indices[beg + k]] - row) << 8) | k;
+      const int32_t col = indices[beg + k];
+      const long long v = ((long long)((pos ? pos[col] : col) - row) << 8) | k;
       int32_t q = k;
       for (; q > 0 && buf[32 * (q - 1) + lane] > v; --q) buf[32 * q + lane] = buf[32 * (q - 1) + lane];
       buf[32 * q + lane] = v;
@@ -295,171 +307,116 @@ __global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* 
       continue;
     }
     // entries: a run's rows in the lead's slots, or in their own order
-    int32_t* t = tab ? tab + tptr[sl] : nullptr;
+    T* t = tab + tptr[sl];
     for (int32_t k = 0, q = 0; k < w; ++k) {
       const int64_t j = b0 + 32 * (int64_t)k + lane;
       const bool have = q < len && (nruns == 0 || off(lane, q) == off(lead, k));
       const int32_t o = have ? off(lane, q) : 0;
       cols[j] = live ? row + o : (int32_t)(n - 1);
+      if (c16) c16[j] = (int16_t)o;
       src[j] = have ? (uint8_t)(buf[32 * q + lane] & 255) : (uint8_t)kRowMax;
-      if (t && nruns == 0) t[32 * k + lane] = o;
+      if (nruns == 0) t[32 * k + lane] = (T)o;
       q += have;
     }
     int32_t nrep[kRuns];
 #pragma unroll
     for (int q = 0; q < kRuns; ++q) nrep[q] = __shfl_sync(0xffffffffu, len, rep[q]);
-    if (t && nruns > 0) {  // piece p of run q starts at word nruns * kPiece * p + q * (the piece's padded entries)
+    if (nruns > 0) {
       for (int32_t k = lane; k < head; k += 32) {
-        const int32_t k0 = k / kPiece * kPiece, pk = min(kPiece, head - k0);
+        // piece p of run q starts at nruns * kPiece * p + q * (the piece's padded entries)
+        const int32_t k0 = sizeof(T) == 2 ? 0 : k / kPiece * kPiece, pk = sizeof(T) == 2 ? head : min(kPiece, head - k0);
 #pragma unroll
         for (int q = 0; q < kRuns; ++q) {
           if (q >= nruns) continue;
-          t[nruns * k0 + q * pk + (k - k0)] = k < nrep[q] ? off(rep[q], k) : 0;
+          t[nruns * k0 + q * pk + (k - k0)] = (T)(k < nrep[q] ? off(rep[q], k) : 0);
         }
       }
     }
-    if (runs && lane == 0) runs[sl] = nruns > 0 ? start[1] | (start[2] << 8) | (start[3] << 16) : -1;
+    if (lane == 0) runs[sl] = nruns > 0 ? start[1] | (start[2] << 8) | (start[3] << 16) : -1;
     __syncwarp();
   }
 }
 
-// int16 column offsets of the slices; *bad is raised when one does not fit
-__global__ void k_sell_c16(const int64_t* __restrict__ sptr, const int32_t* __restrict__ cols, int64_t n,
-                           int64_t nslices, int16_t* __restrict__ c16, int* __restrict__ bad) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < nslices * 32;
-       row += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b0 = sptr[row >> 5] + (row & 31), w = (sptr[(row >> 5) + 1] - sptr[row >> 5]) >> 5;
-    const int64_t self = row < n ? row : n - 1;
-    for (int64_t k = 0; k < w; ++k) {
-      const int64_t d = cols[b0 + 32 * k] - self;
-      if (d < -32768 || d > 32767) *bad = 1;
-      c16[b0 + 32 * k] = (int16_t)d;
-    }
-  }
-}
-
-// Per-slice column table of the bulk-copy SpMV: a slice whose 32 rows share one column-offset
-// sequence (every row of an interior stretch of a structured mesh line) stores it once
-// (w offsets, padded to 8 = 16 bytes); any other slice keeps its 32*w per-entry offsets.
-// len[s] = entries of slice s's table; the table of slice s starts at cptr[s] (a multiple of 8).
-__global__ void k_sell_uni_len(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
-                               int64_t* __restrict__ len) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t b0 = sptr[sl];
-    const int64_t w = (sptr[sl + 1] - b0) / 32;
-    bool uni = true;
-    for (int64_t k = 0; k < w && uni; ++k) {
-      const int16_t c = c16[b0 + 32 * k + lane];
-      uni = __all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0));
-    }
-    if (lane == 0) len[sl] = uni ? (w + 7) / 8 * 8 : 32 * w;
-  }
-}
-
-__global__ void k_sell_uni_fill(const int64_t* __restrict__ sptr, const int16_t* __restrict__ c16, int64_t nslices,
-                                const int64_t* __restrict__ cptr, int16_t* __restrict__ cu) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t sl = warp; sl < nslices; sl += nwarps) {
-    const int64_t b0 = sptr[sl];
-    const int64_t w = (sptr[sl + 1] - b0) / 32;
-    const int64_t c0 = cptr[sl], len = cptr[sl + 1] - c0;
-    if (len == 32 * w) {
-      for (int64_t j = lane; j < len; j += 32) cu[c0 + j] = c16[b0 + j];
-    } else {
-      for (int64_t k = lane; k < len; k += 32) cu[c0 + k] = k < w ? c16[b0 + 32 * k] : (int16_t)0;
-    }
-  }
-}
-
-int build_uniform_columns(femk_plan* p, cudaStream_t s) {
-  if (!p->sell_uni) return FEMK_OK;
-  Temp len;
-  FEMK_CUDA_TRY(cudaMalloc(&len.p, sizeof(int64_t) * (p->n_slices + 1)));
-  FEMK_TRY(dev_alloc(&p->sell_cuptr, p->n_slices + 1));
-  const int sgrid = blocks_for(p->n_slices * 32, kThreads, p->n_sm * 64);
-  k_sell_uni_len<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
-                                                                       (int64_t*)len.p);
-  FEMK_TRY(scan_exclusive_i64((const int64_t*)len.p, p->sell_cuptr, p->n_slices, s));
-  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_cu_len, p->sell_cuptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                s));
+template <typename T>
+int fill_tables(femk_plan* p, int64_t* len, int64_t* tptr, T** tab, int64_t* total, cudaStream_t s) {
+  const int threads = 64, smem = threads * p->max_row * (int)sizeof(long long);
+  const int grid = blocks_for(p->n_slices * 32, threads, p->n_sm * 64);
+  FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<0, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<1, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_sell_order<0, T><<<counted_launch() + grid, threads, smem, s>>>(p->indptr, p->indices, p->perm, p->pos, p->n,
+                                                                    p->n_slices, p->sell_ptr, p->max_row, len, nullptr,
+                                                                    nullptr, nullptr, nullptr, nullptr, nullptr);
+  FEMK_TRY(scan_exclusive_i64(len, tptr, p->n_slices, s));
+  FEMK_CUDA_TRY(cudaMemcpyAsync(total, tptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  FEMK_TRY(dev_alloc(&p->sell_cu, p->sell_cu_len));
-  k_sell_uni_fill<<<::femk::counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_c16, p->n_slices,
-                                                                        p->sell_cuptr, p->sell_cu);
+  FEMK_TRY(dev_alloc(tab, *total));
+  k_sell_order<1, T><<<counted_launch() + grid, threads, smem, s>>>(
+      p->indptr, p->indices, p->perm, p->pos, p->n, p->n_slices, p->sell_ptr, p->max_row, nullptr, p->sell_cols,
+      p->sell_c16, p->sell_src, tptr, *tab, p->sell_runs);
   FEMK_CUDA_TRY(cudaGetLastError());
-  FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   return FEMK_OK;
 }
 
-int build_slices(femk_plan* p, cudaStream_t s) {
-  const int64_t n = p->n;
-  p->n_slices = (n + 31) / 32;
-  Temp slen;
-  FEMK_CUDA_TRY(cudaMalloc(&slen.p, sizeof(int64_t) * (p->n_slices + 1)));
-  FEMK_TRY(dev_alloc(&p->sell_ptr, p->n_slices + 1));
-  const int sgrid = grid_for(p, p->n_slices * 32);
-  k_sell_width<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->perm, n, p->n_slices, (int64_t*)slen.p);
-  FEMK_TRY(scan_exclusive_i64((const int64_t*)slen.p, p->sell_ptr, p->n_slices, s));
-  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_nnz, p->sell_ptr + p->n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+void drop_slices(femk_plan* p) {
+  for (void* q : {p->sell_base, (void*)p->sell_cols, (void*)p->sell_cu, (void*)p->sell_ct})
+    if (q) cudaFree(q);
+  p->sell_base = nullptr;
+  p->sell_ptr = p->sell_cuptr = p->sell_ctptr = nullptr;
+  p->perm = p->pos = p->sell_runs = p->sell_cols = p->sell_ct = nullptr;
+  p->sell_c16 = p->sell_cu = nullptr;
+  p->sell_src = nullptr;
+}
+
+int build_slices(femk_plan* p, const Order& o, cudaStream_t s) {
+  const int64_t n = p->n, ns = (n + 31) / 32;
+  p->n_slices = ns;
+  const bool ordered = o.classes > 0;
+  // few allocations (one takes 0.3 ms): what the slices' number sizes, what the stored entries' number does, the tables
+  FEMK_CUDA_TRY(cudaMalloc(&p->sell_base, sizeof(int64_t) * 3 * (ns + 1) + sizeof(int32_t) * (ns + (ordered ? 2 * n : 0))));
+  p->sell_ptr = (int64_t*)p->sell_base;
+  int64_t* tptr = p->sell_ptr + ns + 1;
+  int64_t* len = tptr + ns + 1;
+  p->sell_runs = (int32_t*)(len + ns + 1);
+  if (ordered) {
+    p->perm = p->sell_runs + ns;
+    p->pos = p->perm + n;
+    FEMK_TRY(fill_order(p, o, s));
+  }
+  const int sgrid = grid_for(p, ns * 32);
+  k_sell_width<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->perm, n, ns, len);
+  FEMK_TRY(scan_exclusive_i64(len, p->sell_ptr, ns, s));
+  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_nnz, p->sell_ptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   if (p->sell_nnz >= INT32_MAX) {
     p->use_sell = 0;
-    cudaFree(p->perm_base);
-    p->perm_base = nullptr;
-    p->perm = p->pos = nullptr;
+    drop_slices(p);
     return FEMK_OK;
   }
-  FEMK_TRY(dev_alloc(&p->sell_cols, p->sell_nnz));
-  if (!p->perm) {
-    if (p->cols16) FEMK_TRY(dev_alloc(&p->sell_c16, p->sell_nnz));
-    k_sell_fill<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->indices, n, p->n_slices, p->sell_ptr,
-                                                              p->sell_cols, p->sell_c16);
+  // 16-bit offsets always fit a system of at most 2^15 rows; past that only the DOF order's are known to
+  const bool c16 = ordered ? n <= 32768 : p->cols16 != nullptr;
+  const bool tables = ordered || (c16 && p->sell_uni);
+  char* base = nullptr;
+  FEMK_CUDA_TRY(cudaMalloc(&base, (p->sell_nnz > 0 ? p->sell_nnz : 1) * (4 + (c16 ? 2 : 0) + (tables ? 1 : 0))));
+  p->sell_cols = (int32_t*)base;
+  base += 4 * p->sell_nnz;  // slices hold 32 entries a column: every part starts on 32 bytes
+  if (c16) {
+    p->sell_c16 = (int16_t*)base;
+    base += 2 * p->sell_nnz;
+  }
+  if (tables) p->sell_src = (uint8_t*)base;
+  if (!tables) {
+    k_sell_fill<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->indptr, p->indices, n, ns, p->sell_ptr, p->sell_cols,
+                                                              p->sell_c16);
+  } else if (c16) {
+    FEMK_TRY(fill_tables(p, len, tptr, &p->sell_cu, &p->sell_cu_len, s));
+    p->sell_cuptr = tptr;
   } else {
-    FEMK_TRY(dev_alloc(&p->sell_src, p->sell_nnz));
-    const bool table = n > 65536 && p->sell_uni;
-    const int threads = 64, smem = threads * p->max_row * (int)sizeof(long long);
-    const int ogrid = blocks_for(p->n_slices * 32, threads, p->n_sm * 64);
-    if (table) {
-      FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      k_sell_order<0><<<counted_launch() + ogrid, threads, smem, s>>>(
-          p->indptr, p->indices, p->perm, p->pos, n, p->n_slices, p->sell_ptr, p->max_row, (int64_t*)slen.p, nullptr,
-          nullptr, nullptr, nullptr, nullptr);
-      p->sell_ctptr = (int64_t*)p->perm_base;
-      FEMK_TRY(scan_exclusive_i64((const int64_t*)slen.p, p->sell_ctptr, p->n_slices, s));
-      FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_ct_len, p->sell_ctptr + p->n_slices, sizeof(int64_t),
-                                    cudaMemcpyDeviceToHost, s));
-      FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-      FEMK_TRY(dev_alloc(&p->sell_ct, p->sell_ct_len));
-      p->sell_runs = p->pos + n;
-    }
-    FEMK_CUDA_TRY(cudaFuncSetAttribute(k_sell_order<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k_sell_order<1><<<counted_launch() + ogrid, threads, smem, s>>>(
-        p->indptr, p->indices, p->perm, p->pos, n, p->n_slices, p->sell_ptr, p->max_row, nullptr, p->sell_cols,
-        p->sell_src, p->sell_ctptr, p->sell_ct, p->sell_runs);
-    if (n <= 65536) {  // larger systems have offsets past 16 bits for certain: the last class is n / 8 rows away
-      Temp bad;
-      int h = 0;
-      FEMK_CUDA_TRY(cudaMalloc(&bad.p, sizeof(int)));
-      FEMK_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-      FEMK_TRY(dev_alloc(&p->sell_c16, p->sell_nnz));
-      k_sell_c16<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_cols, n, p->n_slices, p->sell_c16,
-                                                               (int*)bad.p);
-      FEMK_CUDA_TRY(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-      FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-      if (h) {
-        cudaFree(p->sell_c16);
-        p->sell_c16 = nullptr;
-      }
-    }
+    FEMK_TRY(fill_tables(p, len, tptr, &p->sell_ct, &p->sell_ct_len, s));
+    p->sell_ctptr = tptr;
   }
   FEMK_CUDA_TRY(cudaGetLastError());
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  return p->sell_c16 ? build_uniform_columns(p, s) : FEMK_OK;
+  return FEMK_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -485,36 +442,25 @@ __global__ void k_permute_out(const int32_t* __restrict__ perm, int64_t n, const
 }  // namespace
 
 int build_sell(femk_plan* p, cudaStream_t s) {
-  FEMK_TRY(build_order(p, s));
-  return build_slices(p, s);
+  Order o;
+  FEMK_TRY(find_order(p, &o, s));
+  return build_slices(p, o, s);
 }
 
 int natural_order(femk_plan* p, cudaStream_t s) {
   if (!p->perm) return FEMK_OK;
   FEMK_CUDA_TRY(cudaDeviceSynchronize());  // nothing may still read what is freed here
-  auto drop = [](auto*& q) {
-    if (q) cudaFree(q);
-    q = nullptr;
-  };
-  cudaFree(p->perm_base);
-  p->perm_base = nullptr;
-  p->perm = p->pos = p->sell_runs = nullptr;
-  p->sell_ctptr = nullptr;
-  drop(p->sell_src);
-  drop(p->sell_ptr);
-  drop(p->sell_cols);
-  drop(p->sell_c16);
-  drop(p->sell_cuptr);
-  drop(p->sell_cu);
-  drop(p->sell_ct);
-  drop(p->sell_vals);
-  drop(p->sell_vals32);
+  drop_slices(p);
+  cudaFree(p->sell_vals);
+  cudaFree(p->sell_vals32);
+  p->sell_vals = nullptr;
+  p->sell_vals32 = nullptr;
   for (cudaGraphExec_t* e : {&p->cg_exec, &p->mx_exec, &p->bicg_exec})
     if (*e) {
       cudaGraphExecDestroy(*e);
       *e = nullptr;
     }
-  return build_slices(p, s);
+  return build_slices(p, Order{}, s);
 }
 
 int permute_in(femk_plan* p, const double** b, double** x, const double** dinv, cudaStream_t s) {

@@ -10,7 +10,7 @@
 //   B  x += alpha p;  r -= alpha q;  z = D^-1 r;  <r, z>, <r, r>                                  -> beta, stop test
 // The product forms the new direction at every gather from the pair {z_j, p_j} (one 16-byte load), so the
 // direction needs no phase, and no barrier, of its own. What is left is bound by the two barriers an iteration
-// (4.3 of the 7.1 us at 32^3) and, from 64^3 on, by the gathers and the operator's share that L2 holds. 512
+// (4.3 of the 7.3 us at 32^3) and, from 64^3 on, by the gathers and the operator's share that L2 holds. 512
 // threads: 768 and 1024 spill at 80 and 64 registers (64^3: 12.0 us an iteration, against 12.9 and 14.3).
 // The recurrence q = A z + beta q would gather z alone and gained 5-15 %, but its true residual at tolerances of
 // 1e-13 and below was up to 2.5 times larger, so the product keeps the textbook form.
@@ -26,9 +26,9 @@ namespace {
 
 constexpr int kPT = 512;                    // threads of a block, one block per SM
 constexpr int kPersistSmem = 220 * 1024;    // dynamic shared memory of a block (227 KB less the static part)
-// ... with int32 columns (no banded order): the gathers of the pairs then need L1, which is what shared memory
-// leaves (us an iteration with 220 / 100 KB: P2 26^3 29.2 / 18.5, shuffled P1 40^3 14.0 / 9.6; with int16 columns
-// P1 64^3 11.9 / 12.3, 80^3 20.6 / 30.8)
+// ... with a 32-bit column an entry (no regular order): the gathers of the pairs then need L1, which is what shared
+// memory leaves (us an iteration with 220 / 100 KB: shuffled P1 40^3 14.0 / 9.6; with column tables P1 64^3 11.9 /
+// 12.3, P2 18^3 9.6 / 11.8, 34^3 21.3 / 27.1)
 constexpr int kPersistSmemWide = 100 * 1024;
 
 struct PersistOut {
@@ -41,8 +41,10 @@ struct PersistOut {
 
 struct PcgArgs {
   const int64_t* sptr;
-  const void* cols;
+  const void* cols;  // columns, or the column tables that start at tptr
   const double* svals;
+  const int64_t* tptr;
+  const int32_t* runs;
   int64_t n, nslices;
   const double* b;
   double* x;
@@ -66,7 +68,7 @@ __device__ __forceinline__ long long global_ns() {
   return t;
 }
 
-template <int SET, typename IDX>
+template <int SET, typename IDX, bool TAB>
 __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   extern __shared__ __align__(16) unsigned char ps_smem[];
   constexpr int W = kPT / 32;
@@ -74,13 +76,13 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t nsl = (int32_t)a.nslices;
   const int G = (int)gridDim.x, bid = (int)blockIdx.x;
-  BlockMatrix<IDX> m;
+  BlockMatrix<IDX, TAB> m;
   m.s0 = block_slice(a.sptr, nsl, bid, G);
   m.ns = block_slice(a.sptr, nsl, bid + 1, G) - m.s0;
   const int32_t r0 = m.s0 * 32, nr = m.ns * 32;
   // shared memory: slice offsets, the block's x, r, p, q, D^-1 (and the pairs, when one block owns all), slices
   int32_t* off = reinterpret_cast<int32_t*>(ps_smem);
-  const int32_t head = (4 * (m.ns + 1) + 15) & ~15;
+  const int32_t head = offset_bytes<TAB>(m.ns);
   const bool vin = ONE || head + 40 * nr <= a.smem;
   double* vec = reinterpret_cast<double*>(ps_smem + head);
   double* xs = vin ? vec : a.x + r0;
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   double2* zps = reinterpret_cast<double2*>(vec + 5 * nr);
   unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
-  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, off, mat, a.smem - (int32_t)(mat - ps_smem));
+  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
   BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
   // r = b - A x0, z = D^-1 r
   // gathers of x and of the pairs, range-checked in the bounds-checked build
@@ -100,7 +102,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   for (int32_t s = warp; s < m.ns; s += W) {
     const int32_t i = s * 32 + lane, row = r0 + i;
     if (row >= a.n) continue;
-    const double ax = block_row<16>(m, s, lane, row, xat);
+    const double ax = block_row(m, s, lane, row, xat);
     const double bi = __ldg(a.b + row);
     const double ri = bi - ax;
     const double di = a.dinv ? __ldg(a.dinv + row) : 1.0;
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
     for (int32_t s = warp; s < m.ns; s += W) {
       const int32_t i = s * 32 + lane, row = r0 + i;
       if (row >= a.n) continue;
-      const double qi = block_row<16>(m, s, lane, row, [&](int32_t j) {
+      const double qi = block_row(m, s, lane, row, [&](int32_t j) {
         if (!FEMK_IN_BOUNDS(j, a.n, a.err)) return 0.0;
         const double2 v = ONE ? zps[j] : a.zp[j];
         return fma(beta, v.y, v.x);
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
     for (int32_t s = warp; s < m.ns; s += W) {
       const int32_t row = r0 + s * 32 + lane;
       if (row >= a.n) continue;
-      const double wi = __ldg(a.b + row) - block_row<16>(m, s, lane, row, xat);
+      const double wi = __ldg(a.b + row) - block_row(m, s, lane, row, xat);
       w2[0] += wi * wi;
     }
     if (live) live = grid.template sum<1>(w2);
@@ -228,8 +230,10 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
 
 struct BicgArgs {
   const int64_t* sptr;
-  const void* cols;
+  const void* cols;  // columns, or the column tables that start at tptr
   const double* svals;
+  const int64_t* tptr;
+  const int32_t* runs;
   int64_t n, nslices;
   const double* b;
   double* x;
@@ -252,7 +256,7 @@ struct BicgArgs {
 // the x and r updates with <r, r> and <rhat, r>: four sums and one barrier. The chunked solver's five kernels took
 // 36.5 us an iteration at 2-D P2 131x118 (62,331 rows, vertices in no order), 19.4 us here, 10.5 of them in the five
 // waits; at P1 44x40x47 a Crank-Nicolson march of 12 steps went from 14.6 to 6.9 ms.
-template <int SET, typename IDX>
+template <int SET, typename IDX, bool TAB>
 __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   extern __shared__ __align__(16) unsigned char ps_smem[];
   constexpr int W = kPT / 32;
@@ -260,13 +264,13 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t nsl = (int32_t)a.nslices;
   const int G = (int)gridDim.x, bid = (int)blockIdx.x;
-  BlockMatrix<IDX> m;
+  BlockMatrix<IDX, TAB> m;
   m.s0 = block_slice(a.sptr, nsl, bid, G);
   m.ns = block_slice(a.sptr, nsl, bid + 1, G) - m.s0;
   const int32_t r0 = m.s0 * 32, nr = m.ns * 32;
   // shared memory: slice offsets, the block's x, r, rhat, p, q, s, t, D^-1 (and phat, shat of one block), slices
   int32_t* off = reinterpret_cast<int32_t*>(ps_smem);
-  const int32_t head = (4 * (m.ns + 1) + 15) & ~15;
+  const int32_t head = offset_bytes<TAB>(m.ns);
   const bool vin = ONE || head + 64 * nr <= a.smem;
   double* vec = reinterpret_cast<double*>(ps_smem + head);
   auto slot = [&](int k) { return vin ? vec + (k + 1) * nr : a.work + k * a.vstride + r0; };
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   double* shat = ONE ? vec + 9 * nr : a.shat;
   unsigned char* mat = reinterpret_cast<unsigned char*>(vec + (ONE ? 10 * nr : (vin ? 8 * nr : 0)));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
-  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, off, mat, a.smem - (int32_t)(mat - ps_smem));
+  hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
   BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
   auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
   // body(local row, row) for every row of the block that this thread owns
@@ -290,7 +294,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   double acc[2] = {0.0, 0.0};
   rows([&](int32_t s, int32_t i, int32_t row) {
     const double bi = __ldg(a.b + row);
-    const double ri = bi - block_row<16>(m, s, lane, row, xat);
+    const double ri = bi - block_row(m, s, lane, row, xat);
     rs[i] = ri;
     hs[i] = ri;
     ps[i] = ri;
@@ -318,7 +322,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
     if (!(live = grid.barrier())) break;
     double v1[1] = {0.0};
     rows([&](int32_t s, int32_t i, int32_t row) {
-      const double qi = block_row<16>(m, s, lane, row, [&](int32_t j) {
+      const double qi = block_row(m, s, lane, row, [&](int32_t j) {
         return FEMK_IN_BOUNDS(j, a.n, a.err) ? phat[j] : 0.0;
       });
       qs[i] = qi;
@@ -337,7 +341,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
     const bool early = v1[0] < atol2;
     double v2[2] = {0.0, 0.0};
     rows([&](int32_t s, int32_t i, int32_t row) {
-      const double ti = block_row<16>(m, s, lane, row, [&](int32_t j) {
+      const double ti = block_row(m, s, lane, row, [&](int32_t j) {
         return FEMK_IN_BOUNDS(j, a.n, a.err) ? shat[j] : 0.0;
       });
       ts[i] = ti;
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   if (live) live = grid.barrier();
   if (live) {
     rows([&](int32_t s, int32_t, int32_t row) {
-      const double wi = __ldg(a.b + row) - block_row<16>(m, s, lane, row, xat);
+      const double wi = __ldg(a.b + row) - block_row(m, s, lane, row, xat);
       w2[0] += wi * wi;
     });
     live = grid.template sum<1>(w2);
@@ -399,7 +403,11 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
 }
 
 // Bytes of the sliced-ELL operator: what every iteration reads.
-int64_t operator_bytes(const femk_plan* p) { return p->sell_nnz * (p->sell_c16 ? 10 : 12); }
+int64_t operator_bytes(const femk_plan* p) {
+  if (p->sell_cu) return 8 * p->sell_nnz + 2 * p->sell_cu_len;
+  if (p->sell_ct) return 8 * p->sell_nnz + 4 * p->sell_ct_len;
+  return p->sell_nnz * (p->sell_c16 ? 10 : 12);
+}
 
 // One launch of a persistent kernel: co-resident blocks (a cluster, or a cooperative grid).
 template <typename Args>
@@ -439,26 +447,28 @@ int prepare_kernel(void (*kern)(Args), int set, int device, std::atomic<uint64_t
   return FEMK_OK;
 }
 
-template <int SET, typename IDX>
+template <int SET, typename IDX, bool TAB>
 struct PcgKernel {
-  static constexpr auto fn = k_pcg_persist<SET, IDX>;
+  static constexpr auto fn = k_pcg_persist<SET, IDX, TAB>;
 };
-template <int SET, typename IDX>
+template <int SET, typename IDX, bool TAB>
 struct BicgKernel {
-  static constexpr auto fn = k_bicg_persist<SET, IDX>;
+  static constexpr auto fn = k_bicg_persist<SET, IDX, TAB>;
 };
 
-template <template <int, typename> class K, int SET, typename IDX, typename Args>
+template <template <int, typename, bool> class K, int SET, typename IDX, bool TAB, typename Args>
 int launch_kernel(const femk_plan* p, const Args& a, int grid, cudaStream_t s) {
   static std::atomic<uint64_t> ready{0};
-  FEMK_TRY(prepare_kernel(K<SET, IDX>::fn, SET, p->device, ready));
-  return launch_set(p, K<SET, IDX>::fn, SET, grid, a, s);
+  FEMK_TRY(prepare_kernel(K<SET, IDX, TAB>::fn, SET, p->device, ready));
+  return launch_set(p, K<SET, IDX, TAB>::fn, SET, grid, a, s);
 }
 
-template <template <int, typename> class K, int SET, typename Args>
+template <template <int, typename, bool> class K, int SET, typename Args>
 int launch_columns(const femk_plan* p, const Args& a, int grid, cudaStream_t s) {
-  if (p->sell_c16) return launch_kernel<K, SET, int16_t>(p, a, grid, s);
-  return launch_kernel<K, SET, int32_t>(p, a, grid, s);
+  if (p->sell_cu) return launch_kernel<K, SET, int16_t, true>(p, a, grid, s);
+  if (p->sell_ct) return launch_kernel<K, SET, int32_t, true>(p, a, grid, s);
+  if (p->sell_c16) return launch_kernel<K, SET, int16_t, false>(p, a, grid, s);
+  return launch_kernel<K, SET, int32_t, false>(p, a, grid, s);
 }
 
 // The launch of kernel K for the plan. One block, with no wait for others, when all of it fits one SM
@@ -467,10 +477,14 @@ int launch_columns(const femk_plan* p, const Args& a, int grid, cudaStream_t s) 
 // grid: 2-D P1 100^2, 319 slices, 4.1 / 5.7; P1 20x22x24, 378 slices, 5.8 / 7.0; 2-D P2 60^2, 458 slices, 6.3 /
 // 6.9; 2-D P2 70^2, 622 slices, 7.0 / 6.7; P1 28^3, 763 slices, 8.4 / 7.2). Then a grid of 16 slices a block, a
 // slice a warp, at most a block an SM (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148).
-template <template <int, typename> class K, typename Args>
+template <template <int, typename, bool> class K, typename Args>
 int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
   a.sptr = p->sell_ptr;
-  a.cols = p->sell_c16 ? (const void*)p->sell_c16 : (const void*)p->sell_cols;
+  a.cols = p->sell_cu   ? (const void*)p->sell_cu
+           : p->sell_ct ? (const void*)p->sell_ct
+                        : (p->sell_c16 ? (const void*)p->sell_c16 : (const void*)p->sell_cols);
+  a.tptr = p->sell_cu ? p->sell_cuptr : p->sell_ctptr;
+  a.runs = p->sell_runs;
   a.svals = p->sell_vals;
   a.n = p->n;
   a.nslices = p->n_slices;
@@ -479,9 +493,9 @@ int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
   a.turn = p->persist_turn;
   a.skip = p->skip_arrival;
   a.limit = p->barrier_spin;
-  a.smem = p->sell_c16 ? kPersistSmem : kPersistSmemWide;
+  a.smem = p->sell_c16 || p->sell_ct ? kPersistSmem : kPersistSmemWide;
   a.err = p->dev_err;
-  const int64_t one = 4 * (p->n_slices + 1) + 16 + p->n_slices * 32 * one_row + operator_bytes(p);
+  const int64_t one = 4 * (3 * p->n_slices + 2) + 16 + p->n_slices * 32 * one_row + operator_bytes(p);
   if (one <= a.smem) return launch_columns<K, kOneBlock>(p, a, 1, s);
   if (p->n_slices <= 32 * kMaxCluster) {
     int grid = 2;
@@ -511,12 +525,14 @@ int ensure_persist(femk_plan* p) {
 
 }  // namespace
 
-// Up to 80 MB of operator the single launch wins, above it the chunked solver does: past that the operator, the
+// Up to 85 MB of operator the single launch wins, above it the chunked solver does: past that the operator, the
 // vectors and the pairs no longer stay in L2 together. B200, FP64 PCG to 1e-8, us an iteration, chunked ->
-// single launch: P1 32^3 (5.3 MB) 17.8 -> 7.1, 64^3 (41 MB) 21.3 -> 12.0, 80^3 (79 MB) 28.3 -> 18.5, 84^3 (91 MB)
-// 31.6 -> 31.5, 88^3 (105 MB) 33.6 -> 47.6; P2 26^3 (57 MB) 27.0 -> 18.5, 32^3 (104 MB) 36.8 -> 40.1.
+// single launch (MB of operator): P1 32^3 (4.2) 17.4 -> 7.3, 64^3 (32) 21.4 -> 12.0, 80^3 (63) 29.8 -> 18.3, 84^3 (73)
+// 31.4 -> 20.1, 88^3 (84) 33.1 -> 29.7, 92^3 (96) 36.1 -> 47.6; P2 18^3 (13) 20.1 -> 9.6, 26^3 (38) 22.0 -> 13.6, 34^3
+// (79) 31.7 -> 21.3; vertices in no order (12 B an entry), P1 40^3 (12) 26.5 -> 9.5.
+constexpr int64_t kPersistBytes = 85000000;
 bool pcg_persist_fits(const femk_plan* p) {
-  return p->persist_ok && p->coop && p->use_sell && p->sell_cols && operator_bytes(p) <= 80000000;
+  return p->persist_ok && p->coop && p->use_sell && p->sell_cols && operator_bytes(p) <= kPersistBytes;
 }
 
 int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double* x, const double* dinv, double tol,
@@ -571,7 +587,7 @@ int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double
 }
 
 bool bicg_persist_fits(const femk_plan* p) {
-  return p->persist_ok && p->coop && operator_bytes(p) <= 80000000;
+  return p->persist_ok && p->coop && operator_bytes(p) <= kPersistBytes;
 }
 
 int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, double* ws, double tol, double atol,

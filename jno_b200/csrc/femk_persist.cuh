@@ -160,16 +160,26 @@ struct BlockSum {
   }
 };
 
-// One block's share of the operator: slices [s0, s1), of which the first `fit` are in shared memory.
-template <typename IDX>
+// One block's share of the operator: slices [s0, s0 + ns), of which the first `fit` are in shared memory. IDX: the
+// type of the columns, an offset from the row (16 bits) or absolute (32); TAB: column tables (femk_order.cu), whose
+// entries are offsets of either type, in place of a column an entry.
+template <typename IDX, bool TAB>
 struct BlockMatrix {
   int32_t s0, ns, fit;   // first slice, slices, slices held in shared memory
   const int32_t* off;    // shared: ns + 1 entry offsets from the block's first entry
-  const double* sv;      // shared values and columns of the first `fit` slices
+  const int32_t* toff;   // shared, TAB: ns + 1 table offsets from the block's first table entry
+  const int32_t* runs;   // shared, TAB: run starts of each slice
+  const double* sv;      // shared values and columns (tables) of the first `fit` slices
   const IDX* sc;
-  const double* gv;      // the block's entries in global memory
+  const double* gv;      // the block's entries (tables) in global memory
   const IDX* gc;
 };
+
+// 32-bit words of shared memory for the offsets of ns slices
+template <bool TAB>
+__device__ __forceinline__ int32_t offset_bytes(int32_t ns) {
+  return (4 * (ns + 1 + (TAB ? 2 * ns + 1 : 0)) + 15) & ~15;
+}
 
 // First slice of block b: the blocks get equal shares of the work, counted as the stored entries plus 8 a row
 // for the vector updates (rows may be of unequal length). Every thread gets the same answer.
@@ -210,40 +220,127 @@ __device__ __forceinline__ double lane_row(const double* vb, const IDX* cb, int3
   return acc;
 }
 
-// The block's share, its first slices copied into `mat` (room bytes of shared memory; off: ns + 1 words of shared
+// The same with the offsets of the row's run: run `run` of `nruns`, kPieceRow entries at a time (16-byte loads of
+// the table, one address a run).
+constexpr int kPieceRow = 16;
+template <bool SHARED, typename T, typename G>
+__device__ __forceinline__ double table_row(const double* vb, const T* tab, int32_t w, int run, int nruns, int32_t row,
+                                            const G& g) {
+  constexpr int kPad = sizeof(T) == 2 ? 8 : 4, kVec = 16 / (int)sizeof(T);
+  const int32_t head = (w + kPad - 1) & ~(kPad - 1);
+  double acc = 0.0;
+  for (int32_t k0 = 0; k0 < w; k0 += kPieceRow) {
+    const T* t = sizeof(T) == 2 ? tab + run * head + k0 : tab + nruns * k0 + run * min(kPieceRow, head - k0);
+    double v[kPieceRow];
+    int4 q[kPieceRow / kVec];
+#pragma unroll
+    for (int u = 0; u < kPieceRow / kVec; ++u) {
+      q[u] = make_int4(0, 0, 0, 0);
+      if (k0 + u * kVec < w)
+        q[u] = SHARED ? reinterpret_cast<const int4*>(t)[u] : __ldg(reinterpret_cast<const int4*>(t) + u);
+    }
+#pragma unroll
+    for (int u = 0; u < kPieceRow; ++u) {
+      const int32_t j = (k0 + u) * 32;
+      v[u] = k0 + u < w ? (SHARED ? vb[j] : __ldg(vb + j)) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kPieceRow; ++u)
+      if (k0 + u < w) {
+        const int4 f = q[u / kVec];
+        int32_t c;
+        if (sizeof(T) == 2) {
+          const int h = u % 8 / 2;
+          const int32_t word = h == 0 ? f.x : (h == 1 ? f.y : (h == 2 ? f.z : f.w));
+          c = (u & 1) ? word >> 16 : (int32_t)(int16_t)(word & 0xffff);
+        } else {
+          const int h = u % 4;
+          c = h == 0 ? f.x : (h == 1 ? f.y : (h == 2 ? f.z : f.w));
+        }
+        acc += v[u] * g(row + c);
+      }
+  }
+  return acc;
+}
+
+// An entry's own offset (slices of a table plan with too many runs)
+template <bool SHARED, typename T, typename G>
+__device__ __forceinline__ double offset_row(const double* vb, const T* cb, int32_t w, int32_t row, const G& g) {
+  double acc = 0.0;
+  for (int32_t k0 = 0; k0 < w; k0 += 8) {
+    double v[8];
+    int32_t c[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int32_t j = (k0 + u) * 32;
+      c[u] = k0 + u < w ? (int32_t)(SHARED ? cb[j] : __ldg(cb + j)) : 0;
+      v[u] = k0 + u < w ? (SHARED ? vb[j] : __ldg(vb + j)) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k0 + u < w) acc += v[u] * g(row + c[u]);
+  }
+  return acc;
+}
+
+// The block's share, its first slices copied into `mat` (room bytes of shared memory; off: offset_bytes of shared
 // memory). The whole block calls this.
-template <int THREADS, typename IDX>
-__device__ __forceinline__ void hold_slices(BlockMatrix<IDX>& m, const int64_t* __restrict__ sptr, const void* cols,
-                                            const double* svals, int32_t* off, unsigned char* mat, int32_t room) {
+template <int THREADS, typename IDX, bool TAB>
+__device__ __forceinline__ void hold_slices(BlockMatrix<IDX, TAB>& m, const int64_t* __restrict__ sptr, const void* cols,
+                                            const double* svals, const int64_t* __restrict__ tptr,
+                                            const int32_t* __restrict__ runs, int32_t* off, unsigned char* mat,
+                                            int32_t room) {
   __shared__ int32_t fit_s;
-  const int64_t e0 = __ldg(sptr + m.s0);
-  for (int32_t s = threadIdx.x; s <= m.ns; s += THREADS) off[s] = (int32_t)(__ldg(sptr + m.s0 + s) - e0);
+  const int64_t e0 = __ldg(sptr + m.s0), t0 = TAB ? __ldg(tptr + m.s0) : e0;
+  int32_t* toff = off + m.ns + 1;
+  int32_t* rs = toff + m.ns + 1;
+  for (int32_t s = threadIdx.x; s <= m.ns; s += THREADS) {
+    off[s] = (int32_t)(__ldg(sptr + m.s0 + s) - e0);
+    if (TAB) {
+      toff[s] = (int32_t)(__ldg(tptr + m.s0 + s) - t0);
+      if (s < m.ns) rs[s] = __ldg(runs + m.s0 + s);
+    }
+  }
   if (threadIdx.x == 0) fit_s = 0;
   __syncthreads();
   for (int32_t s = threadIdx.x; s < m.ns; s += THREADS)
-    if ((int64_t)off[s + 1] * (8 + (int)sizeof(IDX)) <= room) atomicMax(&fit_s, s + 1);
+    if (8 * (int64_t)off[s + 1] + (int64_t)sizeof(IDX) * (TAB ? toff[s + 1] : off[s + 1]) <= room)
+      atomicMax(&fit_s, s + 1);
   __syncthreads();
   m.fit = fit_s;
   m.off = off;
+  m.toff = toff;
+  m.runs = rs;
   m.gv = svals + e0;
-  m.gc = reinterpret_cast<const IDX*>(cols) + e0;
-  const int32_t held = off[m.fit];
+  m.gc = reinterpret_cast<const IDX*>(cols) + t0;
+  const int32_t held = off[m.fit], theld = TAB ? toff[m.fit] : held;
   double* sv = reinterpret_cast<double*>(mat);
   IDX* sc = reinterpret_cast<IDX*>(sv + held);
-  for (int32_t k = threadIdx.x; k < held; k += THREADS) {
-    sv[k] = __ldg(m.gv + k);
-    sc[k] = __ldg(m.gc + k);
-  }
+  for (int32_t k = threadIdx.x; k < held; k += THREADS) sv[k] = __ldg(m.gv + k);
+  for (int32_t k = threadIdx.x; k < theld; k += THREADS) sc[k] = __ldg(m.gc + k);
   m.sv = sv;
   m.sc = sc;
   __syncthreads();
 }
 
-template <int B, typename IDX, typename G>
-__device__ __forceinline__ double block_row(const BlockMatrix<IDX>& m, int32_t s, int lane, int32_t row, const G& g) {
+template <typename IDX, bool TAB, typename G>
+__device__ __forceinline__ double block_row(const BlockMatrix<IDX, TAB>& m, int32_t s, int lane, int32_t row,
+                                            const G& g) {
   const int32_t o = m.off[s], w = (m.off[s + 1] - o) >> 5;
-  if (s < m.fit) return lane_row<B, true>(m.sv + o + lane, m.sc + o + lane, w, row, g);
-  return lane_row<B, false>(m.gv + o + lane, m.gc + o + lane, w, row, g);
+  if constexpr (!TAB) {
+    if (s < m.fit) return lane_row<16, true>(m.sv + o + lane, m.sc + o + lane, w, row, g);
+    return lane_row<16, false>(m.gv + o + lane, m.gc + o + lane, w, row, g);
+  } else {
+    const int32_t t = m.toff[s], first = m.runs[s];
+    if (first >= 0) {
+      const int s1 = first & 255, s2 = (first >> 8) & 255, s3 = first >> 16;
+      const int run = (lane >= s1) + (lane >= s2) + (lane >= s3), nruns = 1 + (s1 < 32) + (s2 < 32) + (s3 < 32);
+      if (s < m.fit) return table_row<true>(m.sv + o + lane, m.sc + t, w, run, nruns, row, g);
+      return table_row<false>(m.gv + o + lane, m.gc + t, w, run, nruns, row, g);
+    }
+    if (s < m.fit) return offset_row<true>(m.sv + o + lane, m.sc + t + lane, w, row, g);
+    return offset_row<false>(m.gv + o + lane, m.gc + t + lane, w, row, g);
+  }
 }
 
 }  // namespace femk

@@ -29,13 +29,15 @@ __device__ __forceinline__ int64_t col_at(const int16_t* __restrict__ cols, int3
 // Sliced-ELL copy of CSR values, one warp per 32-row slice (global warp g takes slices g, g + NW,
 // ...): rows 32s ... 32s+31 are one contiguous CSR range, read coalesced into the warp's shared
 // buffer wbuf (room for 32 rows of the plan's longest row), then entry k of row 32s + l is written
-// to out[sptr[s] + 32 k + l] as f(value, row, out index), and padding past the row's length as 0.
+// to out[sptr[s] + 32 k + l] as f(value, row, out index), and padding past the row's length as 0. src (may be NULL):
+// the place of each entry in its CSR row, 255 for padding (femk_order.cu).
 // Both the reads and the writes are coalesced; only the shared-memory reads are strided.
 template <typename T, typename F>
 __device__ __forceinline__ void sell_transpose_warp(double* wbuf, int32_t cap, const int64_t* __restrict__ sptr,
                                                     const int32_t* __restrict__ indptr, int64_t n, int64_t nslices,
                                                     const double* __restrict__ vals, int64_t nnz, T* __restrict__ out,
-                                                    int64_t g, int64_t NW, F f, int* err) {
+                                                    int64_t g, int64_t NW, F f, int* err,
+                                                    const uint8_t* __restrict__ src) {
   const int lane = threadIdx.x & 31;
   for (int64_t sl = g; sl < nslices; sl += NW) {
     const int64_t r0 = sl * 32, row = r0 + lane;
@@ -49,16 +51,23 @@ __device__ __forceinline__ void sell_transpose_warp(double* wbuf, int32_t cap, c
     const int32_t len = row < n ? __ldg(indptr + row + 1) - base - beg : 0;
     const int64_t b0 = sptr[sl] + lane;
     const int32_t w = (int32_t)((sptr[sl + 1] - sptr[sl]) >> 5);
-    for (int32_t k = 0; k < w; ++k) {
-      const int64_t j = b0 + 32 * k;
-      out[j] = (k < len && FEMK_IN_BOUNDS(beg + k, cap, err)) ? f(wbuf[beg + k], row, j) : T(0);
+    if (src) {
+      for (int32_t k = 0; k < w; ++k) {
+        const int64_t j = b0 + 32 * k;
+        const int32_t q = row < n ? (int32_t)__ldg(src + j) : 255;
+        out[j] = (q != 255 && FEMK_IN_BOUNDS(beg + q, cap, err)) ? f(wbuf[beg + q], row, j) : T(0);
+      }
+    } else {
+      for (int32_t k = 0; k < w; ++k) {
+        const int64_t j = b0 + 32 * k;
+        out[j] = (k < len && FEMK_IN_BOUNDS(beg + k, cap, err)) ? f(wbuf[beg + k], row, j) : T(0);
+      }
     }
     __syncwarp();  // the buffer is refilled for the next slice
   }
 }
 
-// The same for a plan with a row order of its own (femk_order.cu): lane l of a slice reads the CSR row of its DOF,
-// entry k from place src of it (255: padding).
+// The same for a plan with a row order of its own (femk_order.cu): lane l of a slice reads the CSR row of its DOF.
 template <typename T, typename F>
 __device__ __forceinline__ void sell_order_warp(const int64_t* __restrict__ sptr, const int32_t* __restrict__ indptr,
                                                 const int32_t* __restrict__ perm, const uint8_t* __restrict__ src,
