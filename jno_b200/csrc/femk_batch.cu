@@ -978,6 +978,9 @@ int batched_impl(const femk_plan* pc, int32_t nprob, const int64_t* row_off, con
   FEMK_TRY(natural_order(p, (cudaStream_t)stream));  // a problem owns a run of DOFs
   FEMK_CHECK_ARG(row_off[0] == 0 && row_off[nprob] == p->n, "femk_pcg_batched: row_off must span [0, n)");
   for (int32_t k = 0; k < nprob; ++k) FEMK_CHECK_ARG(row_off[k + 1] > row_off[k], "femk_pcg_batched: empty problem");
+  if (!mixed && batch_sets_fit(p, nprob, row_off))
+    return batch_sets(p, nprob, row_off, vals, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, status_out,
+                      (cudaStream_t)stream);
   const void* kern = mixed ? (const void*)k_batch_mixed : (const void*)k_batch_pcg;
   // The mixed form's FP32 products stream each slice through a two-stage shared-memory ring a warp
   // (int16 columns, rows of at most 16 entries: 96 KB a block, so 2 blocks of 512 fit an SM)

@@ -240,6 +240,10 @@ struct femk_plan {
   void* batch_ws = nullptr;
   int64_t batch_bytes = 0;
   const void* batch_key[8] = {};
+  void* batch_queue = nullptr;  // the batched solver on sets of blocks: results, problems, queues, barriers
+  int64_t batch_queue_bytes = 0;
+  cudaStream_t batch_side[5] = {};  // ... whose launches run beside one another
+  int batch_fit[5] = {};  // clusters of 2^i blocks that the device holds at once (0: not asked yet)
   cudaGraphExec_t batch_exec = nullptr;
   cudaStream_t batch_stream = nullptr;
   cudaEvent_t batch_ev = nullptr;
@@ -324,9 +328,16 @@ struct ProfData {
 };
 
 // Jacobi-PCG as one persistent launch (femk_persist.cu), for plans whose operator stays on the chip.
+constexpr int64_t kPersistBytes = 85000000;  // operator that L2 and shared memory keep (femk_persist.cu)
+int64_t operator_bytes(const femk_plan* p);
 bool pcg_persist_fits(const femk_plan* p);
 int pcg_persist(const femk_plan* p, const double* vals, const double* b, double* x, const double* dinv, double tol,
                 double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s);
+// Batched PCG, a problem to a set of blocks of its own (femk_batch_sets.cu).
+bool batch_sets_fit(const femk_plan* p, int32_t nprob, const int64_t* row_off);
+int batch_sets(femk_plan* p, int32_t nprob, const int64_t* row_off, const double* vals, const double* b, double* x,
+               const double* dinv, double tol, double atol, int32_t maxiter, int32_t* iters_out, double* relres_out,
+               int32_t* status_out, cudaStream_t s);
 
 // BiCGStab as one persistent launch on the plan's prepared operator; ws: 8 vectors of vstride doubles; *out: pinned.
 struct BicgResult {

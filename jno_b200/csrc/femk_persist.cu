@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
   hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
-  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
+  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u, bid, G};
   // r = b - A x0, z = D^-1 r
   // gathers of x and of the pairs, range-checked in the bounds-checked build
   auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   unsigned char* mat = reinterpret_cast<unsigned char*>(vec + (ONE ? 10 * nr : (vin ? 8 * nr : 0)));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
   hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
-  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u};
+  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u, bid, G};
   auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
   // body(local row, row) for every row of the block that this thread owns
   auto rows = [&](auto&& body) {
@@ -402,13 +402,6 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   }
 }
 
-// Bytes of the sliced-ELL operator: what every iteration reads.
-int64_t operator_bytes(const femk_plan* p) {
-  if (p->sell_cu) return 8 * p->sell_nnz + 2 * p->sell_cu_len;
-  if (p->sell_ct) return 8 * p->sell_nnz + 4 * p->sell_ct_len;
-  return p->sell_nnz * (p->sell_c16 ? 10 : 12);
-}
-
 // One launch of a persistent kernel: co-resident blocks (a cluster, or a cooperative grid).
 template <typename Args>
 int launch_set(const femk_plan* p, void (*kern)(Args), int set, int grid, const Args& a, cudaStream_t s) {
@@ -525,12 +518,18 @@ int ensure_persist(femk_plan* p) {
 
 }  // namespace
 
+// Bytes of the sliced-ELL operator: what every iteration reads.
+int64_t operator_bytes(const femk_plan* p) {
+  if (p->sell_cu) return 8 * p->sell_nnz + 2 * p->sell_cu_len;
+  if (p->sell_ct) return 8 * p->sell_nnz + 4 * p->sell_ct_len;
+  return p->sell_nnz * (p->sell_c16 ? 10 : 12);
+}
+
 // Up to 85 MB of operator the single launch wins, above it the chunked solver does: past that the operator, the
 // vectors and the pairs no longer stay in L2 together. B200, FP64 PCG to 1e-8, us an iteration, chunked ->
 // single launch (MB of operator): P1 32^3 (4.2) 17.4 -> 7.3, 64^3 (32) 21.4 -> 12.0, 80^3 (63) 29.8 -> 18.3, 84^3 (73)
 // 31.4 -> 20.1, 88^3 (84) 33.1 -> 29.7, 92^3 (96) 36.1 -> 47.6; P2 18^3 (13) 20.1 -> 9.6, 26^3 (38) 22.0 -> 13.6, 34^3
 // (79) 31.7 -> 21.3; vertices in no order (12 B an entry), P1 40^3 (12) 26.5 -> 9.5.
-constexpr int64_t kPersistBytes = 85000000;
 bool pcg_persist_fits(const femk_plan* p) {
   return p->persist_ok && p->coop && p->use_sell && p->sell_cols && operator_bytes(p) <= kPersistBytes;
 }

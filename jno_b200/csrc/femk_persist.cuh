@@ -8,7 +8,7 @@
 //
 // Reductions double as barriers over the blocks, and every block ends up with the same bits:
 //  * one block: __syncthreads;
-//  * one cluster of up to 16 blocks: every block stores its partial sums into every other block's shared
+//  * one cluster of up to 16 blocks (or each of a grid's, on its own): every block stores its partial sums into every other block's shared
 //    memory and crosses the hardware cluster barrier (0.7-1.0 us measured with 2-16 blocks of 512 threads);
 //  * a cooperative grid, one block an SM: every block stores its partials in global memory and adds one to a
 //    counter (release), waits until the counter says that all have (acquire), and adds all partials itself in
@@ -40,7 +40,12 @@ struct GridWords {
 
 __device__ __forceinline__ unsigned int cluster_rank() {
   unsigned int r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned int cluster_size() {
+  unsigned int r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
 // stores a double at the address that `p` (own shared memory) has in block `rank` of the cluster
@@ -63,12 +68,13 @@ struct BlockSum {
   long long limit;
   int skip;            // testing: the block that never arrives (-1: none)
   unsigned int phase;  // sums done
+  int rank, size;      // kGrid: this block among those that sum together (all of the grid, or a group with its words)
 
   // one thread of the block: its writes and, after a __syncthreads, its block's are released, the others' acquired
   __device__ __forceinline__ int arrive() {
     unsigned int* c = &words->counter[turn][0];
-    const unsigned int want = gridDim.x * phase;  // wraps with the counter
-    if ((int)blockIdx.x != skip) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
+    const unsigned int want = (unsigned int)size * phase;  // wraps with the counter
+    if (rank != skip) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
     const long long t0 = clock64();
     unsigned int seen, polls = 0;
     for (;;) {
@@ -86,7 +92,7 @@ struct BlockSum {
     __shared__ double tot[2][kSumValues][NB];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int par = (int)(phase & 1);
-    const int G = (int)gridDim.x;
+    const int G = SET == kOneCluster ? (int)cluster_size() : size;
     ++phase;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
@@ -120,7 +126,7 @@ struct BlockSum {
       for (int j = 0; j < NV; ++j) t[j] = warp_sum(lane < W ? red[par][j][lane] : 0.0);
       if (lane == 0) {
 #pragma unroll
-        for (int j = 0; j < NV; ++j) __stcg(&words->part[par][j][blockIdx.x], t[j]);
+        for (int j = 0; j < NV; ++j) __stcg(&words->part[par][j][rank], t[j]);
         ok = arrive();
       }
     }
@@ -166,10 +172,11 @@ struct BlockSum {
 template <typename IDX, bool TAB>
 struct BlockMatrix {
   int32_t s0, ns, fit;   // first slice, slices, slices held in shared memory
+  int32_t tfit;          // TAB: slices whose tables are
   const int32_t* off;    // shared: ns + 1 entry offsets from the block's first entry
   const int32_t* toff;   // shared, TAB: ns + 1 table offsets from the block's first table entry
   const int32_t* runs;   // shared, TAB: run starts of each slice
-  const double* sv;      // shared values and columns (tables) of the first `fit` slices
+  const double* sv;      // shared values and columns of the first `fit` slices (tables: of the first `tfit`)
   const IDX* sc;
   const double* gv;      // the block's entries (tables) in global memory
   const IDX* gc;
@@ -181,11 +188,13 @@ __device__ __forceinline__ int32_t offset_bytes(int32_t ns) {
   return (4 * (ns + 1 + (TAB ? 2 * ns + 1 : 0)) + 15) & ~15;
 }
 
-// First slice of block b: the blocks get equal shares of the work, counted as the stored entries plus 8 a row
-// for the vector updates (rows may be of unequal length). Every thread gets the same answer.
+// First of the nslices slices from sptr on that belongs to block b: the blocks get equal shares of the work, counted
+// as the stored entries plus 8 a row for the vector updates (rows may be of unequal length). Every thread gets the
+// same answer.
 constexpr int kSliceWork = 8 * 32;
 __device__ __forceinline__ int32_t block_slice(const int64_t* __restrict__ sptr, int32_t nslices, int b, int blocks) {
-  const int64_t want = (__ldg(sptr + nslices) + (int64_t)kSliceWork * nslices) * b / blocks;
+  const int64_t e0 = __ldg(sptr);
+  const int64_t want = e0 + (__ldg(sptr + nslices) - e0 + (int64_t)kSliceWork * nslices) * b / blocks;
   int32_t lo = 0, hi = nslices;
   while (lo < hi) {
     const int32_t mid = (lo + hi) >> 1;
@@ -220,10 +229,10 @@ __device__ __forceinline__ double lane_row(const double* vb, const IDX* cb, int3
   return acc;
 }
 
-// The same with the offsets of the row's run: run `run` of `nruns`, kPieceRow entries at a time (16-byte loads of
+// The same with the offsets of the row's run (HELD: the table is in shared memory): run `run` of `nruns`, kPieceRow entries at a time (16-byte loads of
 // the table, one address a run).
 constexpr int kPieceRow = 16;
-template <bool SHARED, typename T, typename G>
+template <bool SHARED, bool HELD, typename T, typename G>
 __device__ __forceinline__ double table_row(const double* vb, const T* tab, int32_t w, int run, int nruns, int32_t row,
                                             const G& g) {
   constexpr int kPad = sizeof(T) == 2 ? 8 : 4, kVec = 16 / (int)sizeof(T);
@@ -237,7 +246,7 @@ __device__ __forceinline__ double table_row(const double* vb, const T* tab, int3
     for (int u = 0; u < kPieceRow / kVec; ++u) {
       q[u] = make_int4(0, 0, 0, 0);
       if (k0 + u * kVec < w)
-        q[u] = SHARED ? reinterpret_cast<const int4*>(t)[u] : __ldg(reinterpret_cast<const int4*>(t) + u);
+        q[u] = HELD ? reinterpret_cast<const int4*>(t)[u] : __ldg(reinterpret_cast<const int4*>(t) + u);
     }
 #pragma unroll
     for (int u = 0; u < kPieceRow; ++u) {
@@ -283,6 +292,8 @@ __device__ __forceinline__ double offset_row(const double* vb, const T* cb, int3
   return acc;
 }
 
+// Tables of lattices take 1/60 of their values' room, and a gather waits for its table entry: all of them are held if
+// they fit a quarter of the room (us an iteration, P1 64^3 11.9 -> 11.6, 80^3 18.3 -> 17.4, P2 34^3 21.3 -> 20.4).
 // The block's share, its first slices copied into `mat` (room bytes of shared memory; off: offset_bytes of shared
 // memory). The whole block calls this.
 template <int THREADS, typename IDX, bool TAB>
@@ -303,17 +314,21 @@ __device__ __forceinline__ void hold_slices(BlockMatrix<IDX, TAB>& m, const int6
   }
   if (threadIdx.x == 0) fit_s = 0;
   __syncthreads();
-  for (int32_t s = threadIdx.x; s < m.ns; s += THREADS)
-    if (8 * (int64_t)off[s + 1] + (int64_t)sizeof(IDX) * (TAB ? toff[s + 1] : off[s + 1]) <= room)
-      atomicMax(&fit_s, s + 1);
+  const int32_t tabs = TAB ? ((int32_t)sizeof(IDX) * toff[m.ns] + 15) & ~15 : 0;
+  const bool all = TAB && tabs <= room / 4;
+  for (int32_t s = threadIdx.x; s < m.ns; s += THREADS) {
+    const int64_t with = all ? tabs : (int64_t)sizeof(IDX) * (TAB ? toff[s + 1] : off[s + 1]);
+    if (8 * (int64_t)off[s + 1] + with <= room) atomicMax(&fit_s, s + 1);
+  }
   __syncthreads();
   m.fit = fit_s;
+  m.tfit = all ? m.ns : m.fit;
   m.off = off;
   m.toff = toff;
   m.runs = rs;
   m.gv = svals + e0;
   m.gc = reinterpret_cast<const IDX*>(cols) + t0;
-  const int32_t held = off[m.fit], theld = TAB ? toff[m.fit] : held;
+  const int32_t held = off[m.fit], theld = TAB ? toff[m.tfit] : held;
   double* sv = reinterpret_cast<double*>(mat);
   IDX* sc = reinterpret_cast<IDX*>(sv + held);
   for (int32_t k = threadIdx.x; k < held; k += THREADS) sv[k] = __ldg(m.gv + k);
@@ -335,8 +350,9 @@ __device__ __forceinline__ double block_row(const BlockMatrix<IDX, TAB>& m, int3
     if (first >= 0) {
       const int s1 = first & 255, s2 = (first >> 8) & 255, s3 = first >> 16;
       const int run = (lane >= s1) + (lane >= s2) + (lane >= s3), nruns = 1 + (s1 < 32) + (s2 < 32) + (s3 < 32);
-      if (s < m.fit) return table_row<true>(m.sv + o + lane, m.sc + t, w, run, nruns, row, g);
-      return table_row<false>(m.gv + o + lane, m.gc + t, w, run, nruns, row, g);
+      if (s < m.fit) return table_row<true, true>(m.sv + o + lane, m.sc + t, w, run, nruns, row, g);
+      if (s < m.tfit) return table_row<false, true>(m.gv + o + lane, m.sc + t, w, run, nruns, row, g);
+      return table_row<false, false>(m.gv + o + lane, m.gc + t, w, run, nruns, row, g);
     }
     if (s < m.fit) return offset_row<true>(m.sv + o + lane, m.sc + t + lane, w, row, g);
     return offset_row<false>(m.gv + o + lane, m.gc + t + lane, w, row, g);

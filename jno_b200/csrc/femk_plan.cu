@@ -735,7 +735,7 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
                   p->diag,     p->dmask,     p->dlist,     p->inc_ptr,   p->inc_elem,  p->cols16,
                   p->work,     p->partials,  p->state,     p->work32,    p->vals32,    p->work64b,
                   p->sell_base, p->sell_cols, p->sell_vals, p->sell_vals32,
-                  p->bar,      p->batch_ws,  p->bicg_ws,   p->bicg_state, p->sell_cu,
+                  p->bar,      p->batch_ws,  p->batch_queue, p->bicg_ws,   p->bicg_state, p->sell_cu,
                   p->coef_tmp, p->theta_ws, p->cmp_ws, p->gm_ws, p->dev_err, p->astr_ptr, p->astr_elem,
                   p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn, p->persist_ws,
                   p->sell_ct, p->perm_ws};
@@ -756,6 +756,8 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
   if (p->batch_exec) cudaGraphExecDestroy(p->batch_exec);
   if (p->batch_ev) cudaEventDestroy(p->batch_ev);
   if (p->batch_stream) cudaStreamDestroy(p->batch_stream);
+  for (cudaStream_t t : p->batch_side)
+    if (t) cudaStreamDestroy(t);
   if (p->bicg_exec) cudaGraphExecDestroy(p->bicg_exec);
   for (cudaEvent_t e : p->bicg_ev)
     if (e) cudaEventDestroy(e);
