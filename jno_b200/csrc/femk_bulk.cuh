@@ -29,6 +29,8 @@
 
 namespace femk {
 
+constexpr int32_t kOneRun = 32 | (32 << 8) | (32 << 16);  // run starts of a slice that is one run
+
 constexpr long long kBulkSpinCycles = 2000000000LL;  // about one second at the B200 boost clock
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -218,7 +220,7 @@ __device__ __forceinline__ bool sell_bulk_rows(unsigned char* wsmem, const int64
     const int32_t w = wid[s], first = rst[s];
     const V* sv = reinterpret_cast<const V*>(stages + s * R::kStage) + lane;
     const IDX* sc = reinterpret_cast<const IDX*>(stages + s * R::kStage + R::kVal);
-    if (first >= 0)  // this lane's run
+    if (first >= 0 && first != kOneRun)  // this lane's run
       sc += ((w + 7) & ~7) * ((lane >= (first & 255)) + (lane >= ((first >> 8) & 255)) + (lane >= (first >> 16)));
     const int32_t row = sl * 32 + lane;
     const bool live = row < n;  // rows past n in the last slice gather nothing

@@ -52,10 +52,16 @@ __device__ __forceinline__ void sell_transpose_warp(double* wbuf, int32_t cap, c
     const int64_t b0 = sptr[sl] + lane;
     const int32_t w = (int32_t)((sptr[sl + 1] - sptr[sl]) >> 5);
     if (src) {
-      for (int32_t k = 0; k < w; ++k) {
-        const int64_t j = b0 + 32 * k;
-        const int32_t q = row < n ? (int32_t)__ldg(src + j) : 255;
-        out[j] = (q != 255 && FEMK_IN_BOUNDS(beg + q, cap, err)) ? f(wbuf[beg + q], row, j) : T(0);
+      for (int32_t k0 = 0; k0 < w; k0 += 8) {
+        int32_t q[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) q[u] = row < n && k0 + u < w ? (int32_t)__ldg(src + b0 + 32 * (k0 + u)) : 255;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (k0 + u >= w) break;
+          const int64_t j = b0 + 32 * (k0 + u);
+          out[j] = (q[u] != 255 && FEMK_IN_BOUNDS(beg + q[u], cap, err)) ? f(wbuf[beg + q[u]], row, j) : T(0);
+        }
       }
     } else {
       for (int32_t k = 0; k < w; ++k) {
