@@ -250,7 +250,7 @@ struct femk_plan {
   int batch_graph_ok = 1;
   // single-launch solvers of systems that stay on the chip (femk_persist.cu)
   int persist_ok = 0;           // 1 unless the options pick the kernels of the chunked solvers
-  void* persist_ws = nullptr;   // f64[6 vstride] {z, p} pairs and vectors, then the GridWords
+  void* persist_ws = nullptr;   // f64[5 vstride] {z, p} pairs and vectors, then the GridWords
   void* persist_words = nullptr;  // (in persist_ws) partial sums and arrival counters of the grid form
   int persist_turn = 0;         // which arrival counter the next launch uses
   void* persist_out = nullptr;  // pinned result

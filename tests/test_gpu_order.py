@@ -95,3 +95,33 @@ def test_batched_solves_put_a_plan_back_into_the_dof_order():
     assert st == 0
     for u in (x, after, mixed):
         assert (torch.linalg.norm(u - before) / torch.linalg.norm(before)).item() <= 1e-7
+
+
+def test_prepared_products_are_capturable_and_hold_no_state():
+    """``spmv_prepared`` on a plan with a row order, straight after ``prepare_operator``: captured in a CUDA graph, and
+    on two streams at once, the bits of the plain call."""
+    from jno_b200.plan import FemPlan
+
+    pts, cells = _mesh(3, (14, 11, 12))
+    plan = FemPlan(pts, cells, 2)
+    vals, _ = plan.assemble(torch.as_tensor(om.logk_field(len(cells), 1020), device="cuda"))
+    plan.prepare_operator(vals)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    xs = [torch.randn(plan.n, dtype=torch.float64, device="cuda", generator=g) for _ in range(2)]
+    ys = [torch.zeros_like(x) for x in xs]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.spmv_prepared(xs[0], ys[0])
+    graph.replay()
+    torch.cuda.synchronize()
+    want = [plan.spmv_prepared(x) for x in xs]
+    assert torch.equal(ys[0], want[0])
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, x, y in zip(streams, xs, ys):
+            with torch.cuda.stream(s):
+                plan.spmv_prepared(x, y)
+    torch.cuda.synchronize()
+    assert torch.equal(ys[0], want[0]) and torch.equal(ys[1], want[1])
