@@ -60,9 +60,9 @@ typedef struct femk_plan_info {
   int32_t cols16;     /* 1 when every column fits an int16 offset from its row (compact inner format) */
   int32_t device;
   int64_t sell_nnz;   /* stored entries of the solver's sliced-ELL copy (padding included), 0 if none */
-  int32_t batch_graph; /* 1 when the last femk_pcg_batched ran as a replayed CUDA graph */
+  int32_t batch_graph; /* 1 when the last femk_pcg_batched* ran as a replayed CUDA graph */
   int64_t sell_col_units; /* column entries the CG-step SpMV streams per product (int16 units when
-                             cols16: per-slice tables, a shared-offset slice stored once) */
+                             cols16: tables by runs of rows, an offset sequence a run) */
   int32_t dim;            /* 2 (triangles) or 3 (tetrahedra) */
 } femk_plan_info;
 
@@ -121,7 +121,8 @@ typedef struct femk_plan_options {
   int32_t size;           /* sizeof(femk_plan_options): set by femk_plan_options_default */
   int32_t solver_layout;  /* 1 (default): the CG loops multiply with a sliced-ELL (SELL-32) copy of the
                              operator; 0: with the canonical CSR itself (the plain method) */
-  int32_t column_tables;  /* 1 (default): a slice whose 32 rows share one column-offset sequence stores it once */
+  int32_t column_tables;  /* 1 (default): rows of a slice with the offsets of one longer row share them (up to four
+                             such runs a slice) */
   int32_t cols16;         /* 1 (default): int16 column offsets in the FP64 sliced-ELL stream when they fit */
   int32_t graph_replay;   /* 1 (default): CG / mixed chunks replayed as CUDA graphs; 0: launched one by one
                              (systems whose operator stays on the chip run femk_pcg as one launch either way) */
@@ -374,10 +375,11 @@ int femk_pcg_mixed(const femk_plan* plan, const double* vals_dev, const double* 
 /*
  * Batched Jacobi-PCG: nprob independent systems held by one plan built on their disjoint union
  * (vertex ids offset per problem), problem k owning rows [row_off[k], row_off[k+1]) (host array,
- * row_off[0] = 0, row_off[nprob] = n). One persistent cooperative launch runs every problem's CG
- * (jax cg semantics, per-problem alpha/beta/stop test) until all have stopped; rows are processed
- * in warp tiles of tile_rows (never crossing a problem) with blocks_per_sm (1 or 2) blocks of 16
- * warps per SM -- the schedule an autotuner chooses. iters_out / relres_out / status_out are host arrays of nprob
+ * row_off[0] = 0, row_off[nprob] = n), each with jax cg semantics (its own alpha/beta/stop test). Problems of up
+ * to 85 MB of operator are each solved by a set of blocks of their own, from a queue; a batch with a larger one, or
+ * on a plan whose options pick kernels of the chunked solvers, advances all problems together in one persistent
+ * cooperative launch, rows in warp tiles of tile_rows (never crossing a problem) with blocks_per_sm (1 or 2) blocks
+ * of 16 warps per SM -- the schedule an autotuner chooses (validated, and without effect, in the first form). iters_out / relres_out / status_out are host arrays of nprob
  * (may be NULL). Returns the first non-OK problem status, FEMK_TIMEOUT if a grid barrier gave up.
  * No reference counterpart (jNO batches by vmap over right-hand sides only).
  */
