@@ -3,7 +3,9 @@
 Each candidate runs the real batched solve once as a warm-up and then ``reps`` (default 3) timed
 times (CUDA events); the candidate with the smallest median is kept and cached in a JSON file
 (``$JNO_B200_TUNE_CACHE``, default ``~/.cache/jno_b200/tune.json``) keyed by the device name, the
-library version and the batch's size signature, so later runs skip the search.
+library version and the batch's size signature, so later runs skip the search. The schedule is the grid
+form's: where FP64 batches run a problem at a time (``femk_batch_sets.cu``, no schedule), the mixed solve,
+which still has one, is what the candidates are timed on.
 """
 
 import json
@@ -53,15 +55,28 @@ def tune(batch, vals, b, inv, tol, candidates=None, reps=3):
     (best, {candidate: median ms})."""
     candidates = CANDIDATES if candidates is None else candidates
     plan = batch.plan
+    _, it, _, _, _ = plan.pcg_batched(batch.row_off, vals, b, None, inv, tol, 0.0, 20_000, *candidates[0])
+    cap = 2 * int(max(it)) + 32  # mixed steps, where FP32 steps do not reach the tolerance
+
+    def solve(tile_rows, bps):
+        if plan.batch_graph:  # the last FP64 solve ran in the grid form
+            plan.pcg_batched(batch.row_off, vals, b, None, inv, tol, 0.0, 20_000, tile_rows, bps)
+            return
+        try:
+            plan.pcg_batched_mixed(batch.row_off, vals, b, inv, None, tol, 0.0, cap, tile_rows, bps)
+        except _lib.FemkError:
+            pass  # a problem that FP32 steps break down on: the others' time still tells
+        plan.batch_graph = False
+
     times = {}
     for tile_rows, bps in candidates:
-        plan.pcg_batched(batch.row_off, vals, b, None, inv, tol, 0.0, 20_000, tile_rows, bps)  # warm-up
+        solve(tile_rows, bps)  # warm-up
         runs = []
         for _ in range(max(1, reps)):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             torch.cuda.synchronize()
             e0.record()
-            plan.pcg_batched(batch.row_off, vals, b, None, inv, tol, 0.0, 20_000, tile_rows, bps)
+            solve(tile_rows, bps)
             e1.record()
             torch.cuda.synchronize()
             runs.append(e0.elapsed_time(e1))
@@ -69,7 +84,7 @@ def tune(batch, vals, b, inv, tol, candidates=None, reps=3):
     best = min(times, key=times.get)
     # leave the plan holding the chosen schedule's graph and tile tables (the last trial's otherwise),
     # so the caller's first solve does not rebuild them
-    plan.pcg_batched(batch.row_off, vals, b, None, inv, tol, 0.0, 20_000, best[0], best[1])
+    solve(*best)
     return {"tile_rows": best[0], "blocks_per_sm": best[1], "ms": times[best]}, times
 
 

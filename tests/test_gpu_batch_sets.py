@@ -109,3 +109,24 @@ def test_one_problem_is_the_single_solve(order, n, shuffled):
     x = plan.pcg_batched([0, plan.n], vals, b, None, inv, 1e-10)[0]
     y = plan.pcg(vals, b, None, inv, 1e-10)[0]
     assert torch.linalg.norm(x - y) <= 1e-7 * torch.linalg.norm(y)
+
+
+def test_the_tuner_times_the_form_that_has_a_schedule(monkeypatch):
+    """FP64 batches that run a problem at a time have no schedule: the candidates are timed on the mixed solve; with the
+    grid form's kernels selected, on the FP64 solve."""
+    from jno_b200 import tuner
+    from jno_b200.batch import BatchedPoisson
+
+    meshes, logk = _problems([6, 9, 5])
+    for opts, called in ((None, "pcg_batched_mixed"), ({"ring64": 14}, "pcg_batched")):
+        batch = BatchedPoisson(meshes, options=opts)
+        vals, b = batch.assemble(logk)
+        inv = batch.plan.jacobi(vals)
+        calls = []
+        for name in ("pcg_batched", "pcg_batched_mixed"):
+            def wrap(*a, _f=getattr(batch.plan, name), _n=name):
+                calls.append(_n)
+                return _f(*a)
+            monkeypatch.setattr(batch.plan, name, wrap)
+        best, times = tuner.tune(batch, vals, b, inv, 1e-8, [(64, 1), (128, 2)], reps=1)
+        assert set(calls[1:]) == {called} and len(calls) == 6 and len(times) == 2
