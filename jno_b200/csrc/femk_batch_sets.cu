@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_sets(SetArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int C = SET == kOneBlock ? 1 : (SET == kOneCluster ? (int)cluster_size() : a.group);
   const int me = SET == kOneBlock ? 0 : (SET == kOneCluster ? (int)cluster_rank() : (int)blockIdx.x % a.group);
-  BlockSum<SET, kCT> all{SET == kGrid ? a.words + blockIdx.x / a.group : nullptr, 0, a.limit, -1, 0u, me, C};
+  BlockSum<SET, kCT> all(SET == kGrid ? a.words + blockIdx.x / a.group : nullptr, 0, a.limit, -1, me, C);
   for (;;) {
     // the next problem; the sum tells every block (whole numbers below 2^53 are exact)
     double next[1] = {me == 0 && threadIdx.x == 0 ? (double)atomicAdd(a.queue, 1u) : 0.0};

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
   hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
-  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u, bid, G};
+  BlockSum<SET, kPT> grid(a.words, a.turn, a.limit, a.skip, bid, G);
   // r = b - A x0, z = D^-1 r
   // gathers of x and of the pairs, range-checked in the bounds-checked build
   auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   unsigned char* mat = reinterpret_cast<unsigned char*>(vec + (ONE ? 10 * nr : (vin ? 8 * nr : 0)));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
   hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
-  BlockSum<SET, kPT> grid{a.words, a.turn, a.limit, a.skip, 0u, bid, G};
+  BlockSum<SET, kPT> grid(a.words, a.turn, a.limit, a.skip, bid, G);
   auto xat = [&](int32_t j) { return FEMK_IN_BOUNDS(j, a.n, a.err) ? __ldcg(a.x + j) : 0.0; };
   // body(local row, row) for every row of the block that this thread owns
   auto rows = [&](auto&& body) {

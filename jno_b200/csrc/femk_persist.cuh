@@ -70,6 +70,14 @@ struct BlockSum {
   unsigned int phase;  // sums done
   int rank, size;      // kGrid: this block among those that sum together (all of the grid, or a group with its words)
 
+  // Every thread of every block, before anything else of this struct. A cluster's blocks store into each other's
+  // shared memory, which exists only once all of them have started: that is waited for here, once a launch (below
+  // 1 us).
+  __device__ __forceinline__ BlockSum(GridWords* words, int turn, long long limit, int skip, int rank, int size)
+      : words(words), turn(turn), limit(limit), skip(skip), phase(0u), rank(rank), size(size) {
+    if (SET == kOneCluster) cluster_sync();
+  }
+
   // one thread of the block: its writes and, after a __syncthreads, its block's are released, the others' acquired
   __device__ __forceinline__ int arrive() {
     unsigned int* c = &words->counter[turn][0];
