@@ -327,7 +327,7 @@ struct ProfData {
   int64_t iters = 0;
 };
 
-// Jacobi-PCG as one persistent launch (femk_persist.cu), for plans whose operator stays on the chip.
+// Jacobi-PCG as one persistent launch (femk_persist.cu), for plans whose operator and vectors stay on the chip.
 constexpr int64_t kPersistBytes = 85000000;  // operator that L2 and shared memory keep (femk_persist.cu)
 int64_t operator_bytes(const femk_plan* p);
 bool pcg_persist_fits(const femk_plan* p);

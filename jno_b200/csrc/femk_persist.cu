@@ -525,14 +525,42 @@ int64_t operator_bytes(const femk_plan* p) {
   return p->sell_nnz * (p->sell_c16 ? 10 : 12);
 }
 
-// Up to 85 MB of operator the single launch wins, above it the chunked solver does: past that the operator, the
-// vectors and the pairs no longer stay in L2 together. B200, FP64 PCG to 1e-8, us an iteration, chunked ->
-// single launch (MB of operator): P1 32^3 (4.2) 17.4 -> 7.3, 64^3 (32) 21.4 -> 12.0, 80^3 (63) 29.8 -> 18.3, 84^3 (73)
-// 31.4 -> 20.1, 88^3 (84) 33.1 -> 29.7, 92^3 (96) 36.1 -> 47.6; P2 18^3 (13) 20.1 -> 9.6, 26^3 (38) 22.0 -> 13.6, 34^3
-// (79) 31.7 -> 21.3; vertices in no order (12 B an entry), P1 40^3 (12) 26.5 -> 9.5.
-bool pcg_persist_fits(const femk_plan* p) {
-  return p->persist_ok && p->coop && p->use_sell && p->sell_cols && operator_bytes(p) <= kPersistBytes;
+// Whether the slices' columns mostly are those of runs of rows (femk_order.cu), not one an entry.
+bool columns_shared(const femk_plan* p) {
+  return (p->sell_cu && 4 * p->sell_cu_len < p->sell_nnz) || (p->sell_ct && 4 * p->sell_ct_len < p->sell_nnz);
 }
+
+// The single launch wins while what an iteration touches stays on the chip: the operator, and 134 B a row of vectors
+// and gathered pairs (fitted: the sizes at which both forms take the same agree on it from 7 to 65 entries a row).
+// Past that its 16 warps an SM wait for HBM where the chunked solver's 64 stream. Columns of their own an entry (no
+// runs) lower the limit: the gathers spread, and more of them miss L1. B200, FP64, us an iteration, chunked -> single
+// launch (MB touched), CG | BiCGStab:
+//   shared columns    P1 32^3 17.4 -> 7.3 (9), 64^3 21.4 -> 12.0, 84^3 30.1 -> 20.1 (156), 86^3 31.8 -> 22.9 (167),
+//                     88^3 32.8 -> 36.3 (179); P2 35^3 32.8 -> 22.6 (132); 2-D P1 900^2 26.0 -> 23.2 (155), 930^2
+//                     27.1 -> 26.4 (165), 960^2 28.0 -> 30.1 (176), 1100^2 34.1 -> 51.6 (231); 2-D P2 415^2
+//                     30.2 -> 23.2 (158), 430^2 31.3 -> 31.4 (170), 460^2 33.8 -> 48.0 (194)
+//                   | P1 80^3 60 -> 45 (135), 84^3 64 -> 62 (156), 88^3 70 -> 88 (179); P2 35^3 64 -> 43 (132);
+//                     2-D P1 850^2 55 -> 47 (138), 900^2 58 -> 59 (155), 960^2 64 -> 75 (176); 2-D P2 400^2
+//                     61.6 -> 58.6 (147), 415^2 62 -> 65 (158)
+//   own columns, P1   shuffled 40^3 26.5 -> 9.5 (21), 76^3 66 -> 44 (143), 2-D 800^2 51 -> 33 (140); shuffled within
+//                     512 vertices 74^3 31.0 -> 29.0 (119), 80^3 36.6 -> 35.8 (150), 2-D 850^2 30.4 -> 28.6 (148),
+//                     900^2 32.5 -> 41.1 (166)
+//                   | shuffled 73^3 86 -> 78 (127), 76^3 90 -> 97 (143), 2-D 700^2 63 -> 54 (107), 800^2 74 -> 78
+//                     (140); within 512 vertices 74^3 65 -> 42 (119), 78^3 72 -> 77 (140)
+//   own columns, P2   shuffled 29^3 39.5 -> 31.5 (106), 2-D 320^2 34.9 -> 31.5 (112), 340^2 36.5 -> 37.5 (126),
+//                     385^2 42.7 -> 55.4 (162)
+//                   | shuffled 29^3 101 -> 64 (106), 2-D 320^2 73 -> 68 (112), 340^2 74 -> 88 (126)
+// The operator alone is held to kPersistBytes as well: no system above it was measured to gain.
+bool persist_fits(const femk_plan* p, bool bicg) {
+  if (!p->persist_ok || !p->coop || !p->use_sell || !p->sell_cols || operator_bytes(p) > kPersistBytes) return false;
+  const double touched = (double)operator_bytes(p) + 134.0 * (double)p->n;
+  const double limit = columns_shared(p) ? (bicg ? 150e6 : 173e6)
+                       : p->order == 1   ? (bicg ? 130e6 : 147e6)
+                                         : (bicg ? 115e6 : 118e6);
+  return touched <= limit;
+}
+
+bool pcg_persist_fits(const femk_plan* p) { return persist_fits(p, false); }
 
 int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double* x, const double* dinv, double tol,
                 double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s) {
@@ -585,9 +613,7 @@ int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double
   return FEMK_OK;
 }
 
-bool bicg_persist_fits(const femk_plan* p) {
-  return p->persist_ok && p->coop && operator_bytes(p) <= kPersistBytes;
-}
+bool bicg_persist_fits(const femk_plan* p) { return persist_fits(p, true); }
 
 int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, double* ws, double tol, double atol,
                  int32_t maxiter, cudaStream_t s, BicgResult* out) {

@@ -1,4 +1,5 @@
-"""Launches of the single-launch and batched solvers: repeated, from other streams, beside other work."""
+"""Launches of the single-launch and batched solvers: which systems take them, repeated, from other streams, beside
+other work."""
 
 import numpy as np
 import pytest
@@ -41,3 +42,48 @@ def test_batches_on_clusters_repeat_to_the_bit():
     for _ in range(30):
         y, jt = batch.plan.pcg_batched(batch.row_off, vals, b, None, inv, 1e-10)[:2]
         assert torch.equal(x, y) and np.array_equal(it, jt)
+
+
+# (dim, cells per axis, order, shuffled, CG in one launch, BiCGStab in one launch): either side of what stays on the
+# chip, where a row has few entries (so that the vectors count) and many, with and without shared columns
+LARGE = [
+    (2, (850, 850), 1, False, True, True),
+    (2, (960, 960), 1, False, False, False),
+    (3, (86, 86, 86), 1, False, True, False),
+    (3, (88, 88, 88), 1, False, False, False),
+    (2, (400, 400), 2, False, True, True),
+    (2, (445, 445), 2, False, False, False),
+    (3, (35, 35, 35), 2, False, True, True),
+    (2, (300, 300), 2, True, True, True),
+    (2, (370, 370), 2, True, False, False),
+    (2, (800, 800), 1, True, True, False),
+]
+
+
+@pytest.mark.parametrize("dim,n,order,shuffled,cg,bicg", LARGE)
+def test_systems_past_the_chip_keep_the_chunked_solvers(dim, n, order, shuffled, cg, bicg):
+    """Few launches tell the single launch. Its first two iterates agree with the chunked solver's to the rounding of
+    row sums, dot products and two quotients: 1e-11 of the largest entry holds with room."""
+    from jno_b200 import _lib
+    from jno_b200.domain import box_points_tets, rect_points_tris
+    from jno_b200.plan import FemPlan
+
+    pts, cells = box_points_tets(*n) if dim == 3 else rect_points_tris(*n)
+    pts = pts[:, :dim]
+    if shuffled:
+        to = np.random.default_rng(4).permutation(len(pts))
+        moved = np.empty_like(pts)
+        moved[to] = pts
+        pts, cells = moved, to[cells]
+    plan = FemPlan(pts, cells, order)
+    chunked = FemPlan(pts, cells, order, options={"ring64": 14})
+    vals, b = plan.assemble(torch.zeros(len(cells), dtype=torch.float64, device="cuda"))
+    inv = plan.jacobi(vals)
+    b = torch.randn(plan.n, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+    launches = _lib.load().femk_kernel_launches
+    for name, one in (("pcg", cg), ("bicgstab", bicg)):
+        before = launches()
+        getattr(plan, name)(vals, b, None, inv, 1e-14, maxiter=30)
+        assert (launches() - before <= 5) == one, name
+        x, y = (getattr(p, name)(vals, b, None, inv, 1e-14, maxiter=2)[0] for p in (plan, chunked))
+        assert (x - y).abs().max() <= 1e-11 * y.abs().max()
