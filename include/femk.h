@@ -376,8 +376,9 @@ int femk_pcg_mixed(const femk_plan* plan, const double* vals_dev, const double* 
  * Batched Jacobi-PCG: nprob independent systems held by one plan built on their disjoint union
  * (vertex ids offset per problem), problem k owning rows [row_off[k], row_off[k+1]) (host array,
  * row_off[0] = 0, row_off[nprob] = n), each with jax cg semantics (its own alpha/beta/stop test). Problems of up
- * to 85 MB of operator are each solved by a set of blocks of their own, from a queue; a batch with a larger one, or
- * on a plan whose options pick kernels of the chunked solvers, advances all problems together in one persistent
+ * to 85 MB of operator are each solved by a set of blocks of their own, from a queue; a batch with a larger one, of
+ * thousands of problems of a few rows or of a numbering in no order, or on a plan whose options pick kernels of the
+ * chunked solvers, advances all problems together in one persistent
  * cooperative launch, rows in warp tiles of tile_rows (never crossing a problem) with blocks_per_sm (1 or 2) blocks
  * of 16 warps per SM -- the schedule an autotuner chooses (validated, and without effect, in the first form). iters_out / relres_out / status_out are host arrays of nprob
  * (may be NULL). Returns the first non-OK problem status, FEMK_TIMEOUT if a grid barrier gave up.

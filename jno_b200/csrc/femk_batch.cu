@@ -1,7 +1,8 @@
 // Batched Jacobi-PCG: many independent problems of uneven size solved in one persistent
 // cooperative launch (captured in a CUDA graph and replayed for repeated solves). FP64 batches whose problems' operators
-// each stay on the chip run in femk_batch_sets.cu instead, up to three times faster; this form serves the others,
-// where a problem wants the whole device, the mixed-precision batches and plans whose options pick chunked kernels.
+// each stay on the chip mostly run in femk_batch_sets.cu instead, up to three times faster; this form serves the others
+// (a problem that wants the whole device, thousands of tiny problems, rows whose gathers spread: batch_sets_fit), the
+// mixed-precision batches and plans whose options pick chunked kernels.
 //
 // The problems live in one plan built on their disjoint union (vertex ids offset per problem), so
 // the plan build and one femk_assemble call serve all of them; problem k owns the contiguous rows

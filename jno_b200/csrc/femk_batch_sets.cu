@@ -332,10 +332,28 @@ void choose_groups(const femk_plan* p, const std::vector<double>& rows, double r
 
 }  // namespace
 
+// Whether a batch runs here or in the grid form. Three things let that one win, beside a problem that does not stay on
+// the chip (B200, FP64 to 1e-8, ms a batch, grid form / here):
+//  * Thousands of problems of a few rows: a problem costs a block 13 us to take, which the grid form does not have.
+//    20000 x 1^3 (8 rows) 0.84 / 1.77, 3000 x 1^3 0.36 / 0.32; 20000 x 2^3 (27 rows) 1.16 / 2.32, 3000 x 2^3 0.39 /
+//    0.38; 20000 x 3^3 (64 rows) 3.09 / 3.92, 6000 x 3^3 1.21 / 1.18; 20000 x 4^3 (125 rows) 6.93 / 5.73.
+//  * Gathers spread over many lines of z: L1 looks up a line a cycle on an SM, and a set is a part of the SMs. Lines a
+//    row, P1: lattices 1.3-2.1 (40 x 30^3 7.2 / 5.0); shuffled within 32 vertices 2 (7.2 / 7.2, 20 x 40^3 11.3 /
+//    10.4); within 128 4.9 (7.2 / 7.7, 11.3 / 11.3); within 512 8.6 (7.3 / 8.5, 11.5 / 12.8), 2-D 20 x 300^2 4.2
+//    (10.2 / 9.0); within 4096, 2-D 5.6 (10.4 / 13.3); all 14 (9.8 / 20.4, 16.7 / 31.1), 2-D 6.1 (13.2 / 28.5).
+//  * ... but not for problems whose z L1 holds (300 x 12^3, 2197 rows, all shuffled 2.7 / 2.05; 150 x 16^3, 4913 rows,
+//    3.5 / 4.1), nor for few rows in all, where the waits count (all shuffled: 40 x 16^3, 197,000 rows, 2.3 / 1.5, 20 x
+//    20^3, 185,000, 2.5 / 2.2, 7 x 30^3, 209,000, 4.4 / 3.6; 14 x 30^3, 417,000, 5.7 / 7.1).
+constexpr double kSpreadLines = 4.5;  // a row
+constexpr int64_t kSmallRows = 2560, kFewRows = 200000;
+
 bool batch_sets_fit(const femk_plan* p, int32_t nprob, const int64_t* row_off) {
   if (!p->persist_ok || !p->use_sell || !p->sell_cols || p->skip_arrival >= 0) return false;
   int64_t rows = 0;
   for (int32_t k = 0; k < nprob; ++k) rows = std::max(rows, row_off[k + 1] - row_off[k]);
+  const double mean = (double)p->n / nprob;
+  if (mean < 96.0 && nprob > 20.0 * p->n_sm * std::max(1.0, mean / 32.0)) return false;
+  if (rows > kSmallRows && p->n > kFewRows && (double)p->sell_lines > kSpreadLines * (double)p->n) return false;
   return (double)rows * operator_bytes(p) <= (double)kPersistBytes * p->n;
 }
 

@@ -171,6 +171,7 @@ struct femk_plan {
   int spmv_L = 16, spmv_U = 2;  // SpMV lanes per row / rows in flight per lane group
   // sliced-ELL solver layout (SELL-32), built with the pattern
   int64_t n_slices = 0, sell_nnz = 0;
+  int64_t sell_lines = 0;        // 128-byte lines of the operand that the gathers of a product touch
   int64_t* sell_ptr = nullptr;   // i64[n_slices+1] first entry of each slice
   int32_t* sell_cols = nullptr;  // i32[sell_nnz] (with sell_c16 and sell_src in one allocation)
   int16_t* sell_c16 = nullptr;   // i16[sell_nnz] col - row, when the bandwidth fits

@@ -337,6 +337,21 @@ __global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* 
   }
 }
 
+// 128-byte lines that the gathers of a product touch, summed over entries and slices (an entry of a slice is one
+// gather of 32 rows): how far apart the columns of neighbouring rows lie.
+__global__ void k_gather_lines(const int64_t* __restrict__ sptr, const int32_t* __restrict__ cols, int64_t nslices,
+                               unsigned long long* __restrict__ lines) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  unsigned long long sum = 0;
+  for (int64_t sl = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; sl < nslices; sl += nwarps)
+    for (int64_t j = sptr[sl] + lane; j < sptr[sl + 1]; j += 32) {
+      const unsigned int same = __match_any_sync(0xffffffffu, cols[j] >> 4);
+      sum += __popc(__ballot_sync(0xffffffffu, __ffs(same) - 1 == lane));
+    }
+  if (lane == 0) atomicAdd(lines, sum);
+}
+
 template <typename T>
 int fill_tables(femk_plan* p, int64_t* len, int64_t* tptr, T** tab, int64_t* total, cudaStream_t s) {
   const int threads = 64, smem = threads * p->max_row * (int)sizeof(long long);
@@ -414,7 +429,10 @@ int build_slices(femk_plan* p, const Order& o, cudaStream_t s) {
     FEMK_TRY(fill_tables(p, len, tptr, &p->sell_ct, &p->sell_ct_len, s));
     p->sell_ctptr = tptr;
   }
+  FEMK_CUDA_TRY(cudaMemsetAsync(len, 0, sizeof(int64_t), s));  // the slices' lengths are not needed any more
+  k_gather_lines<<<counted_launch() + sgrid, kThreads, 0, s>>>(p->sell_ptr, p->sell_cols, ns, (unsigned long long*)len);
   FEMK_CUDA_TRY(cudaGetLastError());
+  FEMK_CUDA_TRY(cudaMemcpyAsync(&p->sell_lines, len, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   return FEMK_OK;
 }

@@ -87,3 +87,45 @@ def test_systems_past_the_chip_keep_the_chunked_solvers(dim, n, order, shuffled,
         assert (launches() - before <= 5) == one, name
         x, y = (getattr(p, name)(vals, b, None, inv, 1e-14, maxiter=2)[0] for p in (plan, chunked))
         assert (x - y).abs().max() <= 1e-11 * y.abs().max()
+
+
+def _shuffled(pts, cells, seed):
+    to = np.random.default_rng(seed).permutation(len(pts))
+    moved = np.empty_like(pts)
+    moved[to] = pts
+    return moved, to[cells]
+
+
+# (side, problems, numbering, the grid form): thousands of tiny problems, and neighbouring rows whose columns lie apart,
+# where the grid form is the faster one
+FORMS = [
+    (3, 500, "lattice", False),
+    (3, 7000, "lattice", True),
+    (1, 3500, "lattice", True),
+    (5, 3500, "lattice", False),
+    (30, 10, "lattice", False),
+    (30, 10, "shuffled", True),
+    (30, 5, "shuffled", False),
+    (12, 120, "shuffled", False),
+]
+
+
+@pytest.mark.parametrize("side,count,numbering,grid", FORMS)
+def test_batches_take_the_form_that_is_faster(side, count, numbering, grid):
+    """Whichever form a batch takes, its solutions are those of the grid form (the bounds of the other batched tests)."""
+    from jno_b200.batch import BatchedPoisson
+
+    mesh = om.equi_distant_box(side, side, side)
+    if numbering == "shuffled":
+        mesh = _shuffled(*mesh, 3)
+    got = []
+    for opts in (None, {"ring64": 14}):
+        batch = BatchedPoisson([mesh] * count, options=opts)
+        logk = torch.as_tensor(om.logk_field(batch.plan.ntet, 941), device="cuda")
+        vals, b = batch.plan.assemble(logk)
+        x, it = batch.plan.pcg_batched(batch.row_off, vals, b, None, batch.plan.jacobi(vals), 1e-10)[:2]
+        got.append((x.view(count, -1), np.asarray(it)))
+        assert batch.plan.batch_graph == (grid or opts is not None)
+    (x, it), (y, jt) = got
+    assert np.abs(it - jt).max() <= 1
+    assert torch.all(torch.linalg.norm(x - y, dim=1) <= 1e-7 * torch.linalg.norm(y, dim=1))
