@@ -1509,8 +1509,7 @@ int ensure_workspace(femk_plan* p) {
   if (p->work) return FEMK_OK;
   FEMK_CUDA_TRY(cudaMalloc(&p->work, sizeof(double) * 5 * p->vstride));
   FEMK_CUDA_TRY(cudaMalloc(&p->partials, sizeof(double) * 4 * (int64_t)p->n_sm * 64));
-  FEMK_CUDA_TRY(cudaMalloc(&p->state, sizeof(CgState)));
-  FEMK_CUDA_TRY(cudaMemset(p->state, 0, sizeof(CgState)));
+  FEMK_CUDA_TRY(cudaMalloc(&p->state, sizeof(CgState)));  // every solve writes all of it first, on its own stream
   FEMK_CUDA_TRY(cudaMallocHost(&p->state_host, 2 * sizeof(CgState)));
   FEMK_CUDA_TRY(cudaMalloc(&p->bar, 64));
   return FEMK_OK;

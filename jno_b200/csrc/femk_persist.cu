@@ -502,15 +502,18 @@ int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
 }
 
 // One allocation for all of the solver's global memory: the pairs, the vectors of blocks whose rows do not fit
-// in shared memory, and the grid's words.
-int ensure_persist(femk_plan* p) {
+// in shared memory, and the grid's words (zeroed on the stream that the launch goes to: another one's clearing could
+// come during the solve).
+int ensure_persist(femk_plan* p, cudaStream_t s) {
   if (!p->persist_ws) {
     const size_t vec = sizeof(double) * 5 * (size_t)p->vstride;
     char* ws = nullptr;
     FEMK_CUDA_TRY(cudaMalloc(&ws, vec + sizeof(GridWords)));
+    const cudaError_t e = cudaMemsetAsync(ws + vec, 0, sizeof(GridWords), s);
+    if (e != cudaSuccess) cudaFree(ws);
+    FEMK_CUDA_TRY(e);
     p->persist_ws = ws;
     p->persist_words = ws + vec;
-    FEMK_CUDA_TRY(cudaMemset(p->persist_words, 0, sizeof(GridWords)));
   }
   if (!p->persist_out) FEMK_CUDA_TRY(cudaMallocHost(&p->persist_out, sizeof(PersistOut)));
   return FEMK_OK;
@@ -565,7 +568,7 @@ bool pcg_persist_fits(const femk_plan* p) { return persist_fits(p, false); }
 int pcg_persist(const femk_plan* pc, const double* vals, const double* b, double* x, const double* dinv, double tol,
                 double atol, int32_t maxiter, int32_t* iters_out, double* relres_out, cudaStream_t s) {
   femk_plan* p = const_cast<femk_plan*>(pc);
-  FEMK_TRY(ensure_persist(p));
+  FEMK_TRY(ensure_persist(p, s));
   FEMK_TRY(ensure_sell_values(p, false));
   FEMK_TRY(launch_sell_values(p, vals, false, s));
   PersistOut* out = (PersistOut*)p->persist_out;
@@ -617,7 +620,7 @@ bool bicg_persist_fits(const femk_plan* p) { return persist_fits(p, true); }
 
 int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, double* ws, double tol, double atol,
                  int32_t maxiter, cudaStream_t s, BicgResult* out) {
-  FEMK_TRY(ensure_persist(p));
+  FEMK_TRY(ensure_persist(p, s));
   out->status = FEMK_TIMEOUT;
   BicgArgs a{};
   a.b = b;

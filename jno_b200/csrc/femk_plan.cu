@@ -876,7 +876,8 @@ extern "C" int femk_plan_create_ex(const double* coords_dev, int dim, int64_t nv
     return st;
   }
   cudaDeviceGetAttribute(&p->coop, cudaDevAttrCooperativeLaunch, p->device);
-  if (cudaMalloc(&p->dev_err, sizeof(int)) != cudaSuccess || cudaMemset(p->dev_err, 0, sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&p->dev_err, sizeof(int)) != cudaSuccess ||
+      cudaMemsetAsync(p->dev_err, 0, sizeof(int), s) != cudaSuccess) {
     femk_plan_destroy(p);
     femk::set_error("femk_plan_create: device allocation failed");
     return FEMK_ENOMEM;

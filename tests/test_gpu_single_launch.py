@@ -129,3 +129,25 @@ def test_batches_take_the_form_that_is_faster(side, count, numbering, grid):
     (x, it), (y, jt) = got
     assert np.abs(it - jt).max() <= 1
     assert torch.all(torch.linalg.norm(x - y, dim=1) <= 1e-7 * torch.linalg.norm(y, dim=1))
+
+
+@pytest.mark.parametrize("n", [(33, 35, 31), (10, 11, 13)])
+@pytest.mark.parametrize("solver", ["pcg", "bicgstab", "pcg_mixed"])
+def test_the_first_solve_of_a_plan_on_a_side_stream_beside_a_busy_default_stream(n, solver):
+    """A plan's workspaces are made during its first solve. Whatever clears them is in the solve's own stream: the
+    default stream's pending work (a sleeping kernel) delays nothing and the second solve has the same bits."""
+    from jno_b200.plan import FemPlan
+
+    pts, cells = om.equi_distant_box(*n)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about 0.1 s of one thread
+    with torch.cuda.stream(side):
+        plan = FemPlan(pts, cells, 1)
+        vals, b = plan.assemble(torch.zeros(len(cells), dtype=torch.float64, device="cuda"))
+        inv = plan.jacobi(vals)
+        args = (vals, b, inv, None, 1e-10) if solver == "pcg_mixed" else (vals, b, None, inv, 1e-10)
+        got = [getattr(plan, solver)(*args) for _ in range(2)]
+    torch.cuda.synchronize()
+    assert got[0][-1] == 0 and got[0][1:] == got[1][1:] and torch.equal(got[0][0], got[1][0])
+    assert (torch.linalg.norm(b - plan.spmv(vals, got[0][0])) <= 2e-10 * torch.linalg.norm(b)).item()

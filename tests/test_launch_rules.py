@@ -38,3 +38,10 @@ def test_a_cluster_has_started_before_any_block_stores_into_another():
     for name in sorted(os.listdir(CSRC)):
         if name != "femk_persist.cuh":
             assert "st_cluster(" not in _code(name), name
+
+
+def test_nothing_is_cleared_on_another_stream_than_the_call_s():
+    """cudaMemset goes to the legacy default stream and does not wait: a solve on a non-blocking stream could run before
+    the clearing of its counters, or beside it."""
+    for name in sorted(os.listdir(CSRC)):
+        assert not re.search(r"\bcudaMemset\s*\(", _code(name)), name
