@@ -928,14 +928,16 @@ bool split_ok(const femk_plan* p, const double* x, const double* dinv) {
   return p->cg_split && aligned16(x) && (dinv == nullptr || aligned16(dinv));
 }
 
-// npq: block shares of <p, q> left by the matrix-free product past kPqShares (0: st->alpha is formed already)
-constexpr int64_t kPqShares = 16384;
+// the matrix-free product's block shares of <p, q>
+double* pq_shares(const femk_plan* p) { return p->partials + (int64_t)kSharesAt * p->n_sm; }
+
+// npq: how many shares it left (0: st->alpha is formed already)
 void launch_update_r(const femk_plan* p, double* r, const double* q, const double* dinv, CgState* st,
                      cudaStream_t s, int npq = 0) {
   auto kern = npq ? (p->l2_mode != 0 ? k_update_r<true, true> : k_update_r<false, true>)
                   : (p->l2_mode != 0 ? k_update_r<true> : k_update_r<false>);
   kern<<<::femk::counted_launch() + vec_grid(kern, kThreads, p), kThreads, 0, s>>>(p->n, r, q, dinv, p->partials, st,
-                                                                                  p->partials + kPqShares, npq);
+                                                                                  pq_shares(p), npq);
 }
 
 // zero_q: q = 0 too (NULL: not)
@@ -1188,14 +1190,14 @@ int ensure_mcells(const femk_plan* pc, cudaStream_t s) {
   return FEMK_OK;
 }
 
-// DOT: *shares block shares of <x, A x> in p->partials + kPqShares
+// DOT: *shares block shares of <x, A x> in pq_shares(p)
 template <bool DOT>
 int launch_matfree_product(const femk_plan* p, const MatFree& m, const double* x, double* y, CgState* st,
                            cudaStream_t s, int* shares = nullptr) {
   MatfreeArgs a{p->xyz, p->kuhn ? p->kuhn : p->mcells, p->kuhn ? p->ntet / 6 : p->ntet, m.param, m.mode, m.scale, x, y,
-                p->dlist, p->n_dir, p->partials + kPqShares, st};
+                p->dlist, p->n_dir, pq_shares(p), st};
   auto launch = [&](auto kern) {
-    const int grid = blocks_for(std::max(a.count, a.ndir), 128, p->n_sm * 16);
+    const int grid = blocks_for(std::max(a.count, a.ndir), 128, p->n_sm * kMatfreeBlocks);
     if (DOT) *shares = grid;
     kern<<<::femk::counted_launch() + grid, 128, 0, s>>>(a);
   };
@@ -1261,7 +1263,7 @@ int enqueue_matfree_chunk(const femk_plan* p, const MatFree& m, double* x, const
       launch_update_r(p, r, q, dinv, st, ws, shares);
       launch_pupdate_x(p, x, pv, r, dinv, q, st, ws);
     } else {
-      k_sum_pq<<<::femk::counted_launch() + 1, kThreads, 0, ws>>>(p->partials + kPqShares, shares, st);
+      k_sum_pq<<<::femk::counted_launch() + 1, kThreads, 0, ws>>>(pq_shares(p), shares, st);
       launch_update(p, x, r, z, pv, q, dinv, p->partials, st, ws);
       launch_pupdate(p, pv, z, st, ws);
       k_zero<<<::femk::counted_launch() + p->n_sm * 8, 256, 0, ws>>>(q, p->n);
@@ -1508,7 +1510,7 @@ int pcg_run(const femk_plan* pc, const double* vals, const MatFree* mf, const do
 int ensure_workspace(femk_plan* p) {
   if (p->work) return FEMK_OK;
   FEMK_CUDA_TRY(cudaMalloc(&p->work, sizeof(double) * 5 * p->vstride));
-  FEMK_CUDA_TRY(cudaMalloc(&p->partials, sizeof(double) * 4 * (int64_t)p->n_sm * 64));
+  FEMK_CUDA_TRY(cudaMalloc(&p->partials, sizeof(double) * kPartialsPerSm * (int64_t)p->n_sm));
   FEMK_CUDA_TRY(cudaMalloc(&p->state, sizeof(CgState)));  // every solve writes all of it first, on its own stream
   FEMK_CUDA_TRY(cudaMallocHost(&p->state_host, 2 * sizeof(CgState)));
   FEMK_CUDA_TRY(cudaMalloc(&p->bar, 64));

@@ -303,6 +303,12 @@ int scan_exclusive_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t 
 
 int ensure_workspace(femk_plan* p);
 
+// The plan's reduction partials, in doubles an SM: the kernels' own reductions (up to three values of 16 blocks) from
+// the start, the matrix-free product's shares of <p, A p> (one a block) from kSharesAt on. In multiples of the SMs, so
+// that a part of a GPU holds them as the whole one does.
+constexpr int kPartialsPerSm = 256, kSharesAt = 64, kMatfreeBlocks = 16;
+static_assert(3 * 16 <= kSharesAt && kSharesAt + kMatfreeBlocks <= kPartialsPerSm, "the shares lie inside the partials");
+
 // The sliced-ELL copy of the pattern in the solver's row order (femk_order.cu). natural_order rebuilds it in the
 // DOF order, for solvers whose problems own runs of DOFs. permute_in copies b, x and dinv (each may be NULL) into
 // plan-owned vectors in the solver's order and redirects the pointers to those; permute_out copies back. Both only

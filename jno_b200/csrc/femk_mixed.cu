@@ -784,7 +784,7 @@ extern "C" int femk_pcg_mixed(const femk_plan* pc, const double* vals, const dou
   femk_plan* p = const_cast<femk_plan*>(pc);
   cudaStream_t s = (cudaStream_t)stream;
   FEMK_TRY(ensure_mixed(p));
-  FEMK_CHECK_ARG(kPartialsA + 4 * (int64_t)update_grid(p) <= 4 * (int64_t)p->n_sm * 64 &&
+  FEMK_CHECK_ARG(kPartialsA + 4 * (int64_t)update_grid(p) <= kPartialsPerSm * (int64_t)p->n_sm &&
                      (int64_t)p->n_sm * 16 * 5 <= kPartialsA,
                  "femk_pcg_mixed: reduction partials do not fit the plan's buffer");
   const int64_t n = p->n;

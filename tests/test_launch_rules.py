@@ -45,3 +45,25 @@ def test_nothing_is_cleared_on_another_stream_than_the_call_s():
     the clearing of its counters, or beside it."""
     for name in sorted(os.listdir(CSRC)):
         assert not re.search(r"\bcudaMemset\s*\(", _code(name)), name
+
+
+def test_matrix_free_shares_lie_inside_the_partials_on_any_number_of_sms():
+    """Where the product's block shares start and how many there are, against the buffer's length, from one SM (a
+    partition of a GPU) to more than the whole one has."""
+    internal, cg = _code("femk_internal.cuh"), _code("femk_cg.cu")
+    values = dict(re.findall(r"\b(k\w+) = (\d+)[,;]", internal))
+    length = re.search(r"cudaMalloc\(&p->partials, sizeof\(double\) \* ([^)]*\)?[^)]*)\)", cg).group(1)
+    start = re.search(r"p->partials \+ ((?:\(int64_t\))?k\w+(?: \* p->n_sm)?)", cg)
+    assert start, "no start of the shares"
+    blocks = re.search(r"blocks_for\(std::max\(a\.count, a\.ndir\), 128, (.*?)\);", cg).group(1)
+
+    def at(expr, n_sm):
+        expr = expr.replace("(int64_t)", "").replace("p->n_sm", str(n_sm))
+        for table in (values, dict(re.findall(r"\b(k\w+) = (\d+)[,;]", cg))):
+            expr = re.sub(r"\bk\w+", lambda m: table.get(m.group(0), m.group(0)), expr)
+        return eval(expr, {}, {})
+
+    for n_sm in (1, 8, 16, 34, 60, 68, 69, 148, 160):
+        # the reductions before the shares: three values of at most 16 blocks an SM
+        assert 3 * 16 * n_sm <= at(start.group(1), n_sm), n_sm
+        assert at(start.group(1), n_sm) + at(blocks, n_sm) <= at(length, n_sm), n_sm
