@@ -232,10 +232,10 @@ int launch_columns(const femk_plan* p, const SetArgs& a, int size, int sets, cud
   return launch_set<SET, int32_t, false>(a, size, sets, s);
 }
 
-// clusters of 2^i blocks that the device holds at once
+// clusters of 2^i blocks that the device holds at once (a part of a GPU may hold none of the larger ones)
 int clusters_fit(femk_plan* p, int i) {
   if (i == 0) return p->n_sm;
-  if (p->batch_fit[i]) return p->batch_fit[i];
+  if (p->batch_fit[i]) return p->batch_fit[i] - 1;
   const auto kern = k_batch_sets<kOneCluster, int16_t, true>;  // the others take the same shared memory and threads
   int fit = 0;
   cudaLaunchConfig_t cfg{};
@@ -254,7 +254,8 @@ int clusters_fit(femk_plan* p, int i) {
     cudaGetLastError();
     fit = 0;
   }
-  return p->batch_fit[i] = std::max(1, fit);
+  p->batch_fit[i] = fit + 1;
+  return fit;
 }
 
 // The set of blocks for a problem: class 0-4 a cluster of 2^i blocks, class 13 - g one of g groups (8 .. 1) of the
@@ -282,6 +283,7 @@ int problem_class(femk_plan* p, int32_t nprob, int64_t rows, double bytes, doubl
   const double want = share * p->n_sm;
   for (int c = 0; c < kClusterClasses; ++c) {
     const bool last = c + 1 == kClusterClasses;
+    if (clusters_fit(p, c) < 1) continue;
     if (last ? std::min<int>(nprob, clusters_fit(p, c)) * bytes > (double)kPersistBytes
              : slices > (c ? kBlockSlices << c : 64))
       continue;

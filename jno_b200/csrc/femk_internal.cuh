@@ -244,7 +244,7 @@ struct femk_plan {
   void* batch_queue = nullptr;  // the batched solver on sets of blocks: results, problems, queues, barriers
   int64_t batch_queue_bytes = 0;
   cudaStream_t batch_side[5] = {};  // ... whose launches run beside one another
-  int batch_fit[5] = {};  // clusters of 2^i blocks that the device holds at once (0: not asked yet)
+  int batch_fit[5] = {};  // 1 + the clusters of 2^i blocks that the device holds at once (0: not asked yet)
   cudaGraphExec_t batch_exec = nullptr;
   cudaStream_t batch_stream = nullptr;
   cudaEvent_t batch_ev = nullptr;

@@ -402,27 +402,32 @@ __global__ void __launch_bounds__(kPT, 1) k_bicg_persist(BicgArgs a) {
   }
 }
 
-// One launch of a persistent kernel: co-resident blocks (a cluster, or a cooperative grid).
-template <typename Args>
-int launch_set(const femk_plan* p, void (*kern)(Args), int set, int grid, const Args& a, cudaStream_t s) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kPT);
-  cfg.dynamicSmemBytes = (size_t)a.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  cfg.attrs = at;
-  cfg.numAttrs = 0;
+constexpr int kNoCluster = -1;  // launch_columns: the device holds no such cluster, nothing was launched
+
+// The launch of co-resident blocks (a cluster, or a cooperative grid).
+void launch_config(int set, int grid, int smem, cudaStream_t s, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+  cfg->gridDim = dim3(grid);
+  cfg->blockDim = dim3(kPT);
+  cfg->dynamicSmemBytes = (size_t)smem;
+  cfg->stream = s;
+  cfg->attrs = at;
+  cfg->numAttrs = set == kOneBlock ? 0 : 1;
   if (set == kOneCluster) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = grid;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
   } else if (set == kGrid) {
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
-    cfg.numAttrs = 1;
   }
+}
+
+// One launch of a persistent kernel.
+template <typename Args>
+int launch_set(void (*kern)(Args), int set, int grid, const Args& a, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  launch_config(set, grid, a.smem, s, &cfg, at);
   counted_launch();
   FEMK_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
   return FEMK_OK;
@@ -453,7 +458,26 @@ template <template <int, typename, bool> class K, int SET, typename IDX, bool TA
 int launch_kernel(const femk_plan* p, const Args& a, int grid, cudaStream_t s) {
   static std::atomic<uint64_t> ready{0};
   FEMK_TRY(prepare_kernel(K<SET, IDX, TAB>::fn, SET, p->device, ready));
-  return launch_set(p, K<SET, IDX, TAB>::fn, SET, grid, a, s);
+  // Whether the device holds a cluster of so many blocks (more than 8, or any with this much shared memory, are not
+  // promised: a part of a GPU may not). Asked once per device and size, a bit for "asked", one for the answer.
+  if constexpr (SET == kOneCluster) {
+    static std::atomic<uint32_t> known[64];
+    std::atomic<uint32_t>& k = known[p->device & 63];
+    const uint32_t bit = (uint32_t)grid;  // 2, 4, 8 or 16
+    if (!(k.load(std::memory_order_acquire) & bit)) {
+      int fit = 0;
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at[1];
+      launch_config(SET, grid, a.smem, s, &cfg, at);
+      if (cudaOccupancyMaxActiveClusters(&fit, K<SET, IDX, TAB>::fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        fit = 0;
+      }
+      k.fetch_or(bit | (fit > 0 ? bit << 16 : 0u), std::memory_order_release);
+    }
+    if (!(k.load(std::memory_order_acquire) & (bit << 16))) return kNoCluster;
+  }
+  return launch_set(K<SET, IDX, TAB>::fn, SET, grid, a, s);
 }
 
 template <template <int, typename, bool> class K, int SET, typename Args>
@@ -469,7 +493,8 @@ int launch_columns(const femk_plan* p, const Args& a, int grid, cudaStream_t s) 
 // as the grid's, until 16 SMs take longer over the rows than that gains (CG, us an iteration, cluster against
 // grid: 2-D P1 100^2, 319 slices, 4.1 / 5.7; P1 20x22x24, 378 slices, 5.8 / 7.0; 2-D P2 60^2, 458 slices, 6.3 /
 // 6.9; 2-D P2 70^2, 622 slices, 7.0 / 6.7; P1 28^3, 763 slices, 8.4 / 7.2). Then a grid of 16 slices a block, a
-// slice a warp, at most a block an SM (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148).
+// slice a warp, at most a block an SM (P1 32^3, 1,124 slices: 71 blocks; the wait takes the same for 148), which also
+// serves devices that hold no such cluster.
 template <template <int, typename, bool> class K, typename Args>
 int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
   a.sptr = p->sell_ptr;
@@ -493,7 +518,8 @@ int launch_persist(femk_plan* p, Args& a, int one_row, cudaStream_t s) {
   if (p->n_slices <= 32 * kMaxCluster) {
     int grid = 2;
     while (grid < kMaxCluster && grid * 16 < p->n_slices) grid *= 2;
-    return launch_columns<K, kOneCluster>(p, a, grid, s);
+    const int rc = launch_columns<K, kOneCluster>(p, a, grid, s);
+    if (rc != kNoCluster) return rc;
   }
   const int grid = (int)std::min<int64_t>(std::min(p->n_sm, kMaxBlocks), (p->n_slices + 15) / 16);
   FEMK_TRY((launch_columns<K, kGrid>(p, a, grid, s)));

@@ -1,7 +1,13 @@
-"""CPU tests of the single-launch and batched solvers' host rules and of what their kernels rely on."""
+"""CPU tests of the single-launch and batched solvers' host rules and of what their kernels rely on.
+
+``launch_harness.cu`` runs the solvers' host code against a made-up CUDA runtime, which logs what is launched where and
+fails the call it is told to."""
 
 import os
 import re
+import subprocess
+
+import pytest
 
 ROOT = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
 CSRC = os.path.join(ROOT, "jno_b200", "csrc")
@@ -67,3 +73,34 @@ def test_matrix_free_shares_lie_inside_the_partials_on_any_number_of_sms():
         # the reductions before the shares: three values of at most 16 blocks an SM
         assert 3 * 16 * n_sm <= at(start.group(1), n_sm), n_sm
         assert at(start.group(1), n_sm) + at(blocks, n_sm) <= at(length, n_sm), n_sm
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    from jno_b200 import _build
+
+    _build.build()
+    out = str(tmp_path_factory.mktemp("harness") / "harness")
+    objs = [os.path.join(ROOT, "_build", o) for o in ("femk_batch_sets.o", "femk_persist.o")]
+    subprocess.run([_build._nvcc(), *_build.ARCH, "-std=c++17", "-O1", "--expt-relaxed-constexpr", "-diag-suppress",
+                    "177,550", "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-o", out,
+                    os.path.join(ROOT, "tests", "launch_harness.cu"), *objs, "-cudart", "none"], check=True)
+
+    def run(*args):
+        return subprocess.run([out, *map(str, args)], check=True, capture_output=True, text=True).stdout.splitlines()
+
+    return run
+
+
+@pytest.mark.parametrize("largest", [16, 8, 4, 2, 1])
+def test_devices_without_large_clusters_get_another_form(harness, largest):
+    """A part of a GPU may hold no cluster of 16 blocks, or none at all: the solvers ask and use the grid."""
+    for rows in (300, 1000, 1500, 4000, 16000, 17000):
+        log = harness(largest, 0, "-", "solve", rows, 15)
+        launches = [line for line in log if line.startswith("launch")]
+        assert len(launches) == 2 and not any(line.startswith("refused") for line in log), log
+        for line in launches:
+            _, _, _, blocks, _, cluster, _, cooperative = line.split()
+            assert int(cluster) <= largest and (int(blocks) == 1 or int(cluster) or cooperative == "1")
+    log = harness(largest, 0, "-", "batch", 100, 1000, 1500, 5000, 9000, 16000, 30000, 120000)
+    assert not any(line.startswith("refused") for line in log), log
