@@ -430,39 +430,49 @@ int batch_sets(femk_plan* p, int32_t nprob, const int64_t* row_off, const double
   // A launch a class, by falling size, those of clusters on streams of their own: the blocks that one has no more
   // problems for go to the next. The groups of a grid wait for one another and run before, one launch at a time.
   bool forked = false;
-  int sides = 0, rc = FEMK_OK;
-  if (cls[0] != cls[nprob - 1]) {
-    if (!p->batch_ev) FEMK_CUDA_TRY(cudaEventCreateWithFlags(&p->batch_ev, cudaEventDisableTiming));
-    for (cudaStream_t& t : p->batch_side)
-      if (!t) FEMK_CUDA_TRY(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
-  }
-  for (int32_t i = 0, j = 0; i < nprob && rc == FEMK_OK; i = j) {
-    const int c = cls[i], size = class_size(p, c);
-    while (j < nprob && cls[j] == c) ++j;
-    const int sets = std::min<int>(j - i, class_sets(p, c));
-    const bool groups = c >= kClusterClasses;
-    a.nprob = j - i;
-    a.order = a.off + nprob + 1 + i;
-    a.queue = (unsigned int*)(a.off + 2 * nprob + 1 + c);
-    a.group = size;
-    if (groups) FEMK_CUDA_TRY(cudaMemsetAsync(a.words, 0, kMaxGroups * sizeof(GridWords), s));
-    cudaStream_t t = s;
-    if (forked) {
-      t = p->batch_side[sides++];
-      FEMK_CUDA_TRY(cudaStreamWaitEvent(t, p->batch_ev, 0));
-    } else if (j < nprob && (!groups || cls[j] < kClusterClasses)) {  // the launches after this one run beside it
-      FEMK_CUDA_TRY(cudaEventRecord(p->batch_ev, s));
-      forked = true;
+  int sides = 0;
+  auto launch_all = [&]() -> int {
+    if (cls[0] != cls[nprob - 1]) {
+      if (!p->batch_ev) FEMK_CUDA_TRY(cudaEventCreateWithFlags(&p->batch_ev, cudaEventDisableTiming));
+      for (cudaStream_t& t : p->batch_side)
+        if (!t) FEMK_CUDA_TRY(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
     }
-    rc = groups   ? launch_columns<kGrid>(p, a, size, sets, t)
-         : c == 0 ? launch_columns<kOneBlock>(p, a, size, sets, t)
-                  : launch_columns<kOneCluster>(p, a, size, sets, t);
-  }
+    for (int32_t i = 0, j = 0; i < nprob; i = j) {
+      const int c = cls[i], size = class_size(p, c);
+      while (j < nprob && cls[j] == c) ++j;
+      const int sets = std::min<int>(j - i, class_sets(p, c));
+      const bool groups = c >= kClusterClasses;
+      a.nprob = j - i;
+      a.order = a.off + nprob + 1 + i;
+      a.queue = (unsigned int*)(a.off + 2 * nprob + 1 + c);
+      a.group = size;
+      if (groups) FEMK_CUDA_TRY(cudaMemsetAsync(a.words, 0, kMaxGroups * sizeof(GridWords), s));
+      cudaStream_t t = s;
+      if (forked) {
+        t = p->batch_side[sides++];
+        FEMK_CUDA_TRY(cudaStreamWaitEvent(t, p->batch_ev, 0));
+      } else if (j < nprob && (!groups || cls[j] < kClusterClasses)) {  // the launches after this one run beside it
+        FEMK_CUDA_TRY(cudaEventRecord(p->batch_ev, s));
+        forked = true;
+      }
+      FEMK_TRY(groups   ? launch_columns<kGrid>(p, a, size, sets, t)
+               : c == 0 ? launch_columns<kOneBlock>(p, a, size, sets, t)
+                        : launch_columns<kOneCluster>(p, a, size, sets, t));
+    }
+    return FEMK_OK;
+  };
+  const int rc = launch_all();
+  // The caller's stream waits for the others also when a call failed: what was launched uses the caller's arrays.
+  cudaError_t joined = cudaSuccess;
   for (int k = 0; k < sides; ++k) {
-    FEMK_CUDA_TRY(cudaEventRecord(p->batch_ev, p->batch_side[k]));
-    FEMK_CUDA_TRY(cudaStreamWaitEvent(s, p->batch_ev, 0));
+    cudaError_t e = cudaEventRecord(p->batch_ev, p->batch_side[k]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->batch_ev, 0);
+    if (e == cudaSuccess) continue;
+    cudaStreamSynchronize(p->batch_side[k]);
+    joined = e;
   }
   FEMK_TRY(rc);
+  FEMK_CUDA_TRY(joined);
   FEMK_CUDA_TRY(cudaMemcpyAsync(out, a.out, nout, cudaMemcpyDeviceToHost, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
   p->batch_graph_used = 0;

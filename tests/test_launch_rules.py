@@ -104,3 +104,27 @@ def test_devices_without_large_clusters_get_another_form(harness, largest):
             assert int(cluster) <= largest and (int(blocks) == 1 or int(cluster) or cooperative == "1")
     log = harness(largest, 0, "-", "batch", 100, 1000, 1500, 5000, 9000, 16000, 30000, 120000)
     assert not any(line.startswith("refused") for line in log), log
+
+
+@pytest.mark.parametrize("name", ["cudaLaunchKernelExC", "cudaStreamWaitEvent", "cudaEventRecord", "cudaMemsetAsync"])
+def test_a_batch_that_fails_half_way_waits_for_what_it_launched(harness, name):
+    """Classes of problems run on streams of their own beside the caller's. Whichever call fails, each of these streams
+    is joined into the caller's (or waited for) after its last launch, before the call returns."""
+    batch = ("batch", 100, 1000, 1500, 5000, 9000, 30000, 120000)
+    assert sum(line.startswith("launch") for line in harness(16, 0, "-", *batch)) == 4
+    for at in range(1, 10):
+        log = harness(16, at, name, *batch)
+        busy, marks = set(), {}
+        for line in log:
+            word = line.split()
+            if word[0] == "launch" and word[1] != "1":
+                busy.add(word[1])
+            elif word[0] == "record":
+                marks[word[1]] = word[2]  # the event now stands for this stream
+            elif word[0] == "wait" and word[1] == "1":
+                busy.discard(marks[word[2]])
+            elif word[0] == "synchronize":
+                busy.discard(word[1])
+        assert not busy, (at, log)
+        if any(line.startswith("failed") for line in log):
+            assert "status 2" in log, (at, log)
