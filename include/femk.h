@@ -380,8 +380,10 @@ int femk_pcg_mixed(const femk_plan* plan, const double* vals_dev, const double* 
  * thousands of problems of a few rows or of a numbering in no order, or on a plan whose options pick kernels of the
  * chunked solvers, advances all problems together in one persistent
  * cooperative launch, rows in warp tiles of tile_rows (never crossing a problem) with blocks_per_sm (1 or 2) blocks
- * of 16 warps per SM -- the schedule an autotuner chooses (validated, and without effect, in the first form). iters_out / relres_out / status_out are host arrays of nprob
- * (may be NULL). Returns the first non-OK problem status, FEMK_TIMEOUT if a grid barrier gave up.
+ * of 16 warps per SM -- the schedule an autotuner chooses (validated, and without effect, in the first form). On a
+ * P2 plan whose solvers have a row order of their own the first call builds a second copy of the layout, in the DOF
+ * order, which the plan keeps (and a copy of the values with it); the other solvers and a prepared operator go on
+ * with the first. iters_out / relres_out / status_out are host arrays of nprob (may be NULL). Returns the first non-OK problem status, FEMK_TIMEOUT if a grid barrier gave up.
  * No reference counterpart (jNO batches by vmap over right-hand sides only).
  */
 int femk_pcg_batched(const femk_plan* plan, int32_t nprob, const int64_t* row_off_host, const double* vals_dev,

@@ -978,9 +978,10 @@ int batched_impl(const femk_plan* pc, int32_t nprob, const int64_t* row_off, con
   FEMK_CHECK_ARG(blocks_per_sm >= 1 && blocks_per_sm <= 2, "femk_pcg_batched: blocks_per_sm must be 1 or 2");
   FEMK_CHECK_ARG(pc->coop, "femk_pcg_batched: the device does not support cooperative launch");
   femk_plan* p = const_cast<femk_plan*>(pc);
-  FEMK_TRY(natural_order(p, (cudaStream_t)stream));  // a problem owns a run of DOFs
   FEMK_CHECK_ARG(row_off[0] == 0 && row_off[nprob] == p->n, "femk_pcg_batched: row_off must span [0, n)");
   for (int32_t k = 0; k < nprob; ++k) FEMK_CHECK_ARG(row_off[k + 1] > row_off[k], "femk_pcg_batched: empty problem");
+  const DofOrder runs(p, (cudaStream_t)stream);  // a problem owns a run of DOFs
+  FEMK_TRY(runs.status);
   if (!mixed && batch_sets_fit(p, nprob, row_off))
     return batch_sets(p, nprob, row_off, vals, b, x, dinv, tol, atol, maxiter, iters_out, relres_out, status_out,
                       (cudaStream_t)stream);

@@ -136,9 +136,36 @@ struct CgState {
   int32_t xpend;    // split update: 1 while x += alpha p of the current iteration is still to be applied
 };
 
+// The sliced-ELL copy of a plan's pattern (SELL-32, femk_order.cu) that its solvers multiply with.
+struct SellLayout {
+  int use_sell = 1;
+  int64_t n_slices = 0, sell_nnz = 0;
+  int64_t sell_lines = 0;        // 128-byte lines of the operand that the gathers of a product touch
+  int64_t* sell_ptr = nullptr;   // i64[n_slices+1] first entry of each slice
+  int32_t* sell_cols = nullptr;  // i32[sell_nnz] (with sell_c16 and sell_src in one allocation)
+  int16_t* sell_c16 = nullptr;   // i16[sell_nnz] col - row, when the bandwidth fits
+  double* sell_vals = nullptr;   // f64[sell_nnz] values gathered for the current solve
+  float* sell_vals32 = nullptr;  // f32[sell_nnz] FP32 values for the mixed-precision inner solve
+  // column tables (femk_order.cu): a slice with up to 4 runs of rows of the same column offsets stores each run's
+  // once, any other slice its 32*w per-entry offsets. 16-bit offsets for the bulk-copy ring ...
+  void* sell_base = nullptr;      // the allocation of sell_ptr, the table starts, sell_runs, perm and pos
+  int32_t* sell_runs = nullptr;   // i32[n_slices] first rows of a slice's second to fourth run (a byte each), -1: per entry
+  int64_t* sell_cuptr = nullptr;  // i64[n_slices+1] first table entry of each slice
+  int16_t* sell_cu = nullptr;     // i16[sell_cu_len]
+  int64_t sell_cu_len = 0;
+  // ... 32-bit ones for the product of wide rows (sell_wide_rows), where 16 bits do not fit
+  int64_t* sell_ctptr = nullptr;  // i64[n_slices+1] first word of each slice
+  int32_t* sell_ct = nullptr;     // i32[sell_ct_len]
+  int64_t sell_ct_len = 0;
+  // the solver's row order (femk_order.cu), NULL: the DOF order
+  int32_t* perm = nullptr;      // i32[n] DOF of each solver row
+  int32_t* pos = nullptr;       // i32[n] solver row of each DOF
+  uint8_t* sell_src = nullptr;  // u8[sell_nnz] place of each entry in its CSR row (255: padding)
+};
+
 }  // namespace femk
 
-struct femk_plan {
+struct femk_plan : femk::SellLayout {
   int device = 0;
   int order = 1, nd = 4;
   int dim = 3, nv = 4;  // spatial dimension, vertices per element (triangles: 2, 3)
@@ -169,32 +196,9 @@ struct femk_plan {
   uint8_t* astr_pos = nullptr;  // u8[astr_len * pb] column positions in the row (0xff: Dirichlet column), pb = nd rounded up to 4
   double* astr_load = nullptr;  // f64[n] integral of the row's basis function (0 on Dirichlet rows)
   int spmv_L = 16, spmv_U = 2;  // SpMV lanes per row / rows in flight per lane group
-  // sliced-ELL solver layout (SELL-32), built with the pattern
-  int64_t n_slices = 0, sell_nnz = 0;
-  int64_t sell_lines = 0;        // 128-byte lines of the operand that the gathers of a product touch
-  int64_t* sell_ptr = nullptr;   // i64[n_slices+1] first entry of each slice
-  int32_t* sell_cols = nullptr;  // i32[sell_nnz] (with sell_c16 and sell_src in one allocation)
-  int16_t* sell_c16 = nullptr;   // i16[sell_nnz] col - row, when the bandwidth fits
-  double* sell_vals = nullptr;   // f64[sell_nnz] values gathered for the current solve
-  float* sell_vals32 = nullptr;  // f32[sell_nnz] FP32 values for the mixed-precision inner solve
-  // column tables (femk_order.cu): a slice with up to 4 runs of rows of the same column offsets stores each run's
-  // once, any other slice its 32*w per-entry offsets. 16-bit offsets for the bulk-copy ring ...
-  int sell_uni = 1;
-  void* sell_base = nullptr;      // the allocation of sell_ptr, the table starts, sell_runs, perm and pos
-  int32_t* sell_runs = nullptr;   // i32[n_slices] first rows of a slice's second to fourth run (a byte each), -1: per entry
-  int64_t* sell_cuptr = nullptr;  // i64[n_slices+1] first table entry of each slice
-  int16_t* sell_cu = nullptr;     // i16[sell_cu_len]
-  int64_t sell_cu_len = 0;
-  // ... 32-bit ones for the product of wide rows (sell_wide_rows), where 16 bits do not fit
-  int64_t* sell_ctptr = nullptr;  // i64[n_slices+1] first word of each slice
-  int32_t* sell_ct = nullptr;     // i32[sell_ct_len]
-  int64_t sell_ct_len = 0;
-  // the solver's row order (femk_order.cu), NULL: the DOF order
-  int32_t* perm = nullptr;      // i32[n] DOF of each solver row
-  int32_t* pos = nullptr;       // i32[n] solver row of each DOF
-  uint8_t* sell_src = nullptr;  // u8[sell_nnz] place of each entry in its CSR row (255: padding)
+  int sell_uni = 1;             // the column_tables plan option
   double* perm_ws = nullptr;    // f64[3 vstride] b, x and D^-1 of a solve in the solver's order
-  int use_sell = 1;
+  femk::SellLayout* dof_order = nullptr;  // a plan with perm: the layout in the DOF order, once a batch needed it
   int l2_mode = 0;               // L2 eviction hints of the FP64 CG kernels (the l2_hints plan option)
   int sell64_c16 = 1;            // FP64 sliced-ELL streams int16 column offsets when available
   int sell_batch = 16;           // entries in flight per thread of the thread-per-row FP64 sliced-ELL kernel
@@ -309,14 +313,26 @@ int ensure_workspace(femk_plan* p);
 constexpr int kPartialsPerSm = 256, kSharesAt = 64, kMatfreeBlocks = 16;
 static_assert(3 * 16 <= kSharesAt && kSharesAt + kMatfreeBlocks <= kPartialsPerSm, "the shares lie inside the partials");
 
-// The sliced-ELL copy of the pattern in the solver's row order (femk_order.cu). natural_order rebuilds it in the
-// DOF order, for solvers whose problems own runs of DOFs. permute_in copies b, x and dinv (each may be NULL) into
+// The sliced-ELL copy of the pattern in the solver's row order (femk_order.cu). permute_in copies b, x and dinv (each may be NULL) into
 // plan-owned vectors in the solver's order and redirects the pointers to those; permute_out copies back. Both only
 // for plans with a row order of their own (p->perm).
 int build_sell(femk_plan* p, cudaStream_t s);
-int natural_order(femk_plan* p, cudaStream_t s);
+void drop_sell(femk_plan* p);
 int permute_in(femk_plan* p, const double** b, double** x, const double** dinv, cudaStream_t s);
 int permute_out(const femk_plan* p, const double* xs, double* x, cudaStream_t s);
+
+// While this lives, the plan's layout is one in the DOF order, for solvers whose problems own runs of DOFs: the plan's
+// own, or on a plan with a row order (p->perm) a second one, built on first use and kept beside it. status: FEMK_OK,
+// or why it could not be built (the plan then is as before).
+struct DofOrder {
+  femk_plan* p;
+  bool swapped = false;
+  int status = FEMK_OK;
+  DofOrder(femk_plan* plan, cudaStream_t s);
+  ~DofOrder();
+  DofOrder(const DofOrder&) = delete;
+  DofOrder& operator=(const DofOrder&) = delete;
+};
 
 // The sliced-ELL value copies of a caller's CSR values (femk_cg.cu): ensure_sell_values allocates
 // sell_vals (and, fp32, sell_vals32) and sets the copy kernels' shared-memory size (not during a

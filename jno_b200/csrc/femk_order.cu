@@ -18,6 +18,8 @@
 // two slices.
 #include <algorithm>
 #include <climits>
+#include <new>
+#include <utility>
 
 #include "femk_element.cuh"
 #include "femk_internal.cuh"
@@ -465,20 +467,45 @@ int build_sell(femk_plan* p, cudaStream_t s) {
   return build_slices(p, o, s);
 }
 
-int natural_order(femk_plan* p, cudaStream_t s) {
-  if (!p->perm) return FEMK_OK;
-  FEMK_CUDA_TRY(cudaDeviceSynchronize());  // nothing may still read what is freed here
-  drop_slices(p);
-  cudaFree(p->sell_vals);
-  cudaFree(p->sell_vals32);
-  p->sell_vals = nullptr;
-  p->sell_vals32 = nullptr;
-  for (cudaGraphExec_t* e : {&p->cg_exec, &p->mx_exec, &p->bicg_exec})
-    if (*e) {
-      cudaGraphExecDestroy(*e);
-      *e = nullptr;
+// frees the plan's layouts
+void drop_sell(femk_plan* p) {
+  for (int i = 0; i < 2; ++i) {
+    drop_slices(p);
+    cudaFree(p->sell_vals);
+    cudaFree(p->sell_vals32);
+    p->sell_vals = nullptr;
+    p->sell_vals32 = nullptr;
+    if (!p->dof_order) break;
+    static_cast<SellLayout&>(*p) = *p->dof_order;
+    delete p->dof_order;
+    p->dof_order = nullptr;
+  }
+}
+
+DofOrder::DofOrder(femk_plan* plan, cudaStream_t s) : p(plan) {
+  if (!p->perm) return;
+  SellLayout& own = *p;
+  if (!p->dof_order) {
+    const SellLayout ordered = own;
+    own = SellLayout{};
+    status = build_slices(p, Order{}, s);
+    if (status != FEMK_OK) drop_slices(p);
+    SellLayout* built = status == FEMK_OK ? new (std::nothrow) SellLayout(own) : nullptr;
+    if (status == FEMK_OK && !built) {
+      drop_slices(p);
+      set_error("femk_pcg_batched: out of host memory");
+      status = FEMK_ENOMEM;
     }
-  return build_slices(p, Order{}, s);
+    own = ordered;
+    if (status != FEMK_OK) return;
+    p->dof_order = built;
+  }
+  std::swap(own, *p->dof_order);
+  swapped = true;
+}
+
+DofOrder::~DofOrder() {
+  if (swapped) std::swap(static_cast<SellLayout&>(*p), *p->dof_order);
 }
 
 int permute_in(femk_plan* p, const double** b, double** x, const double** dinv, cudaStream_t s) {

@@ -734,11 +734,11 @@ extern "C" int femk_plan_destroy(femk_plan* p) {
   void* ptrs[] = {p->xyz,      p->points,    p->cells,     p->indptr,    p->indices,   p->slot,
                   p->diag,     p->dmask,     p->dlist,     p->inc_ptr,   p->inc_elem,  p->cols16,
                   p->work,     p->partials,  p->state,     p->work32,    p->vals32,    p->work64b,
-                  p->sell_base, p->sell_cols, p->sell_vals, p->sell_vals32,
-                  p->bar,      p->batch_ws,  p->batch_queue, p->bicg_ws,   p->bicg_state, p->sell_cu,
+                  p->bar,      p->batch_ws,  p->batch_queue, p->bicg_ws,   p->bicg_state,
                   p->coef_tmp, p->theta_ws, p->cmp_ws, p->gm_ws, p->dev_err, p->astr_ptr, p->astr_elem,
                   p->astr_k, p->astr_pos, p->astr_load, p->kcoef, p->mcells, p->kuhn, p->persist_ws,
-                  p->sell_ct, p->perm_ws};
+                  p->perm_ws};
+  femk::drop_sell(p);
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (p->state_host) cudaFreeHost(p->state_host);

@@ -1,6 +1,8 @@
 """Launches of the single-launch and batched solvers: which systems take them, repeated, from other streams, beside
 other work."""
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -151,3 +153,44 @@ def test_the_first_solve_of_a_plan_on_a_side_stream_beside_a_busy_default_stream
     torch.cuda.synchronize()
     assert got[0][-1] == 0 and got[0][1:] == got[1][1:] and torch.equal(got[0][0], got[1][0])
     assert (torch.linalg.norm(b - plan.spmv(vals, got[0][0])) <= 2e-10 * torch.linalg.norm(b)).item()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_batched_calls_leave_a_plan_s_own_row_order(mixed):
+    """A P2 lattice plan solves in a row order of its own, batches in the DOF order. Neither a batched call that is
+    refused nor one that runs changes what the plan's other calls do: to the bit, prepared operator included."""
+    from jno_b200 import _lib
+
+    plan, logk = _plan((9, 8, 10), 2)
+    vals, b = plan.assemble(logk)
+    inv = plan.jacobi(vals)
+    info = _lib.PlanInfo()
+
+    def layout():
+        _lib.check(plan._lib.femk_plan_get_info(plan.handle, ctypes.byref(info)))
+        return info.sell_nnz, info.sell_col_units
+
+    def calls():
+        return (plan.pcg(vals, b, None, inv, 1e-10)[:3], plan.bicgstab(vals, b, None, inv, 1e-10)[:3],
+                plan.pcg_mixed(vals, b, inv, None, 1e-8)[:4])
+
+    def batched(off):
+        if mixed:
+            return plan.pcg_batched_mixed(off, vals, b, inv, None, 1e-8)
+        return plan.pcg_batched(off, vals, b, None, inv, 1e-10)
+
+    before, want = layout(), calls()
+    x = torch.randn(plan.n, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    plan.prepare_operator(vals)
+    y = plan.spmv_prepared(x)
+    for off in ([0, plan.n - 1], [0, 7, 7, plan.n], [1, plan.n]):
+        with pytest.raises(_lib.FemkError):
+            batched(off)
+        assert layout() == before and torch.equal(plan.spmv_prepared(x), y)
+    for _ in range(2):
+        u = batched([0, plan.n])[0]
+        assert (torch.linalg.norm(u - want[0][0]) <= 1e-6 * torch.linalg.norm(u)).item()
+        assert layout() == before and torch.equal(plan.spmv_prepared(x), y)
+        for w, g in zip(want, calls()):
+            assert torch.equal(w[0], g[0]) and w[1:] == g[1:]
+        plan.prepare_operator(vals)
