@@ -661,7 +661,7 @@ int bicg_persist(femk_plan* p, const double* b, double* x, const double* dinv, d
   a.out = out;
   FEMK_TRY(launch_persist<BicgKernel>(p, a, 80, s));
   FEMK_CUDA_TRY(cudaStreamSynchronize(s));
-  return FEMK_OK;
+  return check_bounds(p, s, "femk_bicgstab");
 }
 
 }  // namespace femk

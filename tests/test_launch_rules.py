@@ -128,3 +128,11 @@ def test_a_batch_that_fails_half_way_waits_for_what_it_launched(harness, name):
         assert not busy, (at, log)
         if any(line.startswith("failed") for line in log):
             assert "status 2" in log, (at, log)
+
+
+def test_the_single_launch_bicgstab_looks_at_its_index_checks(harness):
+    """The bounds-checked build's kernels record a bad index and skip the access; the call has to report it."""
+    for rows in (300, 4000, 17000):
+        log = harness(16, 0, "-", "solve", rows, 15)
+        second = [i for i, line in enumerate(log) if line.startswith("launch")][1]
+        assert "checked" in log[second:], log
