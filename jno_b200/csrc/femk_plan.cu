@@ -479,6 +479,8 @@ int build_pattern(femk_plan* p, int* d_err, int* h_err, cudaStream_t s) {
     k_cols16<<<::femk::counted_launch() + blocks_for(n, kThreads, 65535 * 4), kThreads, 0, s>>>(p->indptr, p->indices,
                                                                                                 n, p->cols16);
   }
+  // positions in a row are bytes in the assembly stream and the solver's layout
+  FEMK_CHECK_ARG(p->max_row < 0xff, "femk_plan_create: a CSR row has 255 or more entries");
   // sliced-ELL copy of the pattern for the solver
   return build_sell(p, s);
 }
@@ -572,7 +574,6 @@ template <int ND>
 int build_assembly_stream(femk_plan* p, cudaStream_t s) {
   constexpr int PB = (ND + 3) / 4 * 4;
   const int64_t n = p->n, ns = (n + 31) / 32;
-  FEMK_CHECK_ARG(p->max_row < 0xff, "femk_plan_create: a CSR row has 255 or more entries");
   Temp len;
   FEMK_CUDA_TRY(cudaMalloc(&len.p, sizeof(int64_t) * (ns + 1)));
   FEMK_TRY(dev_alloc(&p->astr_ptr, ns + 1, s));

@@ -194,3 +194,30 @@ def test_batched_calls_leave_a_plan_s_own_row_order(mixed):
         for w, g in zip(want, calls()):
             assert torch.equal(w[0], g[0]) and w[1:] == g[1:]
         plan.prepare_operator(vals)
+
+
+@pytest.mark.parametrize("spokes", [200, 253, 254, 300, 500, 1200])
+def test_rows_of_255_entries_are_refused_as_such(spokes):
+    """A vertex that all triangles share: 254 entries a row are the most, and more are an argument error with that
+    message, however many."""
+    from scipy.sparse import csr_matrix
+
+    from jno_b200 import _lib
+    from jno_b200.plan import FemPlan
+
+    turn = 2.0 * np.pi * np.arange(spokes) / spokes
+    pts = np.concatenate([[[0.0, 0.0]], np.stack([np.cos(turn), np.sin(turn)], 1)])
+    rim = 1 + np.arange(spokes)
+    cells = np.stack([np.zeros_like(rim), rim, np.roll(rim, -1)], 1)
+    if spokes >= 254:
+        with pytest.raises(_lib.FemkError, match="255 or more entries") as err:
+            FemPlan(pts, cells, 1)
+        assert err.value.status == _lib.FEMK_EINVAL
+        return
+    plan = FemPlan(pts, cells, 1)
+    vals, b = plan.assemble(torch.zeros(spokes, dtype=torch.float64, device="cuda"))
+    x = np.random.default_rng(1).normal(size=plan.n)
+    ptr, col = (t.cpu().numpy() for t in plan.pattern())
+    want = csr_matrix((vals.cpu().numpy(), col, ptr), shape=(plan.n, plan.n)) @ x
+    got = plan.spmv(vals, torch.as_tensor(x, device="cuda")).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-14 * spokes * np.abs(vals.cpu().numpy()).max() * np.abs(x).max()
