@@ -139,11 +139,12 @@ typedef struct femk_plan_options {
   int32_t vec_blocks;     /* blocks per SM of the FP64 CG vector kernels; 0 (default): one full wave */
   int32_t split_updates;  /* 1 (default): FP64 CG vector updates as r-update + direction/x-update kernels */
   int32_t test_skip_arrival; /* testing the bounded waits: the block with this index skips its first
-                                grid-barrier arrival in femk_pcg_batched*, so every other block waits out
-                                barrier_limit_ms and the call returns FEMK_TIMEOUT; -1 (default): none */
+                                grid-barrier arrival in femk_pcg_batched* (which then runs in the grid form) and
+                                all of its arrivals in a solve that runs as one grid, so every other block waits
+                                out barrier_limit_ms and the call returns FEMK_TIMEOUT; -1 (default): none */
   double mixed_delta2;    /* reliable update of the mixed solvers once <r, r> fell by this factor; 0 (default): 1e-4 */
-  double barrier_limit_ms; /* limit of each grid-barrier wait of femk_pcg_batched*, in milliseconds at the
-                              maximum SM clock; 0 (default): 2000 */
+  double barrier_limit_ms; /* limit of each grid-barrier wait of femk_pcg_batched* and of solves that run as one
+                              grid, in milliseconds at the maximum SM clock; 0 (default): 2000 */
 } femk_plan_options;
 
 void femk_plan_options_default(femk_plan_options* opts);
@@ -255,6 +256,13 @@ int femk_spmv_matfree(const femk_plan* plan, const double* param_dev, int coef_m
  * NULL; relres is ||b - A x|| / (||b|| + 1e-30) of the returned x (the eager guard of
  * solver_api.py:224-240). matfree_param_dev != NULL selects the matrix-free operator (vals_dev
  * is then ignored and may be NULL; inv_diag_dev must come from an assembled diagonal).
+ *
+ * A system whose operator and vectors stay on the chip is solved by one launch (so are femk_bicgstab and the steps of
+ * femk_theta_march): one block, one cluster of blocks or, from 16,384 rows on, a cooperative grid of up to a block an
+ * SM. A grid starts when all of its blocks find room at once: beside a long kernel of another stream that keeps SMs
+ * it begins when that one ends. From then on its waits are bounded by barrier_limit_ms (FEMK_TIMEOUT). Larger systems,
+ * and plans with an option that names a kernel of the chunked solver (ring64 = 14, its default, for one), run three
+ * kernels an iteration, which share the SMs with other streams' kernels.
  */
 int femk_pcg(const femk_plan* plan, const double* vals_dev, const double* b_dev, double* x_dev,
              const double* inv_diag_dev, double tol, double atol, int32_t maxiter, int32_t* iters_out,

@@ -16,7 +16,10 @@
 //    together, polled by all blocks, need no second read but took 1.0-5.4 us (the polls of 148 blocks contend),
 //    and 3.0-3.8 us in mailboxes of each reader's own.
 // Only the grid's wait is a spin, and it is bounded: a block that runs out of its clock64 budget gives up and
-// arrives no more, so the others run out too; the kernel returns and the host reports FEMK_TIMEOUT.
+// arrives no more, so the others run out too; the kernel returns and the host reports FEMK_TIMEOUT. The time before
+// all blocks run does not count: a cooperative grid starts as a whole (a grid of 148 blocks with a limit of 1 ms,
+// launched beside a kernel that held one SM for 50 ms, or beside another grid that ran for 11, waited for its end and
+// solved).
 #pragma once
 
 #include <stdint.h>

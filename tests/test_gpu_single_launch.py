@@ -221,3 +221,50 @@ def test_rows_of_255_entries_are_refused_as_such(spokes):
     want = csr_matrix((vals.cpu().numpy(), col, ptr), shape=(plan.n, plan.n)) @ x
     got = plan.spmv(vals, torch.as_tensor(x, device="cuda")).cpu().numpy()
     assert np.abs(got - want).max() <= 1e-14 * spokes * np.abs(vals.cpu().numpy()).max() * np.abs(x).max()
+
+
+def test_solves_of_two_plans_at_once_have_the_bits_of_one_alone():
+    """Two threads, a stream and a plan each: launches that want every SM (a grid of all blocks, a cluster, a batch)
+    take turns or share the device, and neither runs out of time nor changes the other's result."""
+    import threading
+
+    from jno_b200.batch import BatchedPoisson
+
+    def prepare(n):
+        plan, logk = _plan(n)
+        vals, b = plan.assemble(logk)
+        inv = plan.jacobi(vals)
+        return [lambda: plan.pcg(vals, b, None, inv, 1e-10)[:3], lambda: plan.bicgstab(vals, b, None, inv, 1e-10)[:3]]
+
+    meshes = [om.equi_distant_box(n, n, n) for n in (40, 12, 14, 20)]
+    batch = BatchedPoisson(meshes)
+    bvals, load = batch.assemble([om.logk_field(len(t), 950 + i) for i, (_, t) in enumerate(meshes)])
+    binv = batch.plan.jacobi(bvals)
+    calls = [*prepare((45, 46, 47)), *prepare((24, 25, 23)), *prepare((33, 35, 31)),
+             lambda: batch.plan.pcg_batched(batch.row_off, bvals, load, None, binv, 1e-10)[:1]]
+    split = calls[:2] + calls[6:], calls[2:6]
+    torch.cuda.synchronize()
+    want = [[f() for f in mine] for mine in split]
+    got, failed = [[], []], []
+
+    def run(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    got[k].append([f() for f in split[k]])
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001 - reported by the test's thread
+            failed.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for k in range(2):
+        assert len(got[k]) == 20
+        for results in got[k]:
+            for w, g in zip(want[k], results):
+                assert torch.equal(w[0], g[0]) and w[1:] == g[1:]
