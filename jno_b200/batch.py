@@ -2,7 +2,7 @@
 
 The problems are concatenated into one disjoint mesh (vertex ids offset per problem), so one plan,
 one assembly launch and one persistent batched-PCG launch (``femk_pcg_batched``) serve all of them.
-The tile size and blocks per SM of that launch come from :mod:`jno_b200.tuner`.
+The tile size and blocks per SM of the grid form come from :mod:`jno_b200.tuner`.
 No reference counterpart: jNO batches only by ``vmap`` over right-hand sides
 (tests/test_fem_solver_slots.py:123-132).
 """
@@ -57,19 +57,25 @@ class BatchedPoisson:
         ``precision="mixed"``: FP32 inner CG with per-problem FP64 reliable updates
         (``femk_pcg_batched_mixed``); the iterations are then the FP32 ones and ``self.last_outer``
         holds each problem's FP64 residual evaluations."""
-        from .tuner import batched_schedule
+        from .tuner import batched_schedule, cached_schedule
 
         if precision not in ("fp64", "mixed"):
             raise ValueError("precision must be 'fp64' or 'mixed'")
         inv = self.plan.jacobi(vals)
-        sched = schedule or batched_schedule(self, vals, b, inv, tol)
         if precision == "mixed":
+            sched = schedule or batched_schedule(self, vals, b, inv, tol)
             x, it, outer, rel, stv, st = self.plan.pcg_batched_mixed(
                 self.row_off, vals, b, inv, None, tol, 0.0, maxiter, sched["tile_rows"], sched["blocks_per_sm"])
             self.last_outer = outer
         else:
-            x, it, rel, stv, st = self.plan.pcg_batched(self.row_off, vals, b, None, inv, tol, 0.0, maxiter,
-                                                        sched["tile_rows"], sched["blocks_per_sm"])
+            sched = schedule or cached_schedule(self)
+            known = [sched["tile_rows"], sched["blocks_per_sm"]] if sched else []
+            x, it, rel, stv, st = self.plan.pcg_batched(self.row_off, vals, b, None, inv, tol, 0.0, maxiter, *known)
+            if not known and self.plan.batch_graph:
+                # it ran in the grid form, which has a schedule to find; a problem at a time has none
+                sched = batched_schedule(self, vals, b, inv, tol)
+                x, it, rel, stv, st = self.plan.pcg_batched(self.row_off, vals, b, None, inv, tol, 0.0, maxiter,
+                                                            sched["tile_rows"], sched["blocks_per_sm"])
         if st != 0:
             raise RuntimeError(f"batched CG: status {st}, per-problem status {np.unique(stv)}")
         return x, it, rel

@@ -9,7 +9,7 @@
 
 #include "../../include/femk.h"
 
-#define FEMK_VERSION 10300
+#define FEMK_VERSION 10400
 
 namespace femk {
 

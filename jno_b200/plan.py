@@ -59,6 +59,7 @@ class FemPlan:
             if key == "size" or key not in dict(_lib.PlanOptions._fields_):
                 raise ValueError(f"unknown plan option {key!r}")
             setattr(opts, key, value)
+        self.options = dict(options or {})
         handle = ctypes.c_void_p()
         _lib.check(
             lib.femk_plan_create_ex(

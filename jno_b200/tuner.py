@@ -3,9 +3,9 @@
 Each candidate runs the real batched solve once as a warm-up and then ``reps`` (default 3) timed
 times (CUDA events); the candidate with the smallest median is kept and cached in a JSON file
 (``$JNO_B200_TUNE_CACHE``, default ``~/.cache/jno_b200/tune.json``) keyed by the device name, the
-library version and the batch's size signature, so later runs skip the search. The schedule is the grid
-form's: where FP64 batches run a problem at a time (``femk_batch_sets.cu``, no schedule), the mixed solve,
-which still has one, is what the candidates are timed on.
+library version, the batch's size signature and the plan's options, so later runs skip the search. The
+schedule is the grid form's: where FP64 batches run a problem at a time (``femk_batch_sets.cu``, no
+schedule), the mixed solve, which still has one, is what the candidates are timed on.
 """
 
 import json
@@ -47,7 +47,11 @@ def _store(cache):
 def signature(batch):
     name = torch.cuda.get_device_name(batch.plan.device)
     version = _lib.load().femk_version()
-    return f"{name}|femk {version}|nprob={batch.nprob}|n={batch.plan.n}|nnz={batch.plan.nnz}"
+    off = [int(r) for r in batch.row_off]
+    largest = max(b - a for a, b in zip(off, off[1:]))  # with the options it picks the form that is timed
+    options = ",".join(f"{k}={v}" for k, v in sorted(batch.plan.options.items()))
+    return (f"{name}|femk {version}|nprob={batch.nprob}|n={batch.plan.n}|nnz={batch.plan.nnz}|largest={largest}"
+            f"|{options}")
 
 
 def tune(batch, vals, b, inv, tol, candidates=None, reps=3):
@@ -64,8 +68,10 @@ def tune(batch, vals, b, inv, tol, candidates=None, reps=3):
             return
         try:
             plan.pcg_batched_mixed(batch.row_off, vals, b, inv, None, tol, 0.0, cap, tile_rows, bps)
-        except _lib.FemkError:
-            pass  # a problem that FP32 steps break down on: the others' time still tells
+        except _lib.FemkError as e:
+            # a problem that FP32 steps break down on: the others' time still tells. Anything else is no time at all
+            if e.status not in (_lib.FEMK_BREAKDOWN, _lib.FEMK_NONFINITE):
+                raise
         plan.batch_graph = False
 
     times = {}
@@ -86,6 +92,11 @@ def tune(batch, vals, b, inv, tol, candidates=None, reps=3):
     # so the caller's first solve does not rebuild them
     solve(*best)
     return {"tile_rows": best[0], "blocks_per_sm": best[1], "ms": times[best]}, times
+
+
+def cached_schedule(batch):
+    """The schedule that an earlier search left for this batch signature, or None."""
+    return _load().get(signature(batch))
 
 
 def batched_schedule(batch, vals, b, inv, tol):
