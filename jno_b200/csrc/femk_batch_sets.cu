@@ -6,7 +6,8 @@
 // a cluster, or a group of a cooperative grid) takes the next problem of a queue, largest first, solves it alone and
 // takes another. What is in flight is a problem a set, whose operators stay in shared memory and L2 from one iteration
 // to the next, and an iteration's two barriers are the set's own (0.7-1.0 us in a cluster). 96 P1 cubes of sides 8 to
-// 48 (2.2M rows, 306M row-iterations): 18.6 -> 10.3 ms; bound by the latency of a row's loads at 16 warps an SM.
+// 48 (2.2M rows, 306M row-iterations), the solve alone: 18.2 -> 10.1 ms; bound by the latency of a row's loads at 16
+// warps an SM.
 // The steps are those of the grid form (q = A p by the recurrence w + beta q, z the only vector that other blocks
 // gather), its sums in another order:
 //   A  w = A z, p = z + beta p, q = w + beta q, <p, q>      -> alpha
@@ -24,8 +25,8 @@ namespace femk {
 namespace {
 
 constexpr int kCT = 512;  // threads of a block, one block per SM
-constexpr int kUnroll = 4;  // rows in flight a thread in the updates (the 96 cubes on clusters of 16: 1 / 2 / 4 12.4 / 11.9 / 12.0 ms; 9 x 48^3
-                            // 14.3 / 12.6 / 12.6)
+constexpr int kUnroll = 2;  // rows in flight a thread in the updates (1 / 2 / 4: 96 cubes of sides 8 to 48 10.28 / 10.07 /
+                            // 10.31 ms, 9 x 48^3 6.16 / 6.11 / 6.21, 12 x 64^3 24.5 / 24.2 / 24.9)
 constexpr int kSetSmem = 220 * 1024;
 
 struct BatchOut {
@@ -264,7 +265,9 @@ int clusters_fit(femk_plan* p, int i) {
 // alone, 150 a block of a cluster (148 x 0.57 MB of P1 operator), a cluster of 16 as long as the ones that the device
 // holds (7) stay within that, a group of the grid above. A larger set where the problem is so much of the batch that
 // blocks would be left idle. B200, FP64 to 1e-8, ms of a batch, grid form -> clusters of 1 / 2 / 4 / 8 / 16, groups
-// of 24 / 37 / 49 / 74 / 148 blocks (P1 cubes, without the 4 % of own(); the choice in brackets):
+// of 24 / 37 / 49 / 74 / 148 blocks (P1 cubes; the choice in brackets; all columns before own(), which costs 4 %, and
+// the update's two rows in flight, which give back 2: with both the choices take 0.26 / 1.38 / 5.4 / 8.0 on the left and
+// 9.7 / - / - / 24.2 / - on the right):
 //   148 x 10^3   1.24 -> [0.28] / 0.48 / 0.83        28 x 40^3  16.6 -> 17.7 (8) [9.5] (16) / 10.4 / 11.5 / 13.4 / 17.1
 //   148 x 16^3   3.38 -> 2.02 / [1.34] / 1.95        28 x 48^3  32.8 -> 31.3 (16) / [18.7] / 18.6 / 21.8 / 25.5 / 39.5
 //   112 x 24^3   9.52 -> 19.7 / 8.1 / [5.3] / 6.1    24 x 56^3  49.8 -> 60.3 (16) / 43.6 / 30.4 / [28.2] / 31.1 / 44.9
