@@ -25,8 +25,9 @@ namespace femk {
 namespace {
 
 constexpr int kCT = 512;  // threads of a block, one block per SM
-constexpr int kUnroll = 2;  // rows in flight a thread in the updates (1 / 2 / 4: 96 cubes of sides 8 to 48 10.28 / 10.07 /
-                            // 10.31 ms, 9 x 48^3 6.16 / 6.11 / 6.21, 12 x 64^3 24.5 / 24.2 / 24.9)
+// rows in flight a thread in the updates (ms with 1 / 2 / 4: 96 cubes of sides 8 to 48 10.28 / 10.07 / 10.31, 9 x 48^3
+// 6.16 / 6.11 / 6.21, 12 x 64^3 24.5 / 24.2 / 24.9)
+constexpr int kUnroll = 2;
 constexpr int kSetSmem = 220 * 1024;
 
 struct BatchOut {
@@ -265,9 +266,9 @@ int clusters_fit(femk_plan* p, int i) {
 // alone, 150 a block of a cluster (148 x 0.57 MB of P1 operator), a cluster of 16 as long as the ones that the device
 // holds (7) stay within that, a group of the grid above. A larger set where the problem is so much of the batch that
 // blocks would be left idle. B200, FP64 to 1e-8, ms of a batch, grid form -> clusters of 1 / 2 / 4 / 8 / 16, groups
-// of 24 / 37 / 49 / 74 / 148 blocks (P1 cubes; the choice in brackets; all columns before own(), which costs 4 %, and
-// the update's two rows in flight, which give back 2: with both the choices take 0.26 / 1.38 / 5.4 / 8.0 on the left and
-// 9.7 / - / - / 24.2 / - on the right):
+// of 24 / 37 / 49 / 74 / 148 blocks (P1 cubes; the choice in brackets; all columns without own(), which costs 4 %, and
+// with four rows in flight in the updates, which cost 1-3. As it is now: 148 x 10^3 0.26, 148 x 16^3 1.38, 112 x 24^3
+// 5.4, 56 x 32^3 8.0, 28 x 40^3 9.7, 12 x 64^3 24.2):
 //   148 x 10^3   1.24 -> [0.28] / 0.48 / 0.83        28 x 40^3  16.6 -> 17.7 (8) [9.5] (16) / 10.4 / 11.5 / 13.4 / 17.1
 //   148 x 16^3   3.38 -> 2.02 / [1.34] / 1.95        28 x 48^3  32.8 -> 31.3 (16) / [18.7] / 18.6 / 21.8 / 25.5 / 39.5
 //   112 x 24^3   9.52 -> 19.7 / 8.1 / [5.3] / 6.1    24 x 56^3  49.8 -> 60.3 (16) / 43.6 / 30.4 / [28.2] / 31.1 / 44.9
@@ -305,14 +306,16 @@ double groups_time(const femk_plan* p, const std::vector<double>& rows, int i, i
   double busy[kMaxGroups] = {};
   for (int k = i; k < j; ++k) {
     const double over = std::max(0.0, std::min(g, j - i) * rows[k] * row_bytes / (double)kPersistBytes - 1.0);
-    *std::min_element(busy, busy + g) += std::cbrt(rows[k]) * (6.0 + 1.7 * rows[k] / (512.0 * size) * (1.0 + 3.0 * over));
+    const double rounds = rows[k] / (512.0 * size);
+    *std::min_element(busy, busy + g) += std::cbrt(rows[k]) * (6.0 + 1.7 * rounds * (1.0 + 3.0 * over));
   }
   return *std::max_element(busy, busy + g);
 }
 
 // Groups for the problems that want more than a cluster (rows, falling): the first `split` on g1 groups, the rest on
 // g2, in two launches at most.
-void choose_groups(const femk_plan* p, const std::vector<double>& rows, double row_bytes, int* split, int* g1, int* g2) {
+void choose_groups(const femk_plan* p, const std::vector<double>& rows, double row_bytes, int* split, int* g1,
+                   int* g2) {
   const int m = (int)rows.size();
   double best = HUGE_VAL;
   for (int cut = 0; cut < std::min(m, 2 * kMaxGroups); ++cut) {

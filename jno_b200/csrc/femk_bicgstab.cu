@@ -180,7 +180,8 @@ template <int KIND>
 __global__ void __launch_bounds__(kWideWarps * 32, 8) k_bicg_wide(const int64_t* __restrict__ sptr,
                                                               const double* __restrict__ vals,
                                                               const int64_t* __restrict__ tptr,
-                                                              const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n,
+                                                              const int32_t* __restrict__ tab,
+                                                              const int32_t* __restrict__ runs, int64_t n,
                                                               int64_t nslices, const double* __restrict__ x,
                                                               const double* __restrict__ b, Vecs v,
                                                               double* __restrict__ partials, BicgState* st) {
@@ -320,7 +321,8 @@ int launch_spmv(const femk_plan* p, const double* x, const double* b, const Vecs
     if (per_sm > 0) {
       if (!prime)
         kern<<<counted_launch() + p->n_sm * std::min(per_sm, 16), kWideWarps * 32, kSmem, s>>>(
-            p->sell_ptr, p->sell_vals, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, x, b, v, p->partials, st);
+            p->sell_ptr, p->sell_vals, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, x, b, v, p->partials,
+            st);
       FEMK_CUDA_TRY(cudaGetLastError());
       return FEMK_OK;
     }

@@ -259,11 +259,14 @@ __global__ void __launch_bounds__(WPB * 32) k_sell_bulk(const int64_t* __restric
 
 // The CG step on slices of any width with 32-bit column tables (3-D P2 rows; femk_bulk.cuh, sell_wide_rows).
 template <int WPB>
-__global__ void __launch_bounds__(WPB * 32, 8) k_sell_wide(const int64_t* __restrict__ sptr, const double* __restrict__ svals,
-                                                       const int64_t* __restrict__ tptr,
-                                                       const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n, int64_t nslices,
-                                                       const double* __restrict__ x, double* __restrict__ y,
-                                                       double* __restrict__ partials, CgState* st) {
+__global__ void __launch_bounds__(WPB * 32, 8) k_sell_wide(const int64_t* __restrict__ sptr,
+                                                           const double* __restrict__ svals,
+                                                           const int64_t* __restrict__ tptr,
+                                                           const int32_t* __restrict__ tab,
+                                                           const int32_t* __restrict__ runs, int64_t n,
+                                                           int64_t nslices, const double* __restrict__ x,
+                                                           double* __restrict__ y, double* __restrict__ partials,
+                                                           CgState* st) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
   if (blockIdx.x == 0 && threadIdx.x == 0) st->xpend = 0;  // the last x update is applied
   if (st->done) return;

@@ -333,7 +333,8 @@ template <bool REFRESH>
 __global__ void __launch_bounds__(kWideWarps * 32, 8) k_step32_wide(const int64_t* __restrict__ sptr,
                                                                 const float* __restrict__ vals,
                                                                 const int64_t* __restrict__ tptr,
-                                                                const int32_t* __restrict__ tab, const int32_t* __restrict__ runs, int64_t n,
+                                                                const int32_t* __restrict__ tab,
+                                                                const int32_t* __restrict__ runs, int64_t n,
                                                                 int64_t nslices, const float* __restrict__ r,
                                                                 float* __restrict__ w, double* __restrict__ partials,
                                                                 int ga, MixedState* st, int odd) {
@@ -607,8 +608,8 @@ bool launch_step32_wide(const femk_plan* p, const float* r, float* w, MixedState
   if (per_sm <= 0) return false;
   if (prime) return true;
   kern<<<::femk::counted_launch() + p->n_sm * std::min(per_sm, 16), kWideWarps * 32, kSmem, s>>>(
-      p->sell_ptr, p->sell_vals32, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, r, w, p->partials, update_grid(p), st,
-      odd);
+      p->sell_ptr, p->sell_vals32, p->sell_ctptr, p->sell_ct, p->sell_runs, p->n, p->n_slices, r, w, p->partials,
+      update_grid(p), st, odd);
   return true;
 }
 

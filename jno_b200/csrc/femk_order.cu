@@ -54,7 +54,8 @@ int grid_for(const femk_plan* p, int64_t threads) { return blocks_for(threads, k
 template <int ND>
 __global__ void k_edge_ends(const int32_t* __restrict__ cells, int64_t ntet, int64_t nvert, int2* __restrict__ ends) {
   constexpr int NV = Cell<ND>::NV, NE = ND - NV;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ntet * NE; t += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ntet * NE;
+       t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = t / NE;
     const int e = (int)(t % NE);
     const int32_t a = cells[c * ND + cell_edge_a<NV>(e)], b = cells[c * ND + cell_edge_b<NV>(e)];
@@ -326,7 +327,8 @@ __global__ void k_sell_order(const int32_t* __restrict__ indptr, const int32_t* 
     if (nruns > 0) {
       for (int32_t k = lane; k < head; k += 32) {
         // piece p of run q starts at nruns * kPiece * p + q * (the piece's padded entries)
-        const int32_t k0 = sizeof(T) == 2 ? 0 : k / kPiece * kPiece, pk = sizeof(T) == 2 ? head : min(kPiece, head - k0);
+        const int32_t k0 = sizeof(T) == 2 ? 0 : k / kPiece * kPiece;
+        const int32_t pk = sizeof(T) == 2 ? head : min(kPiece, head - k0);
 #pragma unroll
         for (int q = 0; q < kRuns; ++q) {
           if (q >= nruns) continue;
@@ -389,7 +391,8 @@ int build_slices(femk_plan* p, const Order& o, cudaStream_t s) {
   p->n_slices = ns;
   const bool ordered = o.classes > 0;
   // few allocations (one takes 0.3 ms): what the slices' number sizes, what the stored entries' number does, the tables
-  FEMK_CUDA_TRY(cudaMalloc(&p->sell_base, sizeof(int64_t) * 3 * (ns + 1) + sizeof(int32_t) * (ns + (ordered ? 2 * n : 0))));
+  const int64_t words = ns + (ordered ? 2 * n : 0);
+  FEMK_CUDA_TRY(cudaMalloc(&p->sell_base, sizeof(int64_t) * 3 * (ns + 1) + sizeof(int32_t) * words));
   p->sell_ptr = (int64_t*)p->sell_base;
   int64_t* tptr = p->sell_ptr + ns + 1;
   int64_t* len = tptr + ns + 1;

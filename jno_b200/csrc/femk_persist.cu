@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg_persist(PcgArgs a) {
   double* qs = vin ? vec + 3 * nr : a.work + 2 * a.vstride + r0;
   const double* ds = vin ? vec + 4 * nr : a.dinv + r0;  // not read without a preconditioner
   double2* zps = reinterpret_cast<double2*>(vec + 5 * nr);
-  unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr) : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
+  unsigned char* mat = ONE ? reinterpret_cast<unsigned char*>(zps + nr)
+                           : reinterpret_cast<unsigned char*>(vec + (vin ? 5 * nr : 0));
   if (SET == kGrid && bid == 0 && threadIdx.x == 0) a.words->counter[a.turn ^ 1][0] = 0u;
   hold_slices<kPT>(m, a.sptr, a.cols, a.svals, a.tptr, a.runs, off, mat, a.smem - (int32_t)(mat - ps_smem));
   BlockSum<SET, kPT> grid(a.words, a.turn, a.limit, a.skip, bid, G);

@@ -8,8 +8,9 @@
 //
 // Reductions double as barriers over the blocks, and every block ends up with the same bits:
 //  * one block: __syncthreads;
-//  * one cluster of up to 16 blocks (or each of a grid's, on its own): every block stores its partial sums into every other block's shared
-//    memory and crosses the hardware cluster barrier (0.7-1.0 us measured with 2-16 blocks of 512 threads);
+//  * one cluster of up to 16 blocks (or each of a grid's, on its own): every block stores its partial sums into every
+//    other block's shared memory and crosses the hardware cluster barrier (0.7-1.0 us measured with 2-16 blocks of 512
+//    threads);
 //  * a cooperative grid, one block an SM: every block stores its partials in global memory and adds one to a
 //    counter (release), waits until the counter says that all have (acquire), and adds all partials itself in
 //    block order: 2.1 us, the same for 2 and for 148 blocks. Words that carry the partial and a phase number
@@ -54,7 +55,8 @@ __device__ __forceinline__ unsigned int cluster_size() {
 // stores a double at the address that `p` (own shared memory) has in block `rank` of the cluster
 __device__ __forceinline__ void st_cluster(const double* p, unsigned int rank, double v) {
   uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  const uint32_t own = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own), "r"(rank));
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
@@ -193,7 +195,7 @@ struct BlockMatrix {
   const IDX* gc;
 };
 
-// 32-bit words of shared memory for the offsets of ns slices
+// bytes of shared memory for the offsets (and, TAB, the run starts) of ns slices
 template <bool TAB>
 __device__ __forceinline__ int32_t offset_bytes(int32_t ns) {
   return (4 * (ns + 1 + (TAB ? 2 * ns + 1 : 0)) + 15) & ~15;
@@ -240,8 +242,8 @@ __device__ __forceinline__ double lane_row(const double* vb, const IDX* cb, int3
   return acc;
 }
 
-// The same with the offsets of the row's run (HELD: the table is in shared memory): run `run` of `nruns`, kPieceRow entries at a time (16-byte loads of
-// the table, one address a run).
+// The same with the offsets of the row's run (HELD: the table is in shared memory): run `run` of `nruns`, kPieceRow
+// entries at a time (16-byte loads of the table, one address a run).
 constexpr int kPieceRow = 16;
 template <bool SHARED, bool HELD, typename T, typename G>
 __device__ __forceinline__ double table_row(const double* vb, const T* tab, int32_t w, int run, int nruns, int32_t row,
@@ -303,13 +305,13 @@ __device__ __forceinline__ double offset_row(const double* vb, const T* cb, int3
   return acc;
 }
 
-// Tables of lattices take 1/60 of their values' room, and a gather waits for its table entry: all of them are held if
-// they fit a quarter of the room (us an iteration, P1 64^3 11.9 -> 11.6, 80^3 18.3 -> 17.4, P2 34^3 21.3 -> 20.4).
 // The block's share, its first slices copied into `mat` (room bytes of shared memory; off: offset_bytes of shared
-// memory). The whole block calls this.
+// memory). The whole block calls this. Tables of lattices take 1/60 of their values' room, and a gather waits for its
+// table entry: all of them are held if they fit a quarter of the room (us an iteration, P1 64^3 11.9 -> 11.6, 80^3
+// 18.3 -> 17.4, P2 34^3 21.3 -> 20.4).
 template <int THREADS, typename IDX, bool TAB>
-__device__ __forceinline__ void hold_slices(BlockMatrix<IDX, TAB>& m, const int64_t* __restrict__ sptr, const void* cols,
-                                            const double* svals, const int64_t* __restrict__ tptr,
+__device__ __forceinline__ void hold_slices(BlockMatrix<IDX, TAB>& m, const int64_t* __restrict__ sptr,
+                                            const void* cols, const double* svals, const int64_t* __restrict__ tptr,
                                             const int32_t* __restrict__ runs, int32_t* off, unsigned char* mat,
                                             int32_t room) {
   __shared__ int32_t fit_s;
