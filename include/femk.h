@@ -139,9 +139,10 @@ typedef struct femk_plan_options {
   int32_t vec_blocks;     /* blocks per SM of the FP64 CG vector kernels; 0 (default): one full wave */
   int32_t split_updates;  /* 1 (default): FP64 CG vector updates as r-update + direction/x-update kernels */
   int32_t test_skip_arrival; /* testing the bounded waits: the block with this index skips its first
-                                grid-barrier arrival in femk_pcg_batched* (which then runs in the grid form) and
-                                all of its arrivals in a solve that runs as one grid, so every other block waits
-                                out barrier_limit_ms and the call returns FEMK_TIMEOUT; -1 (default): none */
+                                grid-barrier arrival in femk_pcg_batched* (in the grid form, which the option
+                                picks for all but one problem of more than 32,768 rows) and all of its arrivals
+                                in a solve that runs as one grid, so every other block waits out
+                                barrier_limit_ms and the call returns FEMK_TIMEOUT; -1 (default): none */
   double mixed_delta2;    /* reliable update of the mixed solvers once <r, r> fell by this factor; 0 (default): 1e-4 */
   double barrier_limit_ms; /* limit of each grid-barrier wait of femk_pcg_batched* and of solves that run as one
                               grid, in milliseconds at the maximum SM clock; 0 (default): 2000 */

@@ -48,6 +48,7 @@ struct SetArgs {
   int32_t group;         // kGrid: blocks of a group
   GridWords* words;      // kGrid: a group's words each, zeroed
   long long limit;
+  int32_t skip;          // kGrid, testing: the block of a group that never arrives (-1: none)
   const double* b;
   double* x;
   const double* dinv;
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_sets(SetArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int C = SET == kOneBlock ? 1 : (SET == kOneCluster ? (int)cluster_size() : a.group);
   const int me = SET == kOneBlock ? 0 : (SET == kOneCluster ? (int)cluster_rank() : (int)blockIdx.x % a.group);
-  BlockSum<SET, kCT> all(SET == kGrid ? a.words + blockIdx.x / a.group : nullptr, 0, a.limit, -1, me, C);
+  BlockSum<SET, kCT> all(SET == kGrid ? a.words + blockIdx.x / a.group : nullptr, 0, a.limit, a.skip, me, C);
   for (;;) {
     // the next problem; the sum tells every block (whole numbers below 2^53 are exact)
     double next[1] = {me == 0 && threadIdx.x == 0 ? (double)atomicAdd(a.queue, 1u) : 0.0};
@@ -356,9 +357,11 @@ constexpr double kSpreadLines = 4.5;  // a row
 constexpr int64_t kSmallRows = 2560, kFewRows = 200000;
 
 bool batch_sets_fit(const femk_plan* p, int32_t nprob, const int64_t* row_off) {
-  if (!p->persist_ok || !p->use_sell || !p->sell_cols || p->skip_arrival >= 0) return false;
+  if (!p->persist_ok || !p->use_sell || !p->sell_cols) return false;
   int64_t rows = 0;
   for (int32_t k = 0; k < nprob; ++k) rows = std::max(rows, row_off[k + 1] - row_off[k]);
+  // testing the bounded waits: here only a group of the grid waits so, which one large problem is sure to get
+  if (p->skip_arrival >= 0 && (nprob > 1 || rows <= 2 * 32 * 32 * kMaxCluster)) return false;
   const double mean = (double)p->n / nprob;
   if (mean < 96.0 && nprob > 20.0 * p->n_sm * std::max(1.0, mean / 32.0)) return false;
   if (rows > kSmallRows && p->n > kFewRows && (double)p->sell_lines > kSpreadLines * (double)p->n) return false;
@@ -422,6 +425,7 @@ int batch_sets(femk_plan* p, int32_t nprob, const int64_t* row_off, const double
   a.off = (const int32_t*)(base + nout);
   a.words = (GridWords*)(base + words0);
   a.limit = p->barrier_spin;
+  a.skip = p->skip_arrival;
   a.b = b;
   a.x = x;
   a.dinv = dinv;

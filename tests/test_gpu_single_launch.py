@@ -268,3 +268,25 @@ def test_solves_of_two_plans_at_once_have_the_bits_of_one_alone():
         for results in got[k]:
             for w, g in zip(want[k], results):
                 assert torch.equal(w[0], g[0]) and w[1:] == g[1:]
+
+
+def test_a_batch_group_s_wait_that_runs_out_is_a_status():
+    """Block 0 of the group that solves the one problem never arrives: the others give up after the limit, the call
+    reports it and leaves the problem that status, and the device goes on."""
+    from jno_b200 import _lib
+
+    bad, logk = _plan((34, 33, 32), options={"test_skip_arrival": 0, "barrier_limit_ms": 5.0})
+    vals, b = bad.assemble(logk)
+    inv = bad.jacobi(vals)
+    for _ in range(2):
+        status = np.zeros(1, dtype=np.int32)
+        off = np.asarray([0, bad.n], dtype=np.int64)
+        x = torch.zeros_like(b)
+        st = bad._lib.femk_pcg_batched(bad.handle, 1, ctypes.c_void_p(off.ctypes.data), _lib.ptr(vals), _lib.ptr(b),
+                                       _lib.ptr(x), _lib.ptr(inv), 1e-8, 0.0, 1000, 64, 2, None, None,
+                                       ctypes.c_void_p(status.ctypes.data), _lib.stream_handle())
+        assert st == _lib.FEMK_TIMEOUT and status[0] == _lib.FEMK_TIMEOUT
+        assert b"gave up" in bad._lib.femk_last_error_string()
+    good = _plan((34, 33, 32))[0]
+    x, it, rel, stv, st = good.pcg_batched([0, good.n], vals, b, None, inv, 1e-8)
+    assert st == 0 and rel[0] <= 2e-8 and not good.batch_graph
